@@ -39,6 +39,9 @@ struct Params {
     float inv_rest;        // 1 / rest_density
     float inv_rest_sq;     // 1 / rest_density^2
     float settles;         // |gravity| spacing: the speed under which water settles on a body (couple.rs:390)
+    float slope_scale;     // scale * -20 (mod.rs:154)
+    float one;             // 1, where the compiler cannot see it (sum2)
+    uint32_t odd_radius;   // the radius is outside the range whose divisions take the reciprocal (div_radius2)
 };
 
 // Per-substep constants, in device memory so a captured substep reads the current ones.
@@ -150,6 +153,8 @@ struct GridDev {
     uint32_t cells;        // sorted: occupied cells
     const uint32_t* start; // dense: volume + 1; sorted: cells + 1
     const int4* keys;      // sorted: key of each occupied cell
+    const uint32_t* near;  // dense, optional: for each cell, which of the 27 cells around it hold points (bit
+                           // (dz + 1) * 9 + (dy + 1) * 3 + dx + 1, the list order)
 
 #ifdef __CUDACC__
     __device__ __forceinline__ bool range(long long cx, long long cy, long long cz, uint32_t& b,
@@ -425,6 +430,43 @@ __device__ __forceinline__ void each_near(const Params& p, const GridDev& g, con
             }
         }
     }
+}
+
+// ---- two f32 values an instruction -------------------------------------------------------------
+// sm_100's packed f32 operations: each half rounds on its own, exactly as the scalar operation.
+// ptxas contracts a packed multiplication and a packed addition of its result into one fma whatever
+// their rounding modifiers and --fmad say, so sums of packed products go through sum2.
+
+struct f32x2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ f32x2 splat2(float x) { return pack2(x, x); }
+__device__ __forceinline__ void unpack2(f32x2 a, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// a + b as a * 1 + b, the 1 out of the compiler's sight: rounds as the addition, and nothing
+// contracts into it.
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c);
+__device__ __forceinline__ f32x2 sum2(const Params& p, f32x2 a, f32x2 b) { return fma2(a, splat2(p.one), b); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
 }
 
 // f32 bits for atomicMax on non-negative floats.

@@ -103,6 +103,22 @@ __global__ void k_count_cells(Params p, const float4* __restrict__ pos, const in
     slot[i] = atomicAdd(&count[l], 1u);
 }
 
+// GridDev::near of a dense table, a thread a cell
+__global__ void k_grid_near(GridDev g, uint32_t* __restrict__ near) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= uint32_t(g.sx) * uint32_t(g.sy) * uint32_t(g.sz)) return;
+    const int z = int(c % uint32_t(g.sz)), y = int(c / uint32_t(g.sz) % uint32_t(g.sy)),
+              x = int(c / uint32_t(g.sz) / uint32_t(g.sy));
+    uint32_t mask = 0;
+    for (int t = 0; t < 27; ++t) {
+        const int qx = x + t % 3 - 1, qy = y + t / 3 % 3 - 1, qz = z + t / 9 - 1;
+        if (qx < 0 || qx >= g.sx || qy < 0 || qy >= g.sy || qz < 0 || qz >= g.sz) continue;
+        const uint32_t q = (uint32_t(qx) * uint32_t(g.sy) + uint32_t(qy)) * uint32_t(g.sz) + uint32_t(qz);
+        if (__ldg(&g.start[q + 1]) > __ldg(&g.start[q])) mask |= 1u << t;
+    }
+    near[c] = mask;
+}
+
 __global__ void k_scatter_members(uint32_t n, const uint32_t* __restrict__ lin, const uint32_t* __restrict__ slot,
                                   const uint32_t* __restrict__ start, const uint32_t* __restrict__ ids,
                                   uint32_t* members) {
@@ -261,35 +277,197 @@ __device__ __forceinline__ float ground_near(const TerrainDev& T, float px, floa
     return ground;
 }
 
-// The second half of a list-building walk: for each of row's first m listed neighbours, in list
-// order, q = pts[index] and the entry's factor becomes f(q, index, k * 32), k the entry's place
-// in the list (k * 32: its offset from the row's first entry in the warp-tiled layout).  Four
-// entries and their points are read ahead of their use (the entries were written by this thread
-// just before: plain loads).
-template <class F>
-__device__ __forceinline__ void relist(const PairLists& l, uint32_t row, uint32_t m, const float4* __restrict__ pts,
-                                       F&& f) {
-    if (m == 0) return;
-    uint2* base = l.e + l.at(row, 0);
-    uint32_t j[4];
+// ---- the density pass's two halves: the candidate scan, then the pair terms -------------------
+// What bounds the pass: instruction issue and the latency of its gathers (the lists it writes are
+// ~0.75 GB at 1M particles with kept gradients, 115 us at the copy rate).  Against a scan that
+// branched per candidate, checked every cell's bounds, searched the walls' 27 cells for every
+// particle, and divided three times a pair with one pair at a time (us, EXACT): 583 -> 433 (1M
+// DFSPH), 198 -> 141 (250k DFSPH), 241 -> 159 (315k WCSPH), 474 -> 304 (64k WCSPH at support 4),
+// 87 -> 59 (75k WCSPH).
+// Four candidates and two pairs in flight, at 64 registers and four blocks a SM: two candidates
+// measured 470 us at 1M, six 522, eight 556 (spills; 497 at 109 registers and two blocks), four
+// pairs 482, and 48 registers for five blocks 571.
+constexpr int kScanUnroll = 4;
+constexpr int kPairUnroll = 2;
+
+// Lists the points of cells [b, e) within reach of `at`, in array order: each kept index goes to
+// out[nf * 32] (room for `cap`; the count goes on past it).  Four candidates' gathers are in flight
+// at a time, and a kept one costs a predicated store and an add: no branch, so the lanes of a warp
+// that keep nothing do not wait for those that do.  axy, az: the negated position; x and y of the
+// test run packed, each operation rounded as each_in_cell's.
+__device__ __forceinline__ void scan_range(const Params& p, const float4* __restrict__ pts, uint32_t b, uint32_t e,
+                                           f32x2 axy, float az, uint32_t* out, uint32_t cap,
+                                           uint32_t& nf) {
+    const ulonglong2* __restrict__ q2 = reinterpret_cast<const ulonglong2*>(pts);
+#pragma unroll 1
+    for (uint32_t j = b; j < e; j += kScanUnroll) {
+        ulonglong2 q[kScanUnroll];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) j[u] = base[size_t(u < (int)m ? u : m - 1) * 32u].x;
-    for (uint32_t k = 0; k < m; k += 4) {
-        float4 q[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) q[u] = __ldg(&pts[j[u]]);
-        uint32_t next[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            uint32_t kk = k + 4 + u;
-            next[u] = base[size_t(kk < m ? kk : m - 1) * 32u].x;
+        for (int u = 0; u < kScanUnroll; ++u) {
+            if (j + u < e) q[u] = __ldg(q2 + j + u);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (k + u < m)
-                base[size_t(k + u) * 32u] = make_uint2(j[u], __float_as_uint(f(q[u], j[u], (k + u) * 32u)));
+        for (int u = 0; u < kScanUnroll; ++u) {
+            const f32x2 oxy = add2(f32x2{q[u].x}, axy);
+            const float oz = __uint_as_float(uint32_t(q[u].y)) + az;
+            float x2, y2;
+            unpack2(mul2(oxy, oxy), x2, y2);
+            const bool keep = j + u < e && (x2 + y2) + oz * oz < p.reach;
+            if (keep && nf < cap) out[size_t(nf) * 32u] = j + u;
+            nf += keep ? 1u : 0u;
+        }
+    }
+}
+
+// The scan through tables that need bounds checks or a search, out of line: what it would hold in
+// registers stays out of the density pass.
+__device__ __noinline__ uint32_t scan_checked(const Params& p, const GridDev& g, const float4* __restrict__ pts,
+                                              int3 cell, float x, float y, float z, uint32_t* out,
+                                              uint32_t cap) {
+    uint32_t nf = 0;
+    each_near(p, g, pts, cell, x, y, z, [&](uint32_t j, float4) {
+        if (nf < cap) out[size_t(nf) * 32u] = j;
+        ++nf;
+    });
+    return nf;
+}
+
+// Lists the points of `g` within reach of (x, y, z) in the reference's list order (each_near's).
+// Where the table knows which of a cell's 27 cells hold points (GridDev::near, the walls), only those
+// are visited; a cell with its 26 neighbours inside a dense table needs no bounds checks (the world
+// pads the fluid's table so that every particle's has).
+__device__ __forceinline__ uint32_t scan_near(const Params& p, const GridDev& g, const float4* __restrict__ pts,
+                                              int3 cell, float x, float y, float z, uint32_t* out,
+                                              uint32_t cap) {
+    if (g.mode == 0) return 0u;
+    const long long bx = (long long)cell.x - g.lx, by = (long long)cell.y - g.ly, bz = (long long)cell.z - g.lz;
+    const int edge = g.near ? 0 : 1;  // cells that a walk without checks keeps away from the box's faces
+    if (g.mode != 1 || bx < edge || bx + edge >= g.sx || by < edge || by + edge >= g.sy || bz < edge ||
+        bz + edge >= g.sz)
+        return scan_checked(p, g, pts, cell, x, y, z, out, cap);
+    const f32x2 axy = pack2(-x, -y);
+    const float az = -z;
+    const uint32_t slab = uint32_t(g.sy) * uint32_t(g.sz);
+    const uint32_t c0 = (uint32_t(bx) * uint32_t(g.sy) + uint32_t(by)) * uint32_t(g.sz) + uint32_t(bz);
+    uint32_t nf = 0;
+#pragma unroll 1
+    for (uint32_t mask = g.near ? __ldg(&g.near[c0]) : (1u << 27) - 1u; mask; mask &= mask - 1u) {
+        const int t = __ffs(int(mask)) - 1;
+        const uint32_t c = c0 + uint32_t((t % 3 - 1) * int(slab) + (t / 3 % 3 - 1) * g.sz + t / 9 - 1);
+        scan_range(p, pts, __ldg(&g.start[c]), __ldg(&g.start[c + 1]), axy, az, out, cap, nf);
+    }
+    return nf;
+}
+
+// a / radius, rounded as the IEEE division rounds it, without one: with y = RN(1 / r),
+// q = RN(a y), the remainder a - q r is exact in one fma and RN(q + remainder y) is RN(a / r)
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990).  Three
+// operations against the division's ten or so.  The remainder must not underflow: the settings'
+// radius is checked on the host (odd_radius) and numerators under 2^-100 divide.  LOW: whether
+// the numerator may be so small (a distance is 0 or at least 2^-75).
+template <bool LOW>
+__device__ __forceinline__ f32x2 div_radius2(const Params& p, f32x2 a) {
+    const f32x2 y = splat2(p.inv_radius);
+    const f32x2 q = mul2(a, y);
+    f32x2 r = fma2(fma2(splat2(-p.radius), q, a), y, q);
+    bool plain = p.odd_radius != 0u;
+    if (LOW) {
+        float a0, a1;
+        unpack2(a, a0, a1);
+        // 0 < |a| < 2^-100, by the bits (zero wraps round)
+        const uint32_t edge = (127u - 100u) << 23;
+        plain = plain || (__float_as_uint(a0) & 0x7fffffffu) - 1u < edge - 1u ||
+                (__float_as_uint(a1) & 0x7fffffffu) - 1u < edge - 1u;
+    }
+    if (plain) {
+        float a0, a1;
+        unpack2(a, a0, a1);
+        r = pack2(a0 / p.radius, a1 / p.radius);
+    }
+    return r;
+}
+
+// Kernel::value and the gradient factor (kernel_value, kernel_slope / d) of two pairs at squared
+// distances d2, each half the scalar functions' bits.
+__device__ __forceinline__ void kernel_pair(const Params& p, f32x2 d2, f32x2& value, float& g0, float& g1) {
+    float s0, s1;
+    unpack2(d2, s0, s1);
+    const float d0 = sqrtf(s0), d1 = sqrtf(s1);
+    const f32x2 q = div_radius2<false>(p, pack2(d0, d1));
+    const f32x2 one = splat2(1.0f);
+    const f32x2 om = fma2(q, splat2(-1.0f), one);  // 1 - q: the product is exact
+    const f32x2 om2 = mul2(om, om);
+    value = mul2(mul2(splat2(p.scale), mul2(om2, om2)), fma2(splat2(4.0f), q, one));  // 4 q is exact
+    const f32x2 slope = div_radius2<true>(p, mul2(mul2(splat2(p.slope_scale), q), mul2(om, om2)));
+    float l0, l1, q0, q1;
+    unpack2(slope, l0, l1);
+    unpack2(q, q0, q1);
+    g0 = q0 < 1.0f && d0 > 0.0f ? l0 / d0 : 0.0f;
+    g1 = q1 < 1.0f && d1 > 0.0f ? l1 / d1 : 0.0f;
+    if (!(q0 < 1.0f && q1 < 1.0f)) {  // at the very edge: value is zero from there on
+        float v0, v1;
+        unpack2(value, v0, v1);
+        value = pack2(q0 < 1.0f ? v0 : 0.0f, q1 < 1.0f ? v1 : 0.0f);
+    }
+}
+
+// The pair terms over a scanned list: for each of the first m indices in `from` (32 words apart),
+// its entry {index, g} (and, with GRADIENT and room kept for it, its whole gradient G) goes to the
+// row's list, and pair(v, gx, gy, gz) takes the kernel's value and G in list order.  Two pairs run
+// packed, and the next ones' indices are requested before their terms are formed.  (`from` was
+// written by this thread, and is rewritten for its next list: never a read-only load.)
+template <bool GRADIENT, class Pair>
+__device__ __forceinline__ void pair_terms(const Params& p, const PairLists& l, uint32_t row, uint32_t m,
+                                           const uint32_t* from, const float4* __restrict__ pts, float4 a,
+                                           bool walls, Pair&& pair) {
+    constexpr int U = kPairUnroll;
+    static_assert(U % 2 == 0, "pairs run two at a time");
+    if (m == 0) return;
+    uint2* e = l.e + l.at(row, 0);
+    float4* gv = GRADIENT && l.gv ? l.gv + l.at(row, 0) : nullptr;
+    uint32_t j[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) j[u] = next[u];
+    for (int u = 0; u < U; ++u) j[u] = from[size_t(u < (int)m ? u : m - 1) * 32u];
+#pragma unroll 1
+    for (uint32_t k = 0; k < m; k += U) {
+        float4 q[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) q[u] = __ldg(&pts[j[u]]);
+        uint32_t next[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t kk = k + U + u;
+            next[u] = from[size_t(kk < m ? kk : m - 1) * 32u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u += 2) {
+            const f32x2 ox = pack2(q[u].x - a.x, q[u + 1].x - a.x), oy = pack2(q[u].y - a.y, q[u + 1].y - a.y),
+                        oz = pack2(q[u].z - a.z, q[u + 1].z - a.z);
+            f32x2 value;
+            float g[2], v[2];
+            kernel_pair(p, sum2(p, sum2(p, mul2(ox, ox), mul2(oy, oy)), mul2(oz, oz)), value, g[0], g[1]);
+            unpack2(value, v[0], v[1]);
+            float gx[2] = {0.0f, 0.0f}, gy[2] = {0.0f, 0.0f}, gz[2] = {0.0f, 0.0f};
+            if (GRADIENT) {
+                // (at - other) g: both signs of the product turned, the same bits
+                const f32x2 ng = pack2(-g[0], -g[1]);
+                unpack2(mul2(ox, ng), gx[0], gx[1]);
+                unpack2(mul2(oy, ng), gy[0], gy[1]);
+                unpack2(mul2(oz, ng), gz[0], gz[1]);
+            }
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                if (k + u + w < m) {
+                    e[size_t(k + u + w) * 32u] = make_uint2(j[u + w], __float_as_uint(g[w]));
+                    if (GRADIENT && gv)
+                        gv[size_t(k + u + w) * 32u] =
+                            make_float4(gx[w], gy[w], gz[w], walls ? 0.0f : __uint_as_float(j[u + w]));
+                    pair(v[w], gx[w], gy[w], gz[w]);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) j[u] = next[u];
     }
 }
 
@@ -352,84 +530,71 @@ __device__ __forceinline__ uint32_t warp_list_near(const Params& p, const GridDe
 // (step.rs:147-172) or the DFSPH factors (dfsph.rs:108-163) --------------------------------
 
 // four blocks a SM (64 registers), as the pass compiled before it strode over rows
-template <int SOLVER>
-__global__ void __launch_bounds__(kBlock, 4) k_density(Params p, GridDev fg, GridDev wg, const float4* __restrict__ pos,
-                                                    const float4* __restrict__ walls, PairLists fl, PairLists wl,
-                                                    float* __restrict__ rho, float* __restrict__ press,
-                                                    float* __restrict__ scaled, float* __restrict__ alpha, Status* st,
-                                                    TerrainDev T, float4* __restrict__ slope, MoverDev M) {
+// What the pass lists: the fluid (0), then the walls (1).
+struct DensityIn {
+    GridDev grid[2];
+    const float4* pts[2];
+    PairLists list[2];
+};
+
+// EXTRA: terrain regions or coupled bodies add their terms
+template <int SOLVER, bool EXTRA>
+__global__ void __launch_bounds__(kBlock, 4)
+    k_density(const __grid_constant__ Params p, const __grid_constant__ DensityIn in, float* __restrict__ rho,
+              float* __restrict__ press, float* __restrict__ scaled, float* __restrict__ alpha, Status* st, TerrainDev T,
+              float4* __restrict__ slope, MoverDev M, uint32_t* scratch) {
     uint32_t compressed = 0, longest = 0;
+    const float4* __restrict__ pos = in.pts[0];
+    // this warp's unfinished list, entry k of a lane at k * 32: the same few megabytes for every row
+    // the grid strides to, so the scan's stores stay in the L2 and only finished entries go to DRAM
+    uint32_t* const idx = scratch + size_t(blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)) * 32u * in.list[0].cap +
+                          (threadIdx.x & 31u);
     // rows of the walk order, a grid's width apart (one each when the grid covers them all)
     for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < p.n; row += gridDim.x * blockDim.x) {
-        const uint32_t i = fl.particle(row);
+        const uint32_t i = in.list[0].particle(row);
         float4 a = pos[i];
         int3 cell = cell_of(p, a.x, a.y, a.z);
         // The walk first only lists the neighbours (a tight loop over the ~216 candidates of 27
         // cells, of which ~16 % are kept), then takes the sums over the list, in list order, so
         // the arithmetic of the kept pairs runs without the candidates' divergence.  A list over
         // its room is incomplete and the host runs the pass again with more room.
-        uint32_t nf = 0, nw = 0;
-        each_near(p, fg, pos, cell, a.x, a.y, a.z, [&](uint32_t j, float4) {
-            if (nf < fl.cap) fl.e[fl.at(row, nf)].x = j;
-            ++nf;
-        });
-        each_near(p, wg, walls, cell, a.x, a.y, a.z, [&](uint32_t j, float4) {
-            if (nw < wl.cap) wl.e[wl.at(row, nw)].x = j;
-            ++nw;
-        });
-        fl.count[row] = nf;
-        wl.count[row] = nw;
-        longest = max(longest, nf > nw ? nf : nw);
-        float sum = 0.0f, wsum = 0.0f;
-        float sx = 0.0f, sy = 0.0f, sz = 0.0f, squares = 0.0f;
-        float4* const fgv = fl.gv ? fl.gv + fl.at(row, 0) : nullptr;
-        float4* const wgv = wl.gv ? wl.gv + wl.at(row, 0) : nullptr;
-        relist(fl, row, nf < fl.cap ? nf : fl.cap, pos, [&](float4 q, uint32_t j, uint32_t at) {
-            float ox = q.x - a.x, oy = q.y - a.y, oz = q.z - a.z;
-            float d = sqrtf(dot3(ox, oy, oz, ox, oy, oz));
-            sum += kernel_value(p, d);
-            float g = d <= 0.0f ? 0.0f : kernel_slope(p, d) / d;
-            if (SOLVER == 1) {
-                // gradient(at - other) (dfsph.rs:118), then factors (dfsph.rs:149-153)
-                float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
-                float gx = rx * g, gy = ry * g, gz = rz * g;
-                if (fgv) fgv[at] = make_float4(gx, gy, gz, __uint_as_float(j));
-                float px = gx * p.mass, py = gy * p.mass, pz = gz * p.mass;
-                sx = sx + px;
-                sy = sy + py;
-                sz = sz + pz;
-                squares += dot3(px, py, pz, px, py, pz);
-            }
-            return g;
-        });
-        relist(wl, row, nw < wl.cap ? nw : wl.cap, walls, [&](float4 q, uint32_t, uint32_t at) {
-            float ox = q.x - a.x, oy = q.y - a.y, oz = q.z - a.z;
-            float d = sqrtf(dot3(ox, oy, oz, ox, oy, oz));
-            wsum += kernel_value(p, d);
-            float g = d <= 0.0f ? 0.0f : kernel_slope(p, d) / d;
-            if (SOLVER == 1) {
-                float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
-                float gx = rx * g, gy = ry * g, gz = rz * g;
-                if (wgv) wgv[at] = make_float4(gx, gy, gz, 0.0f);
-                sx = sx + gx * p.mass;
-                sy = sy + gy * p.mass;
-                sz = sz + gz * p.mass;
-            }
-            return g;
-        });
+        float sums[2], sx = 0.0f, sy = 0.0f, sz = 0.0f, squares = 0.0f;
+#pragma unroll 1
+        for (int w = 0; w < 2; ++w) {  // the fluid, then the walls
+            const PairLists& l = in.list[w];
+            const float4* __restrict__ pts = in.pts[w];
+            const uint32_t found = scan_near(p, in.grid[w], pts, cell, a.x, a.y, a.z, idx, l.cap);
+            l.count[row] = found;
+            longest = max(longest, found);
+            float sum = 0.0f;
+            pair_terms<SOLVER == 1>(p, l, row, found < l.cap ? found : l.cap, idx, pts, a, w == 1,
+                                    [&](float v, float gx, float gy, float gz) {
+                                        sum += v;
+                                        if (SOLVER == 1) {  // factors (dfsph.rs:149-153); walls add no squares
+                                            float px = gx * p.mass, py = gy * p.mass, pz = gz * p.mass;
+                                            sx = sx + px;
+                                            sy = sy + py;
+                                            sz = sz + pz;
+                                            squares += w == 0 ? dot3(px, py, pz, px, py, pz) : 0.0f;
+                                        }
+                                    });
+            sums[1] = sum;
+            if (w == 0) sums[0] = sum;
+        }
+        const float sum = sums[0], wsum = sums[1];
         // the coupled bodies' points, in their list order (mod.rs:648-656)
         float msum = 0.0f;
-        if (M.count)
+        if (EXTRA && M.count)
             each_near(p, M.grid, M.pos, cell, a.x, a.y, a.z, [&](uint32_t, float4 q) {
                 float ox = q.x - a.x, oy = q.y - a.y, oz = q.z - a.z;
                 msum += kernel_value(p, sqrtf(dot3(ox, oy, oz, ox, oy, oz)));
             });
         // mass (fluid + walls + body points) + ground (mod.rs:657-663)
-        float3 gslope;
-        float ground = T.regions ? ground_near(T, a.x, a.y, a.z, gslope) : 0.0f;
+        float3 gslope = make_float3(0.0f, 0.0f, 0.0f);
+        float ground = EXTRA && T.regions ? ground_near(T, a.x, a.y, a.z, gslope) : 0.0f;
         float density = p.mass * (sum + wsum + msum) + ground;
         rho[i] = density;
-        if (slope) slope[i] = make_float4(gslope.x, gslope.y, gslope.z, 0.0f);
+        if (EXTRA && slope) slope[i] = make_float4(gslope.x, gslope.y, gslope.z, 0.0f);
         if (SOLVER == 0) {
             float ratio = fminf(density / p.rest, 1.1f);
             float pressure = fmaxf(p.stiffness * (pow7(ratio) - 1.0f), 0.0f);
@@ -1698,8 +1863,8 @@ void prepare_solver_grids() {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0], k_rate<0>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1], k_rate<1>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[2], k_push, kBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[3], k_density<0>, kBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[4], k_density<1>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[3], k_density<0, true>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[4], k_density<1, false>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[5], k_viscous, kBlock, 0);
     for (int k = 0; k < 6; ++k) g_resident[k].store(uint32_t(std::max(per[k], 0) * std::max(sms, 0)));
 }
@@ -1731,6 +1896,11 @@ void launch_count_cells(const Params& p, const float4* pos, const int4* cells, i
     if (p.n) k_count_cells<<<blocks_for(p.n), kBlock, 0, s>>>(p, pos, cells, low, span, count, lin, slot);
 }
 
+void launch_grid_near(const GridDev& g, uint32_t* near, cudaStream_t s) {
+    const uint32_t volume = uint32_t(g.sx) * uint32_t(g.sy) * uint32_t(g.sz);
+    if (g.mode == 1 && volume) k_grid_near<<<blocks_for(volume), kBlock, 0, s>>>(g, near);
+}
+
 size_t scan_tiles(uint32_t m) { return (m + kScanTile - 1) / kScanTile; }
 
 void launch_exclusive_scan(uint32_t* data, uint32_t m, uint32_t* tile_sums, cudaStream_t s) {
@@ -1760,9 +1930,17 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
                                                         skip_begin, skip_end, st, dest);
 }
 
+size_t density_scratch_words(uint32_t n, uint32_t cap) {
+    // one list room a thread of the density pass's grid
+    const uint32_t nb = (n + kBlock - 1) / kBlock, r0 = g_resident[3].load(), r1 = g_resident[4].load();
+    const uint32_t resident = r0 && r1 ? std::max(r0, r1) : nb;
+    return size_t(std::min(resident, nb)) * kBlock * cap;
+}
+
 void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, const float4* pos, const float4* walls,
                     const PairLists& fl, const PairLists& wl, float* rho, float* press, float* scaled, float* alpha,
-                    Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M) {
+                    Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M,
+                    uint32_t* scratch) {
     if (!p.n) return;
     if (warp_rows(p.n, p.radius, p.spacing) && T.regions == 0 && M.count == 0) {
         // a scene this small leaves most SMs idle a thread a particle: a warp a particle (terrain
@@ -1775,12 +1953,14 @@ void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, const
                                                                        scaled, alpha, st, T, slope, M);
         return;
     }
-    if (p.solver == 0)
-        k_density<0><<<solver_blocks(p.n, 3), kBlock, 0, s>>>(p, fg, wg, pos, walls, fl, wl, rho, press, scaled, alpha, st,
-                                                        T, slope, M);
+    const uint32_t nb = solver_blocks(p.n, p.solver == 0 ? 3 : 4);
+    const DensityIn in{{fg, wg}, {pos, walls}, {fl, wl}};
+    if (p.solver != 0)  // DFSPH takes neither terrain nor bodies
+        k_density<1, false><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch);
+    else if (T.regions || M.count || slope)
+        k_density<0, true><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch);
     else
-        k_density<1><<<solver_blocks(p.n, 4), kBlock, 0, s>>>(p, fg, wg, pos, walls, fl, wl, rho, press, scaled, alpha, st,
-                                                        T, slope, M);
+        k_density<0, false><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch);
 }
 
 void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,

@@ -17,6 +17,8 @@ void launch_max_compression(const Params& p, const float* rho, Status* st, cudaS
 // counting sort by dense cell index; cells (cell-relative positions) optional
 void launch_count_cells(const Params& p, const float4* pos, const int4* cells, int3 low, int3 span, uint32_t* count,
                         uint32_t* lin, uint32_t* slot, cudaStream_t s);
+// a dense table's masks (GridDev::near), one word a cell
+void launch_grid_near(const GridDev& g, uint32_t* near, cudaStream_t s);
 size_t scan_tiles(uint32_t m);
 // exclusive scan of data[0, m) in place; data[m] receives the total.  tile_sums holds
 // scan_tiles(m) + 1 entries.
@@ -57,7 +59,10 @@ void launch_walk_order(uint32_t volume, int3 span, const uint32_t* start, uint32
 // T: terrain regions (regions = 0: none); slope (optional): each particle's ground density gradient
 void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, const float4* pos, const float4* walls,
                     const PairLists& fl, const PairLists& wl, float* rho, float* press, float* scaled, float* alpha,
-                    Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M = MoverDev{});
+                    Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M,
+                    uint32_t* scratch);
+// words of launch_density's scratch for n particles and lists of cap slots
+size_t density_scratch_words(uint32_t n, uint32_t cap);
 // vel_pre (optional): the velocity before the wall clamp, its w lane the bits of the components
 // the clamp zeroed (1 x, 2 y, 4 z), for the adjoint
 void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,

@@ -351,6 +351,7 @@ struct World {
     // EXACT DFSPH: each pair's kernel gradient at the same slots (PairLists::gv), for the check
     DevBuf<float4> fgv, wgv;
     DevBuf<uint32_t> fcnt, wcnt;
+    DevBuf<uint32_t> dscratch;  // the EXACT density pass's unfinished lists (density_scratch_words)
     uint32_t list_cap = 0;
     DevBuf<uint8_t> partials;
     bool stats_fresh = false;  // status holds bbox and speed of the committed state
@@ -373,6 +374,7 @@ struct World {
     DevBuf<float4> dwalls;
     DevBuf<uint32_t> dwstart;
     DevBuf<int4> dwkeys;
+    DevBuf<uint32_t> dwnear;  // dense walls: which of the 27 cells around each cell hold points
     GridDev wgrid{};
     bool walls_dirty = true;
 
@@ -553,7 +555,7 @@ struct World {
     ~World() {
         if (stream) {
             for (auto* b : {&pos[0], &pos[1], &pos[2], &vel[0], &vel[1], &vel[2]}) b->release(stream);
-            for (auto* b : {&ids[0], &ids[1], &lin, &cslot, &members, &count, &tiles, &keep, &dwstart, &fcnt, &wcnt,
+            for (auto* b : {&ids[0], &ids[1], &lin, &cslot, &members, &count, &tiles, &keep, &dwstart, &dwnear, &fcnt, &wcnt, &dscratch,
                             &worder, &wkeys, &wsums, &etaken, &etiles})
                 b->release(stream);
             for (auto* b : {&rho[0], &rho[1], &press, &scaled, &alpha}) b->release(stream);
@@ -835,8 +837,10 @@ struct World {
 
     // The cell table of points sorted by cell (keys in order, m = keys.size()): dense over their
     // box while it holds at most 64 cells per occupied one plus 4096 (mod.rs:214-216), else the
-    // occupied cells for search; uploaded into dstart / dkeys, described by g.
-    int32_t grid_from_keys(const std::vector<Key3>& keys, GridDev& g, DevBuf<uint32_t>& dstart, DevBuf<int4>& dkeys);
+    // occupied cells for search; uploaded into dstart / dkeys, described by g.  dnear (optional):
+    // takes a dense table's masks (GridDev::near).
+    int32_t grid_from_keys(const std::vector<Key3>& keys, GridDev& g, DevBuf<uint32_t>& dstart, DevBuf<int4>& dkeys,
+                           DevBuf<uint32_t>* dnear = nullptr);
 
     // Uploads the walls and their cell table: dense over the walls' box while it holds at most 64
     // cells per occupied one plus 4096 (mod.rs:214-216), else the occupied cells for search.

@@ -213,6 +213,9 @@ Params World::params() const {
     p.grad_scale = scale * -20.0f / (radius * radius);
     p.inv_rest = 1.0f / s.rest_density;
     p.inv_rest_sq = 1.0f / (s.rest_density * s.rest_density);
+    p.slope_scale = scale * -20.0f;
+    p.one = 1.0f;
+    p.odd_radius = radius >= 1.220703125e-4f && radius <= 1024.0f ? 0u : 1u;
     p.settles = std::sqrt(s.gravity[0] * s.gravity[0] + s.gravity[1] * s.gravity[1] + s.gravity[2] * s.gravity[2]) *
                 s.spacing;
     return p;
@@ -339,6 +342,7 @@ int32_t World::ensure_work_buffers() {
     SLF_TRY(cslot.ensure(n, 0, stream));
     SLF_TRY(members.ensure(n, 0, stream));
     SLF_TRY(partials.ensure(rate_partial_bytes(uint32_t(n)), 0, stream));
+    if (!fast()) SLF_TRY(dscratch.ensure(density_scratch_words(uint32_t(n), list_cap), 0, stream));
     return SLF_OK;
 }
 
@@ -349,7 +353,7 @@ void World::density_pass(const Params& p, int a, const PairLists& fl, const Pair
                             alpha.p, d_status, on);
     else
         launch_density(p, fgrid, wgrid, pos[a].p, dwalls.p, fl, wl, rh, press.p, scaled.p, alpha.p, d_status,
-                       tdev, ground_slopes(), on, mover_dev());
+                       tdev, ground_slopes(), on, mover_dev(), dscratch.p);
 }
 
 void World::force_pass(const Params& p, const PairLists& fl, const PairLists& wl, int a, int b, int nid, cudaStream_t on) {
@@ -462,6 +466,22 @@ int32_t World::plan_sort(SortPlan& sp, bool stable) {
             for (int a = 0; a < 3; ++a) {
                 lo[a] = wl[a];
                 hi[a] = wh[a];
+            }
+    }
+    // an empty cell around the box, where the table still fits: every particle's 27 cells then lie
+    // inside it, and the density scan needs no bounds checks (cell order does not depend on the box)
+    {
+        int64_t pl[3], ph[3];
+        bool inside = true;
+        for (int a = 0; a < 3; ++a) {
+            pl[a] = lo[a] - 1;
+            ph[a] = hi[a] + 1;
+            inside = inside && pl[a] >= INT32_MIN && ph[a] <= INT32_MAX;
+        }
+        if (inside && fits(volume_of(pl, ph)))
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = pl[a];
+                hi[a] = ph[a];
             }
     }
     __int128 vol = volume_of(lo, hi);

@@ -231,7 +231,7 @@ void World::drop_substep_graphs() {
 }
 
 std::vector<uint8_t> World::substep_key(const Params& p, int a, int b, int nid, const SortPlan& sp) {
-    static_assert(sizeof(GridDev) == 48, "GridDev has no padding");
+    static_assert(sizeof(GridDev) == 56, "GridDev has no padding");
     std::vector<uint8_t> k;
     key_add(k, int32_t(s.solver));
     key_add(k, int32_t(fast()));
@@ -252,7 +252,8 @@ std::vector<uint8_t> World::substep_key(const Params& p, int a, int b, int nid, 
              pos[cpos].p, vel[cpos].p, cells_of(cpos), ids[cid].p, ids[nid].p, rho[cid].p, rho[nid].p,
              pos[a].p, vel[a].p, cells_of(a), pos[b].p, vel[b].p, cells_of(b), warm_in(), warm_out(),
              sort_dest, count.p, tiles.p, lin.p, cslot.p, members.p, worder.p, wkeys.p, wsums.p, press.p,
-             scaled.p, alpha.p, dwalls.p, partials.p, d_status, d_consts, vel_pre, h_reset})
+             scaled.p, alpha.p, dwalls.p, partials.p, d_status, d_consts, vel_pre, h_reset,
+             dscratch.p})
         key_add(k, q);
     return k;
 }

@@ -151,7 +151,8 @@ void World::settle_walls() {
     walls_dirty = true;
 }
 
-int32_t World::grid_from_keys(const std::vector<Key3>& keys, GridDev& g, DevBuf<uint32_t>& dstart, DevBuf<int4>& dkeys) {
+int32_t World::grid_from_keys(const std::vector<Key3>& keys, GridDev& g, DevBuf<uint32_t>& dstart, DevBuf<int4>& dkeys,
+                              DevBuf<uint32_t>* dnear) {
     g = GridDev{};
     size_t m = keys.size();
     if (m == 0) return SLF_OK;
@@ -194,6 +195,11 @@ int32_t World::grid_from_keys(const std::vector<Key3>& keys, GridDev& g, DevBuf<
         g.sy = int(sy);
         g.sz = int(sz);
         g.start = dstart.p;
+        if (dnear) {
+            SLF_TRY(dnear->ensure(volume, 0, stream));
+            launch_grid_near(g, dnear->p, stream);
+            g.near = dnear->p;
+        }
         SLF_CUDA(cudaStreamSynchronize(stream));
     } else {
         std::vector<int4> k4(cells.size());
@@ -234,7 +240,7 @@ int32_t World::upload_walls() {
     }
     SLF_TRY(dwalls.ensure(m, 0, stream));
     SLF_CUDA(cudaMemcpyAsync(dwalls.p, w.data(), m * sizeof(float4), cudaMemcpyHostToDevice, stream));
-    SLF_TRY(grid_from_keys(keys, wgrid, dwstart, dwkeys));
+    SLF_TRY(grid_from_keys(keys, wgrid, dwstart, dwkeys, &dwnear));
     walls_dirty = false;
     return SLF_OK;
 }
