@@ -81,9 +81,18 @@ __global__ void k_max_compression(Params p, const float* __restrict__ rho, Statu
 // ---- spatial hash: counting sort by dense cell index, then id within each cell ------------
 
 // cells (cell-relative positions) non-null: the cell is stored, not computed
+// begin (a substep recorded as a graph): the status starts afresh, and the substep's constants come
+// from the host's copy, which it writes before each launch of the graph
 __global__ void k_count_cells(Params p, const float4* __restrict__ pos, const int4* __restrict__ cells, int3 low,
-                              int3 span, uint32_t* count, uint32_t* lin, uint32_t* slot) {
+                              int3 span, uint32_t* count, uint32_t* lin, uint32_t* slot, SubstepBegin begin) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (begin.status && i == 0) {
+        Status z{};
+        z.cell_lo[0] = z.cell_lo[1] = z.cell_lo[2] = INT_MAX;
+        z.cell_hi[0] = z.cell_hi[1] = z.cell_hi[2] = INT_MIN;
+        *begin.status = z;
+        *begin.consts = *begin.from;
+    }
     if (i >= p.n) return;
     int3 c;
     if (cells) {
@@ -127,8 +136,44 @@ __global__ void k_scatter_members(uint32_t n, const uint32_t* __restrict__ lin, 
     members[start[lin[i]] + slot[i]] = ids[i];
 }
 
+// ---- the walk order of the list passes (PairLists::order) -------------------------------------
+// Cells taken in 2 x 2-column bricks whose z is split in quads, key = ((x / 2, y / 2), z / 4, x % 2,
+// y % 2, z % 4): 256 consecutive rows cover about 2 x 2 x 8 cells instead of a 1 x 1 x 32 column,
+// and a warp's 32 rows are (about) four consecutive cells of one column, whose neighbours lie in
+// consecutive cells of the same neighbouring columns.
+//
+// The row of cell (x, y, z)'s first member needs no scan over the keys: the particles are sorted
+// x-major, so the members of any run of cells along z, or of a run of columns along y, are one
+// difference of the cell table.  Before the cell come the slab pairs before its own, the bricks
+// before its own in the slab pair, the quads before its own in the four columns, the columns
+// before its own in the quad, and the cells before it in its column.  A dozen loads from the table's
+// cache lines in k_rank_reorder (17 -> 21 us at 1M) in place of a count, a scan and a fill of the
+// keys (six nodes, 30 us at 1M and 26 at 75k).
+__device__ __forceinline__ uint32_t walk_row(const uint32_t* __restrict__ start, int3 span, uint32_t lin) {
+    const uint32_t sy = uint32_t(span.y), sz = uint32_t(span.z);
+    const uint32_t z = lin % sz, y = lin / sz % sy, x = lin / sz / sy;
+    const uint32_t x0 = x & ~1u, y0 = y & ~1u, z0 = z & ~3u, z1 = min(z0 + 4u, sz);
+    uint32_t row = __ldg(&start[x0 * sy * sz]);
+#pragma unroll
+    for (uint32_t dx = 0; dx < 2; ++dx) {
+        if (x0 + dx >= uint32_t(span.x)) continue;
+        const uint32_t slab = (x0 + dx) * sy * sz;
+        row += __ldg(&start[slab + y0 * sz]) - __ldg(&start[slab]);
+#pragma unroll
+        for (uint32_t dy = 0; dy < 2; ++dy) {
+            if (y0 + dy >= sy) continue;
+            const uint32_t column = slab + (y0 + dy) * sz;
+            // columns before the cell's own in the quad count whole quads up to this one
+            const uint32_t upto = 2u * dx + dy < (x & 1u) * 2u + (y & 1u) ? z1 : z0;
+            row += __ldg(&start[column + upto]) - __ldg(&start[column]);
+        }
+    }
+    return row + __ldg(&start[lin]) - __ldg(&start[lin - z + z0]);
+}
+
 // Final place = cell start + number of the cell's ids below this one's: the (cell, id) order
-// of mod.rs:550, whatever order the atomics handed out the slots in.
+// of mod.rs:550, whatever order the atomics handed out the slots in.  order (optional): the walk
+// order's row of each particle, its cell's row and its rank in the cell.
 __global__ void k_rank_reorder(uint32_t n, const uint32_t* __restrict__ lin, const uint32_t* __restrict__ start,
                                const uint32_t* __restrict__ members, const uint32_t* __restrict__ ids_in,
                                const float4* __restrict__ pos_in, const float4* __restrict__ vel_in,
@@ -137,20 +182,22 @@ __global__ void k_rank_reorder(uint32_t n, const uint32_t* __restrict__ lin, con
                                float4* __restrict__ vel_out, float* __restrict__ rho_out,
                                int4* __restrict__ cells_out, const float2* __restrict__ warm_in,
                                float2* __restrict__ warm_out, uint32_t skip_begin, uint32_t skip_end, Status* st,
-                               uint32_t* __restrict__ dest) {
+                               uint32_t* __restrict__ dest, int3 span, uint32_t* __restrict__ order) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     // a job left undone (the fault injection of the dispatcher tests) places nothing; the count
     // of placed particles tells the host whether every particle was placed
     bool work = i < n && !(i >= skip_begin && i < skip_end);
     uint32_t placed = block_reduce(work ? 1u : 0u, SumU(), 0u);
     if (threadIdx.x == 0 && placed) atomicAdd(&st->processed, placed);
-    if (!work) return;
+    if (i >= n) return;
     uint32_t l = lin[i];
     uint32_t b = start[l], e = start[l + 1];
     uint32_t id = ids_in[i];
     uint32_t rank = 0;
     for (uint32_t k = b; k < e; ++k) rank += members[k] < id ? 1u : 0u;
     uint32_t f = b + rank;
+    if (order) order[walk_row(start, span, l) + rank] = f;  // every row, a skipped job's too
+    if (!work) return;
     if (dest) dest[i] = f;  // where each particle went, for the adjoint's way back
     ids_out[f] = id;
     pos_out[f] = pos_in[i];
@@ -164,6 +211,8 @@ __global__ void k_rank_reorder(uint32_t n, const uint32_t* __restrict__ lin, con
 
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kBlock * kScanItems;
+// tiles up to which each tile adds up its predecessors' sums itself (up to eight loads a thread)
+constexpr uint32_t kScanOwnSums = 2048;
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total) {
     __shared__ uint32_t warp_sums[kBlock / 32];
@@ -192,23 +241,68 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
     return warp_prefix + x - v;
 }
 
-__global__ void k_scan_tiles(uint32_t* data, uint32_t m, uint32_t* tile_sums) {
-    uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
+// this thread's kScanItems of a tile at `base`; wide: the data is 16-byte aligned
+__device__ __forceinline__ void scan_load(const uint32_t* data, uint32_t base, uint32_t m, bool wide,
+                                          uint32_t (&v)[kScanItems]) {
+    if (wide && base + kScanItems <= m) {
+        const uint4 a = *reinterpret_cast<const uint4*>(data + base), b = *reinterpret_cast<const uint4*>(data + base + 4);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) v[k] = base + k < m ? data[base + k] : 0u;
+}
+__device__ __forceinline__ void scan_store(uint32_t* data, uint32_t base, uint32_t m, bool wide,
+                                           const uint32_t (&v)[kScanItems]) {
+    if (wide && base + kScanItems <= m) {
+        *reinterpret_cast<uint4*>(data + base) = make_uint4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<uint4*>(data + base + 4) = make_uint4(v[4], v[5], v[6], v[7]);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k)
+        if (base + k < m) data[base + k] = v[k];
+}
+
+__global__ void k_scan_tiles(uint32_t* data, uint32_t m, uint32_t* tile_sums, int wide) {
+    const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    uint32_t v[kScanItems], out[kScanItems];
+    scan_load(data, base, m, wide != 0, v);
     uint32_t sum = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        v[k] = base + k < m ? data[base + k] : 0u;
-        sum += v[k];
-    }
+    for (int k = 0; k < kScanItems; ++k) sum += v[k];
     uint32_t total;
     uint32_t prefix = block_exclusive_scan(sum, &total);
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
-        if (base + k < m) data[base + k] = prefix;
+        out[k] = prefix;
         prefix += v[k];
     }
-    if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+    scan_store(data, base, m, wide != 0, out);
+    if (threadIdx.x == 0) {
+        tile_sums[blockIdx.x] = total;
+        if (gridDim.x == 1) data[m] = total;
+    }
+}
+
+// Each tile adds up the sums of the tiles before it by itself (few enough of them that reading
+// them again costs less than a launch that scans them) and adds that to its items: the scan 15.6
+// -> 11 us at 1M (138 tiles), and 12 -> 6.5 where one tile holds the table.
+__global__ void k_scan_finish(uint32_t* data, uint32_t m, const uint32_t* __restrict__ tile_sums, int wide) {
+    __shared__ uint32_t before_s;
+    uint32_t before = 0;
+    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kBlock) before += tile_sums[t];
+    before = block_reduce(before, SumU(), 0u);
+    if (threadIdx.x == 0) before_s = before;
+    __syncthreads();
+    before = before_s;
+    const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    uint32_t v[kScanItems];
+    scan_load(data, base, m, wide != 0, v);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) v[k] += before;
+    scan_store(data, base, m, wide != 0, v);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) data[m] = before + tile_sums[blockIdx.x];
 }
 
 // One block scans the tile sums (any count) in place.
@@ -1579,45 +1673,6 @@ __global__ void k_list_fill(Params p, GridDev g, const float4* __restrict__ pos,
     each_near(p, g, pts, cell, a.x, a.y, a.z, [&](uint32_t j, float4) { items[k++] = j; });
 }
 
-// ---- the walk order of the list passes (PairLists::order) -------------------------------------
-// Cells taken in 2 x 2-column bricks, so 256 consecutive rows cover about 2 x 2 x 8 cells instead
-// of a 1 x 1 x 32 column.  SLF_WALK_ZQUAD 0: key = ((x / 2, y / 2), z, x % 2, y % 2); 1: the
-// brick's z split in quads, key = ((x / 2, y / 2), z / 4, x % 2, y % 2, z % 4), so a warp's 32
-// rows are (about) four consecutive cells of one column, whose neighbours lie in consecutive
-// cells of the same neighbouring columns: a warp's gathers touch fewer cache lines.
-#ifndef SLF_WALK_ZQUAD
-#define SLF_WALK_ZQUAD 1
-#endif
-
-__host__ __device__ __forceinline__ uint32_t walk_quads(int z) { return SLF_WALK_ZQUAD ? (uint32_t(z) + 3u) / 4u : uint32_t(z); }
-
-__device__ __forceinline__ uint32_t brick_key(uint32_t lin, int3 span) {
-    uint32_t z = lin % (uint32_t)span.z, xy = lin / (uint32_t)span.z;
-    uint32_t y = xy % (uint32_t)span.y, x = xy / (uint32_t)span.y;
-    uint32_t by = ((uint32_t)span.y + 1u) / 2u;
-    if (SLF_WALK_ZQUAD)
-        return ((((x >> 1) * by + (y >> 1)) * walk_quads(span.z) + (z >> 2)) * 4u + (x & 1u) * 2u + (y & 1u)) * 4u +
-               (z & 3u);
-    return (((x >> 1) * by + (y >> 1)) * (uint32_t)span.z + z) * 4u + (x & 1u) * 2u + (y & 1u);
-}
-
-// bcount[key(cell)] = members of the cell (bcount cleared beforehand: keys of the padding stay 0)
-__global__ void k_brick_count(uint32_t volume, int3 span, const uint32_t* __restrict__ start,
-                              uint32_t* __restrict__ bcount) {
-    uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= volume) return;
-    bcount[brick_key(c, span)] = start[c + 1] - start[c];
-}
-
-// each cell's members, contiguous in the sorted arrays, go to the rows its key's scan names
-__global__ void k_brick_fill(uint32_t volume, int3 span, const uint32_t* __restrict__ start,
-                             const uint32_t* __restrict__ bstart, uint32_t* __restrict__ order) {
-    uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= volume) return;
-    uint32_t b = start[c], e = start[c + 1], r = bstart[brick_key(c, span)];
-    for (uint32_t m = b; m < e; ++m) order[r + (m - b)] = m;
-}
-
 // ---- domain (mod.rs:451-486): keep flags, then a stable compaction -------------------------
 
 // The f32 position the readouts give: cell-relative ones rebuilt in double and rounded once.
@@ -1892,8 +1947,8 @@ void launch_max_compression(const Params& p, const float* rho, Status* st, cudaS
 }
 
 void launch_count_cells(const Params& p, const float4* pos, const int4* cells, int3 low, int3 span, uint32_t* count,
-                        uint32_t* lin, uint32_t* slot, cudaStream_t s) {
-    if (p.n) k_count_cells<<<blocks_for(p.n), kBlock, 0, s>>>(p, pos, cells, low, span, count, lin, slot);
+                        uint32_t* lin, uint32_t* slot, cudaStream_t s, SubstepBegin begin) {
+    if (p.n) k_count_cells<<<blocks_for(p.n), kBlock, 0, s>>>(p, pos, cells, low, span, count, lin, slot, begin);
 }
 
 void launch_grid_near(const GridDev& g, uint32_t* near, cudaStream_t s) {
@@ -1905,9 +1960,15 @@ size_t scan_tiles(uint32_t m) { return (m + kScanTile - 1) / kScanTile; }
 
 void launch_exclusive_scan(uint32_t* data, uint32_t m, uint32_t* tile_sums, cudaStream_t s) {
     if (m == 0) return;
-    uint32_t tiles = (uint32_t)scan_tiles(m);
-    g_launches.fetch_add(3, std::memory_order_relaxed);
-    k_scan_tiles<<<tiles, kBlock, 0, s>>>(data, m, tile_sums);
+    const uint32_t tiles = (uint32_t)scan_tiles(m);
+    const int wide = (reinterpret_cast<uintptr_t>(data) & 15u) == 0;
+    k_scan_tiles<<<tiles, kBlock, 0, s>>>(data, m, tile_sums, wide);
+    g_launches.fetch_add(tiles == 1 ? 1 : tiles <= kScanOwnSums ? 2 : 3, std::memory_order_relaxed);
+    if (tiles == 1) return;
+    if (tiles <= kScanOwnSums) {
+        k_scan_finish<<<tiles, kBlock, 0, s>>>(data, m, tile_sums, wide);
+        return;
+    }
     k_scan_sums<<<1, kBlock, 0, s>>>(tile_sums, tiles);
     k_scan_add<<<tiles, kBlock, 0, s>>>(data, m, tile_sums);
 }
@@ -1921,13 +1982,12 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
                          const uint32_t* ids_in, const float4* pos_in, const float4* vel_in, const float* rho_in,
                          const int4* cells_in, uint32_t* ids_out, float4* pos_out, float4* vel_out, float* rho_out,
                          int4* cells_out, const float2* warm_in, float2* warm_out, uint32_t skip_begin,
-                         uint32_t skip_end, Status* st, uint32_t* dest,
-                         cudaStream_t s) {
+                         uint32_t skip_end, Status* st, uint32_t* dest, int3 span, uint32_t* order, cudaStream_t s) {
     if (n)
         k_rank_reorder<<<blocks_for(n), kBlock, 0, s>>>(n, lin, start, members, ids_in, pos_in, vel_in, rho_in,
                                                         cells_in, ids_out, pos_out, vel_out, rho_out, cells_out,
                                                         warm_in, warm_out,
-                                                        skip_begin, skip_end, st, dest);
+                                                        skip_begin, skip_end, st, dest, span, order);
 }
 
 size_t density_scratch_words(uint32_t n, uint32_t cap) {
@@ -2083,20 +2143,6 @@ __global__ void k_warm_kappa(Params p, const StepConsts* __restrict__ sc, float 
 
 void launch_warm_kappa(const Params& p, const StepConsts* sc, float share, float* applied, float4* pos, cudaStream_t s) {
     if (p.n) k_warm_kappa<<<blocks_for(p.n), kBlock, 0, s>>>(p, sc, share, applied, pos);
-}
-
-size_t walk_order_keys(int3 span) {
-    return size_t((span.x + 1) / 2) * size_t((span.y + 1) / 2) * size_t(walk_quads(span.z)) * (SLF_WALK_ZQUAD ? 16u : 4u);
-}
-
-void launch_walk_order(uint32_t volume, int3 span, const uint32_t* start, uint32_t* bcount, uint32_t* tile_sums,
-                       uint32_t* order, cudaStream_t s) {
-    if (!volume) return;
-    size_t keys = walk_order_keys(span);
-    cudaMemsetAsync(bcount, 0, (keys + 1) * sizeof(uint32_t), s);
-    k_brick_count<<<blocks_for(volume), kBlock, 0, s>>>(volume, span, start, bcount);
-    launch_exclusive_scan(bcount, uint32_t(keys), tile_sums, s);
-    k_brick_fill<<<blocks_for(volume), kBlock, 0, s>>>(volume, span, start, bcount, order);
 }
 
 void launch_viscous(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl, const float4* pos,

@@ -14,9 +14,17 @@ namespace slf {
 void launch_state_stats(const Params& p, const float4* pos, const float4* vel, Status* st, cudaStream_t s);
 void launch_max_compression(const Params& p, const float* rho, Status* st, cudaStream_t s);
 
+// What the first kernel of a recorded substep sets (status null: nothing): the status afresh, and the
+// constants from the host's pinned copy.
+struct SubstepBegin {
+    Status* status;
+    StepConsts* consts;
+    const StepConsts* from;
+};
+
 // counting sort by dense cell index; cells (cell-relative positions) optional
 void launch_count_cells(const Params& p, const float4* pos, const int4* cells, int3 low, int3 span, uint32_t* count,
-                        uint32_t* lin, uint32_t* slot, cudaStream_t s);
+                        uint32_t* lin, uint32_t* slot, cudaStream_t s, SubstepBegin begin = SubstepBegin{});
 // a dense table's masks (GridDev::near), one word a cell
 void launch_grid_near(const GridDev& g, uint32_t* near, cudaStream_t s);
 size_t scan_tiles(uint32_t m);
@@ -29,13 +37,8 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
                          const uint32_t* ids_in, const float4* pos_in, const float4* vel_in, const float* rho_in,
                          const int4* cells_in, uint32_t* ids_out, float4* pos_out, float4* vel_out, float* rho_out,
                          int4* cells_out, const float2* warm_in, float2* warm_out, uint32_t skip_begin,
-                         uint32_t skip_end, Status* st, uint32_t* dest,
-                         cudaStream_t s);
+                         uint32_t skip_end, Status* st, uint32_t* dest, int3 span, uint32_t* order, cudaStream_t s);
 
-// The list passes' walk order (PairLists::order) over the dense cell box `span` of a sort:
-// start is the sort's cell table (volume + 1), bcount holds walk_order_keys(span) + 1 words,
-// tile_sums scan_tiles(walk_order_keys(span)) + 1, order n.
-size_t walk_order_keys(int3 span);
 // Particle counts up to which the EXACT density pass and the WCSPH force pass, without terrain or
 // coupled bodies, run a warp a particle (k_density_warp, k_wcsph_force_warp), which then needs no
 // walk order: below one 256-thread block per SM (148 on B200) a thread a particle leaves SMs idle
@@ -52,8 +55,6 @@ constexpr uint32_t kWarpPassMax = 32768u;
 inline bool warp_rows(uint32_t n, float radius, float spacing) {
     return n <= kWarpPassMax || (n <= SLF_WARP_PASS_WIDE_MAX && radius >= 3.0f * spacing);
 }
-void launch_walk_order(uint32_t volume, int3 span, const uint32_t* start, uint32_t* bcount, uint32_t* tile_sums,
-                       uint32_t* order, cudaStream_t s);
 
 // pair passes: the density pass builds the substep's neighbour lists, the others walk them
 // T: terrain regions (regions = 0: none); slope (optional): each particle's ground density gradient

@@ -228,11 +228,10 @@ struct Profiler {
 // vectors).  The spatial hash's 72 bytes (read position, velocity, id; write them sorted; write
 // and read the cell key) are split over its kernels.
 namespace bytes_per_particle {
-constexpr double count_cells = 20, scan = 2, scatter = 8, reorder = 44;
+constexpr double count_cells = 20, scan = 2, scatter = 8, reorder = 48;  // (4: the walk order)
 constexpr double density_wcsph = 16, density_dfsph = 20, wcsph_force = 52;
 constexpr double rate_divergence = 32, rate_density = 36, push = 40, viscosity = 40, advance = 48;
 constexpr double stats = 24;
-constexpr double walk_order = 4;  // one row index written a particle
 }  // namespace bytes_per_particle
 
 
@@ -358,7 +357,7 @@ struct World {
 
     // fluid cell table of the last sort, and the list passes' walk order over it
     GridDev fgrid{};
-    DevBuf<uint32_t> worder, wkeys, wsums;
+    DevBuf<uint32_t> worder;
     bool worder_valid = false;
     int lists_pos = -1;  // slot of the positions the last sort produced
     uint64_t lists_n = 0;
@@ -401,8 +400,8 @@ struct World {
 
     Status* d_status = nullptr;
     Status* h_status = nullptr;
-    Status* h_reset = nullptr;  // pinned: the status a substep starts from (a graph copies it)
     StepConsts* d_consts = nullptr;
+    StepConsts* h_consts = nullptr;  // pinned: the constants of the next substep run as a graph
 
     int64_t skip_job = -1;  // testing: next sort leaves this 512-particle job undone
     // set while the adjoint recomputes a substep: the sort's destinations, the pre-clamp velocity
@@ -556,7 +555,7 @@ struct World {
         if (stream) {
             for (auto* b : {&pos[0], &pos[1], &pos[2], &vel[0], &vel[1], &vel[2]}) b->release(stream);
             for (auto* b : {&ids[0], &ids[1], &lin, &cslot, &members, &count, &tiles, &keep, &dwstart, &dwnear, &fcnt, &wcnt, &dscratch,
-                            &worder, &wkeys, &wsums, &etaken, &etiles})
+                            &worder, &etaken, &etiles})
                 b->release(stream);
             for (auto* b : {&rho[0], &rho[1], &press, &scaled, &alpha}) b->release(stream);
             for (auto* b : {&cell[0], &cell[1], &cell[2]}) b->release(stream);
@@ -603,7 +602,7 @@ struct World {
             if (d_status) cudaFree(d_status);
             if (d_consts) cudaFree(d_consts);
             if (h_status) cudaFreeHost(h_status);
-            if (h_reset) cudaFreeHost(h_reset);
+            if (h_consts) cudaFreeHost(h_consts);
             cudaStreamDestroy(stream);
         }
     }
@@ -881,7 +880,7 @@ struct World {
     struct SortPlan {
         int3 lo{}, span{};
         uint32_t volume = 0;
-        size_t keys = 0;  // walk-order keys; 0 when the lists keep the particle order
+        bool ordered = false;  // the lists get a walk order (else they keep the particle order)
         uint32_t job_lo = 0, job_hi = 0;
     };
     // stable: the table's box is the container's cells joined with the particles' (their own box
@@ -889,8 +888,8 @@ struct World {
     // holds them, so the sort's order, and everything after it, is the same over either box.
     int32_t plan_sort(SortPlan& sp, bool stable);
 
-    // the planned sort's launches on stream `on`
-    int32_t enqueue_sort(int to, const SortPlan& sp, cudaStream_t on);
+    // the planned sort's launches on stream `on`; begin: what its first kernel sets
+    int32_t enqueue_sort(int to, const SortPlan& sp, cudaStream_t on, SubstepBegin begin = SubstepBegin{});
 
     int32_t update_neighbors();
 

@@ -49,8 +49,7 @@ int32_t World::init(const slf_settings& settings) {
     SLF_CUDA(cudaMalloc(&d_consts, sizeof(StepConsts)));
     SLF_CUDA(cudaMallocHost(&h_status, sizeof(Status)));
     std::memset(h_status, 0, sizeof(Status));
-    SLF_CUDA(cudaMallocHost(&h_reset, sizeof(Status)));
-    *h_reset = fresh_status();
+    SLF_CUDA(cudaMallocHost(&h_consts, sizeof(StepConsts)));
     SLF_CUDA(cudaMemsetAsync(d_status, 0, sizeof(Status), stream));
     build_ground_sites();
     return SLF_OK;
@@ -499,19 +498,13 @@ int32_t World::plan_sort(SortPlan& sp, bool stable) {
     SLF_TRY(ensure_work_buffers());
     SLF_TRY(count.ensure(size_t(sp.volume) + 1, 0, stream));
     SLF_TRY(tiles.ensure(scan_tiles(sp.volume) + 1, 0, stream));
-    // the walk order of this sort's lists (identity where its key space would not fit 32 bits,
-    // and where every pass over the lists runs a warp a particle)
-    size_t keys = walk_order_keys(sp.span);
-    sp.keys = 0;
+    // the walk order of this sort's lists (none where every pass over the lists runs a warp a
+    // particle)
     bool warp_passes = !fast() && s.solver == SLF_SOLVER_WCSPH && warp_rows(uint32_t(n), radius, s.spacing) &&
                        terrains.empty() && m_pos.empty();
-    if (keys < (size_t(1) << 31) && !warp_passes) {
-        SLF_TRY(worder.ensure(n, 0, stream));
-        SLF_TRY(wkeys.ensure(keys + 1, 0, stream));
-        SLF_TRY(wsums.ensure(scan_tiles(uint32_t(keys)) + 1, 0, stream));
-        sp.keys = keys;
-    }
-    worder_valid = sp.keys != 0;
+    sp.ordered = !warp_passes;
+    if (sp.ordered) SLF_TRY(worder.ensure(n, 0, stream));
+    worder_valid = sp.ordered;
     fgrid = GridDev{};
     fgrid.mode = 1;
     fgrid.lx = sp.lo.x;
@@ -524,11 +517,12 @@ int32_t World::plan_sort(SortPlan& sp, bool stable) {
     return SLF_OK;
 }
 
-int32_t World::enqueue_sort(int to, const SortPlan& sp, cudaStream_t on) {
+int32_t World::enqueue_sort(int to, const SortPlan& sp, cudaStream_t on, SubstepBegin begin) {
     Params p = params();
     SLF_CUDA(cudaMemsetAsync(count.p, 0, (size_t(sp.volume) + 1) * 4, on));
     timed("hash_count", bytes_per_particle::count_cells, [&] {
-        launch_count_cells(p, pos[cpos].p, cells_of(cpos), sp.lo, sp.span, count.p, lin.p, cslot.p, on);
+        launch_count_cells(p, pos[cpos].p, cells_of(cpos), sp.lo, sp.span, count.p, lin.p, cslot.p, on,
+                           begin);
     });
     timed("hash_scan", bytes_per_particle::scan,
           [&] { launch_exclusive_scan(count.p, sp.volume, tiles.p, on); });
@@ -538,11 +532,9 @@ int32_t World::enqueue_sort(int to, const SortPlan& sp, cudaStream_t on) {
     timed("hash_reorder", bytes_per_particle::reorder, [&] {
         launch_rank_reorder(uint32_t(n), lin.p, count.p, members.p, ids[cid].p, pos[cpos].p, vel[cpos].p,
                             rho[cid].p, cells_of(cpos), ids[1 - cid].p, pos[to].p, vel[to].p, rho[1 - cid].p,
-                            cells_of(to), warm_in(), warm_out(), sp.job_lo, sp.job_hi, d_status, sort_dest, on);
+                            cells_of(to), warm_in(), warm_out(), sp.job_lo, sp.job_hi, d_status, sort_dest, sp.span,
+                            sp.ordered ? worder.p : nullptr, on);
     });
-    if (sp.keys)
-        timed("walk_order", bytes_per_particle::walk_order,
-              [&] { launch_walk_order(sp.volume, sp.span, count.p, wkeys.p, wsums.p, worder.p, on); });
     return SLF_OK;
 }
 

@@ -241,7 +241,7 @@ std::vector<uint8_t> World::substep_key(const Params& p, int a, int b, int nid, 
     key_add(k, sp.lo);
     key_add(k, sp.span);
     key_add(k, sp.volume);
-    key_add(k, sp.keys);
+    key_add(k, int32_t(sp.ordered));
     key_add(k, sp.job_lo);
     key_add(k, sp.job_hi);
     key_add(k, fgrid);
@@ -251,8 +251,8 @@ std::vector<uint8_t> World::substep_key(const Params& p, int a, int b, int nid, 
     for (const void* q : std::initializer_list<const void*>{
              pos[cpos].p, vel[cpos].p, cells_of(cpos), ids[cid].p, ids[nid].p, rho[cid].p, rho[nid].p,
              pos[a].p, vel[a].p, cells_of(a), pos[b].p, vel[b].p, cells_of(b), warm_in(), warm_out(),
-             sort_dest, count.p, tiles.p, lin.p, cslot.p, members.p, worder.p, wkeys.p, wsums.p, press.p,
-             scaled.p, alpha.p, dwalls.p, partials.p, d_status, d_consts, vel_pre, h_reset,
+             sort_dest, count.p, tiles.p, lin.p, cslot.p, members.p, worder.p, press.p,
+             scaled.p, alpha.p, dwalls.p, partials.p, d_status, d_consts, vel_pre, h_consts,
              dscratch.p})
         key_add(k, q);
     return k;
@@ -265,8 +265,7 @@ int32_t World::capture_substep(const Params& p, int a, int b, int nid, const Sor
     uint64_t before = kernel_launches();
     SLF_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     auto record = [&]() -> int32_t {
-        SLF_TRY(enqueue_sort(a, sp, cs));
-        SLF_CUDA(cudaMemcpyAsync(d_status, h_reset, sizeof(Status), cudaMemcpyHostToDevice, cs));
+        SLF_TRY(enqueue_sort(a, sp, cs, SubstepBegin{d_status, d_consts, h_consts}));
         PairLists fl = fluid_lists(), wl = wall_lists();
         density_pass(p, a, fl, wl, rho[nid].p, cs);
         if (s.solver == SLF_SOLVER_WCSPH) {
@@ -330,7 +329,7 @@ int32_t World::substep_graph(float dt, const Params& p, int a, int b, int nid, c
     }
     hit->used = ++graph_clock;
     ++hit->runs;
-    launch_set_consts(consts(dt), d_consts, stream);
+    *h_consts = consts(dt);  // (the last launch that read them was waited for)
     SLF_CUDA(cudaGraphLaunch(hit->exec, stream));
     note_launches(hit->outside);
     graph_solves = s.solver == SLF_SOLVER_DFSPH ? 3u : 0u;
