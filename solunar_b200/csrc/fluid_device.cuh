@@ -391,6 +391,8 @@ __device__ __forceinline__ void each_near(const Params& p, const GridDev& g, con
         // dense table (under 2^31 cells): the cell's place in it once, in 64 bits as cells near
         // the i32 limits overflow, each neighbour's index in 32 bits once it is known inside
         const long long bx = (long long)cell.x - g.lx, by = (long long)cell.y - g.ly, bz = (long long)cell.z - g.lz;
+        // nothing near: most particles' answer where the points are a body's
+        if (bx < -1 || bx > g.sx || by < -1 || by > g.sy || bz < -1 || bz > g.sz) return;
 #pragma unroll 1
         for (int dz = -1; dz <= 1; ++dz) {
             long long z = bz + dz;

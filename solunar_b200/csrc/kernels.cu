@@ -9,6 +9,7 @@
 #include <atomic>
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 #include "fluid_device.cuh"
 #include "launch.h"
@@ -17,18 +18,16 @@
 namespace slf {
 
 // Bounding box of cells, fastest speed, held-back count and non-finite flag of a block's
-// particles, folded into the status with one atomic each.
-__device__ __forceinline__ void fold_advance_stats(Status* st, bool valid, int3 c, float speed, uint32_t held,
-                                                   uint32_t bad) {
-    int lox = valid ? c.x : INT_MAX, loy = valid ? c.y : INT_MAX, loz = valid ? c.z : INT_MAX;
-    int hix = valid ? c.x : INT_MIN, hiy = valid ? c.y : INT_MIN, hiz = valid ? c.z : INT_MIN;
-    uint32_t sb = (valid && speed > 0.0f) ? __float_as_uint(speed) : 0u;
-    lox = block_reduce(lox, MinI(), INT_MAX);
-    loy = block_reduce(loy, MinI(), INT_MAX);
-    loz = block_reduce(loz, MinI(), INT_MAX);
-    hix = block_reduce(hix, MaxI(), INT_MIN);
-    hiy = block_reduce(hiy, MaxI(), INT_MIN);
-    hiz = block_reduce(hiz, MaxI(), INT_MIN);
+// particles, folded into the status with one atomic each (a thread without particles: an empty box).
+__device__ __forceinline__ void fold_advance_box(Status* st, int3 lo, int3 hi, float speed, uint32_t held,
+                                                 uint32_t bad) {
+    uint32_t sb = speed > 0.0f ? __float_as_uint(speed) : 0u;
+    int lox = block_reduce(lo.x, MinI(), INT_MAX);
+    int loy = block_reduce(lo.y, MinI(), INT_MAX);
+    int loz = block_reduce(lo.z, MinI(), INT_MAX);
+    int hix = block_reduce(hi.x, MaxI(), INT_MIN);
+    int hiy = block_reduce(hi.y, MaxI(), INT_MIN);
+    int hiz = block_reduce(hi.z, MaxI(), INT_MIN);
     sb = block_reduce(sb, MaxU(), 0u);
     held = block_reduce(held, SumU(), 0u);
     bad = block_reduce(bad, MaxU(), 0u);
@@ -45,6 +44,13 @@ __device__ __forceinline__ void fold_advance_stats(Status* st, bool valid, int3 
         if (held) atomicAdd(&st->held, held);
         if (bad) atomicMax(&st->nonfinite, 1u);
     }
+}
+
+// The same with one particle a thread (valid: whether it has one).
+__device__ __forceinline__ void fold_advance_stats(Status* st, bool valid, int3 c, float speed, uint32_t held,
+                                                   uint32_t bad) {
+    const int3 lo = make_int3(INT_MAX, INT_MAX, INT_MAX), hi = make_int3(INT_MIN, INT_MIN, INT_MIN);
+    fold_advance_box(st, valid ? c : lo, valid ? c : hi, valid ? speed : 0.0f, held, bad);
 }
 
 // ---- bounding box and fastest speed of the current state ---------------------------------
@@ -380,15 +386,17 @@ __device__ __forceinline__ float ground_near(const TerrainDev& T, float px, floa
 // 87 -> 59 (75k WCSPH).
 // Four candidates and two pairs in flight, at 64 registers and four blocks a SM: two candidates
 // measured 470 us at 1M, six 522, eight 556 (spills; 497 at 109 registers and two blocks), four
-// pairs 482, and 48 registers for five blocks 571.
-constexpr int kScanUnroll = 4;
-constexpr int kPairUnroll = 2;
+// pairs 482, and 48 registers for five blocks 571.  A grid of at most two blocks a SM runs wide
+// instead (eight candidates and four pairs in flight, up to 128 registers): it has no other warps
+// to hide behind.  74k particles: 57 -> 48 us, at support 4 378 -> 302; 111k, three blocks a SM,
+// stay.
 
 // Lists the points of cells [b, e) within reach of `at`, in array order: each kept index goes to
 // out[nf * 32] (room for `cap`; the count goes on past it).  Four candidates' gathers are in flight
 // at a time, and a kept one costs a predicated store and an add: no branch, so the lanes of a warp
 // that keep nothing do not wait for those that do.  axy, az: the negated position; x and y of the
 // test run packed, each operation rounded as each_in_cell's.
+template <int kScanUnroll>
 __device__ __forceinline__ void scan_range(const Params& p, const float4* __restrict__ pts, uint32_t b, uint32_t e,
                                            f32x2 axy, float az, uint32_t* out, uint32_t cap,
                                            uint32_t& nf) {
@@ -417,10 +425,10 @@ __device__ __forceinline__ void scan_range(const Params& p, const float4* __rest
 // registers stays out of the density pass.
 __device__ __noinline__ uint32_t scan_checked(const Params& p, const GridDev& g, const float4* __restrict__ pts,
                                               int3 cell, float x, float y, float z, uint32_t* out,
-                                              uint32_t cap) {
+                                              uint32_t cap, uint32_t stride) {
     uint32_t nf = 0;
     each_near(p, g, pts, cell, x, y, z, [&](uint32_t j, float4) {
-        if (nf < cap) out[size_t(nf) * 32u] = j;
+        if (nf < cap) out[size_t(nf) * stride] = j;
         ++nf;
     });
     return nf;
@@ -430,6 +438,7 @@ __device__ __noinline__ uint32_t scan_checked(const Params& p, const GridDev& g,
 // Where the table knows which of a cell's 27 cells hold points (GridDev::near, the walls), only those
 // are visited; a cell with its 26 neighbours inside a dense table needs no bounds checks (the world
 // pads the fluid's table so that every particle's has).
+template <int kScanUnroll>
 __device__ __forceinline__ uint32_t scan_near(const Params& p, const GridDev& g, const float4* __restrict__ pts,
                                               int3 cell, float x, float y, float z, uint32_t* out,
                                               uint32_t cap) {
@@ -438,7 +447,7 @@ __device__ __forceinline__ uint32_t scan_near(const Params& p, const GridDev& g,
     const int edge = g.near ? 0 : 1;  // cells that a walk without checks keeps away from the box's faces
     if (g.mode != 1 || bx < edge || bx + edge >= g.sx || by < edge || by + edge >= g.sy || bz < edge ||
         bz + edge >= g.sz)
-        return scan_checked(p, g, pts, cell, x, y, z, out, cap);
+        return scan_checked(p, g, pts, cell, x, y, z, out, cap, 32u);
     const f32x2 axy = pack2(-x, -y);
     const float az = -z;
     const uint32_t slab = uint32_t(g.sy) * uint32_t(g.sz);
@@ -448,7 +457,7 @@ __device__ __forceinline__ uint32_t scan_near(const Params& p, const GridDev& g,
     for (uint32_t mask = g.near ? __ldg(&g.near[c0]) : (1u << 27) - 1u; mask; mask &= mask - 1u) {
         const int t = __ffs(int(mask)) - 1;
         const uint32_t c = c0 + uint32_t((t % 3 - 1) * int(slab) + (t / 3 % 3 - 1) * g.sz + t / 9 - 1);
-        scan_range(p, pts, __ldg(&g.start[c]), __ldg(&g.start[c + 1]), axy, az, out, cap, nf);
+        scan_range<kScanUnroll>(p, pts, __ldg(&g.start[c]), __ldg(&g.start[c + 1]), axy, az, out, cap, nf);
     }
     return nf;
 }
@@ -486,7 +495,9 @@ __device__ __forceinline__ f32x2 div_radius2(const Params& p, f32x2 a) {
 __device__ __forceinline__ void kernel_pair(const Params& p, f32x2 d2, f32x2& value, float& g0, float& g1) {
     float s0, s1;
     unpack2(d2, s0, s1);
-    const float d0 = sqrtf(s0), d1 = sqrtf(s1);
+    // the particle itself (s = 0) stays off the slow paths of the root and the division
+    const float r0 = sqrtf(s0 > 0.0f ? s0 : 1.0f), r1 = sqrtf(s1 > 0.0f ? s1 : 1.0f);
+    const float d0 = s0 > 0.0f ? r0 : 0.0f, d1 = s1 > 0.0f ? r1 : 0.0f;
     const f32x2 q = div_radius2<false>(p, pack2(d0, d1));
     const f32x2 one = splat2(1.0f);
     const f32x2 om = fma2(q, splat2(-1.0f), one);  // 1 - q: the product is exact
@@ -496,8 +507,11 @@ __device__ __forceinline__ void kernel_pair(const Params& p, f32x2 d2, f32x2& va
     float l0, l1, q0, q1;
     unpack2(slope, l0, l1);
     unpack2(q, q0, q1);
-    g0 = q0 < 1.0f && d0 > 0.0f ? l0 / d0 : 0.0f;
-    g1 = q1 < 1.0f && d1 > 0.0f ? l1 / d1 : 0.0f;
+    const bool p0 = q0 < 1.0f && d0 > 0.0f, p1 = q1 < 1.0f && d1 > 0.0f;
+    g0 = (p0 ? l0 : 1.0f) / (p0 ? d0 : 1.0f);
+    g1 = (p1 ? l1 : 1.0f) / (p1 ? d1 : 1.0f);
+    g0 = p0 ? g0 : 0.0f;
+    g1 = p1 ? g1 : 0.0f;
     if (!(q0 < 1.0f && q1 < 1.0f)) {  // at the very edge: value is zero from there on
         float v0, v1;
         unpack2(value, v0, v1);
@@ -510,11 +524,10 @@ __device__ __forceinline__ void kernel_pair(const Params& p, f32x2 d2, f32x2& va
 // row's list, and pair(v, gx, gy, gz) takes the kernel's value and G in list order.  Two pairs run
 // packed, and the next ones' indices are requested before their terms are formed.  (`from` was
 // written by this thread, and is rewritten for its next list: never a read-only load.)
-template <bool GRADIENT, class Pair>
+template <bool GRADIENT, int U, class Pair>
 __device__ __forceinline__ void pair_terms(const Params& p, const PairLists& l, uint32_t row, uint32_t m,
                                            const uint32_t* from, const float4* __restrict__ pts, float4 a,
                                            bool walls, Pair&& pair) {
-    constexpr int U = kPairUnroll;
     static_assert(U % 2 == 0, "pairs run two at a time");
     if (m == 0) return;
     uint2* e = l.e + l.at(row, 0);
@@ -565,65 +578,18 @@ __device__ __forceinline__ void pair_terms(const Params& p, const PairLists& l, 
     }
 }
 
-// One warp lists row `row`'s neighbours in grid g, in each_near's order: lanes 0-26 take the 27
-// cells' ranges (dz outer, dy, dx inner) and sum their lengths; then 32 consecutive candidates of
-// the cells laid end to end are tested at a time, a lane finding its cell by a binary search over
-// the sums, and the kept ones are written in order through a ballot.  The test is each_in_cell's,
-// so the list is the one-thread walk's entry for entry.  Returns the count (every lane).
-__device__ __forceinline__ uint32_t warp_list_near(const Params& p, const GridDev& g, const float4* __restrict__ pts,
-                                                   int3 cell, float ax, float ay, float az, const PairLists& l,
-                                                   uint32_t row, uint32_t lane) {
-    if (g.mode == 0) return 0u;
-    uint32_t b = 0, len = 0;
-    if (lane < 27u) {
-        int dz = int(lane / 9u) - 1, dy = int((lane / 3u) % 3u) - 1, dx = int(lane % 3u) - 1;
-        uint32_t e = 0;
-        if (g.range((long long)cell.x + dx, (long long)cell.y + dy, (long long)cell.z + dz, b, e) && e > b) len = e - b;
-    }
-    uint32_t incl = len;  // inclusive prefix sum of the lengths over the lanes
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= uint32_t(o)) incl += up;
-    }
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t m = 0;
-    for (uint32_t t0 = 0; t0 < total; t0 += 32u) {
-        uint32_t t = t0 + lane;
-        // the first cell whose inclusive sum exceeds t (cells 0-26; lanes past the end search too)
-        uint32_t lo = 0, hi = 26;
-#pragma unroll
-        for (int step = 0; step < 5; ++step) {
-            uint32_t mid = (lo + hi) >> 1;
-            uint32_t at = __shfl_sync(0xffffffffu, incl, mid);
-            if (t < at) hi = mid;
-            else lo = mid + 1u;
-        }
-        uint32_t k = lo < 26u ? lo : 26u;
-        uint32_t kb = __shfl_sync(0xffffffffu, b, k), kincl = __shfl_sync(0xffffffffu, incl, k),
-                 klen = __shfl_sync(0xffffffffu, len, k);
-        bool keep = false;
-        uint32_t j = 0;
-        if (t < total) {
-            j = kb + (t - (kincl - klen));
-            float4 q = __ldg(&pts[j]);
-            float ox = q.x - ax, oy = q.y - ay, oz = q.z - az;
-            keep = dot3(ox, oy, oz, ox, oy, oz) < p.reach;
-        }
-        uint32_t mask = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-            uint32_t at = m + __popc(mask & ((1u << lane) - 1u));
-            if (at < l.cap) l.e[l.at(row, at)].x = j;
-        }
-        m += __popc(mask);
-    }
-    return m;
-}
-
 // ---- densities (mod.rs:621-675) and the substep's neighbour lists, with WCSPH pressure
 // (step.rs:147-172) or the DFSPH factors (dfsph.rs:108-163) --------------------------------
 
 // four blocks a SM (64 registers), as the pass compiled before it strode over rows
+// Where the density pass leaves what the later passes gather of a neighbour beside its position and
+// velocity, so that one 16-byte gather brings both: p / rho^2 in the position's spare lane (WCSPH;
+// DFSPH's checks put the stiffness there), the density in the velocity's.
+struct PairRecords {
+    float* pos_w;
+    float* vel_w;
+};
+
 // What the pass lists: the fluid (0), then the walls (1).
 struct DensityIn {
     GridDev grid[2];
@@ -632,11 +598,11 @@ struct DensityIn {
 };
 
 // EXTRA: terrain regions or coupled bodies add their terms
-template <int SOLVER, bool EXTRA>
-__global__ void __launch_bounds__(kBlock, 4)
+template <int SOLVER, bool EXTRA, bool WIDE>
+__global__ void __launch_bounds__(kBlock, WIDE ? 2 : 4)
     k_density(const __grid_constant__ Params p, const __grid_constant__ DensityIn in, float* __restrict__ rho,
               float* __restrict__ press, float* __restrict__ scaled, float* __restrict__ alpha, Status* st, TerrainDev T,
-              float4* __restrict__ slope, MoverDev M, uint32_t* scratch) {
+              float4* __restrict__ slope, MoverDev M, uint32_t* scratch, PairRecords rec) {
     uint32_t compressed = 0, longest = 0;
     const float4* __restrict__ pos = in.pts[0];
     // this warp's unfinished list, entry k of a lane at k * 32: the same few megabytes for every row
@@ -657,11 +623,11 @@ __global__ void __launch_bounds__(kBlock, 4)
         for (int w = 0; w < 2; ++w) {  // the fluid, then the walls
             const PairLists& l = in.list[w];
             const float4* __restrict__ pts = in.pts[w];
-            const uint32_t found = scan_near(p, in.grid[w], pts, cell, a.x, a.y, a.z, idx, l.cap);
+            const uint32_t found = scan_near<WIDE ? 8 : 4>(p, in.grid[w], pts, cell, a.x, a.y, a.z, idx, l.cap);
             l.count[row] = found;
             longest = max(longest, found);
             float sum = 0.0f;
-            pair_terms<SOLVER == 1>(p, l, row, found < l.cap ? found : l.cap, idx, pts, a, w == 1,
+            pair_terms<SOLVER == 1, WIDE ? 4 : 2>(p, l, row, found < l.cap ? found : l.cap, idx, pts, a, w == 1,
                                     [&](float v, float gx, float gy, float gz) {
                                         sum += v;
                                         if (SOLVER == 1) {  // factors (dfsph.rs:149-153); walls add no squares
@@ -693,11 +659,14 @@ __global__ void __launch_bounds__(kBlock, 4)
             float ratio = fminf(density / p.rest, 1.1f);
             float pressure = fmaxf(p.stiffness * (pow7(ratio) - 1.0f), 0.0f);
             press[i] = pressure;
-            scaled[i] = pressure / (density * density);
+            const float over = pressure > 0.0f ? pressure / (density * density) : 0.0f;
+            scaled[i] = over;
+            rec.pos_w[4 * size_t(i) + 3] = over;
         } else {
             float total = dot3(sx, sy, sz, sx, sy, sz) + squares;
             alpha[i] = total > 0.0f ? 1.0f / total : 0.0f;
         }
+        rec.vel_w[4 * size_t(i) + 3] = density;
         float c = density / p.rest - 1.0f;
         if (c > 0.0f) compressed = max(compressed, __float_as_uint(c));
     }
@@ -709,119 +678,351 @@ __global__ void __launch_bounds__(kBlock, 4)
     }
 }
 
-// The density pass for scenes too small to fill the GPU a thread a particle: a warp a row.  The
-// lists come from warp_list_near; each lane takes every 32nd listed neighbour's terms, and the
-// sums run in list order, one term after the other through shuffles, so every sum and factor is
-// k_density's bit for bit.  Body points and ground are taken by every lane alike.
-template <int SOLVER>
-__global__ void __launch_bounds__(kBlock) k_density_warp(Params p, GridDev fg, GridDev wg,
-                                                         const float4* __restrict__ pos, const float4* __restrict__ walls,
-                                                         PairLists fl, PairLists wl, float* __restrict__ rho,
-                                                         float* __restrict__ press, float* __restrict__ scaled,
-                                                         float* __restrict__ alpha, Status* st, TerrainDev T,
-                                                         float4* __restrict__ slope, MoverDev M) {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+// ---- scenes too small for a thread a row: L lanes a row -----------------------------------------
+// A thread a row leaves a scene of 64,000 particles 13 warps a SM, each with one long chain of
+// gathers, divisions and ordered adds; 8,000 particles leave most schedulers without a warp.  Here a warp takes 32 / L rows (lane = row + (32 / L) * sub,
+// so that a step's list entries lie side by side), each lane every L-th candidate or pair; the terms
+// meet in shared memory and one lane per (row, component) adds them in list order, so every sum is
+// the one-thread walk's bit for bit.  A term past a list's end is +0, which leaves a sum that began
+// at +0, and any value it is subtracted from, as it was.  Measured (density + force, us, against a
+// warp a row whose lanes passed the terms round by shuffles): group_lanes.
+
+constexpr int kGroupBlock = 128;
+constexpr int kGroupBlocks = 8;  // a SM: 64 registers
+
+template <int L, int NC>
+struct GroupSums {
+    static constexpr int kRows = 32 / L;
+    static constexpr int kChunk = L < 16 ? 32 : 2 * L;  // pairs of a row between two rounds of adds
+    static constexpr int kStride = kChunk + 4;          // 16-byte rows whose lanes fall in other banks
+    static constexpr int kChains = kRows * NC;
+    static constexpr int kRounds = (kChains + 31) / 32;
+    float term[kChains * kStride];
+
+    // this row's term c of its chunk's k-th pair
+    __device__ __forceinline__ void put(int row, int c, int k, float v) { term[(row * NC + c) * kStride + k] = v; }
+
+    // Adds (or, NEGATE, subtracts) the first `count` terms of every chain to its lane's acc, in order.
+    template <bool NEGATE>
+    __device__ __forceinline__ void add(float (&acc)[kRounds], uint32_t lane, uint32_t count) {
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kRounds; ++q) {
+            if (lane + 32u * q < uint32_t(kChains)) {
+                const float4* t = reinterpret_cast<const float4*>(term + (lane + 32u * q) * kStride);
+                float s = acc[q];
+#pragma unroll 4
+                for (uint32_t k = 0; k < count; k += 4) {
+                    const float4 v = t[k / 4];
+                    s = NEGATE ? s - v.x : s + v.x;
+                    s = NEGATE ? s - v.y : s + v.y;
+                    s = NEGATE ? s - v.z : s + v.z;
+                    s = NEGATE ? s - v.w : s + v.w;
+                }
+                acc[q] = s;
+            }
+        }
+        __syncwarp();
+    }
+
+    // Every lane of a row gets the row's sums: out[c].
+    __device__ __forceinline__ void spread(const float (&acc)[kRounds], uint32_t lane, int row, float (&out)[NC]) {
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kRounds; ++q)
+            if (lane + 32u * q < uint32_t(kChains)) term[lane + 32u * q] = acc[q];
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < NC; ++c) out[c] = term[row * NC + c];
+        __syncwarp();
+    }
+};
+
+// scan_near by the L lanes of a row, for cells of many points: the list goes to out[k * 32 / L], the
+// count comes back in every lane.  The warp walks the cells that any of its rows visits together, the
+// lanes of a row testing L points of its cell at a time, kFlight of them each in flight.
+template <int L, int kFlight>
+__device__ __forceinline__ uint32_t scan_cells_group(const Params& p, const GridDev& g, const float4* __restrict__ pts,
+                                                    bool valid, int3 cell, float x, float y, float z, uint32_t* out,
+                                                    uint32_t cap, uint32_t lane) {
+    constexpr uint32_t R = 32u / L;
+    if (g.mode == 0) return 0u;
+    const uint32_t sub = lane / R;
+    const uint32_t own = (L == 32 ? 0xffffffffu : L == 16 ? 0x55555555u : L == 8 ? 0x11111111u : 0x01010101u)
+                         << (lane % R);
+    const uint32_t below = own & ((1u << lane) - 1u);
+    const long long bx = (long long)cell.x - g.lx, by = (long long)cell.y - g.ly, bz = (long long)cell.z - g.lz;
+    const int edge = g.near ? 0 : 1;
+    const bool plain = g.mode == 1 && bx >= edge && bx + edge < g.sx && by >= edge && by + edge < g.sy && bz >= edge &&
+                       bz + edge < g.sz;
+    const f32x2 axy = pack2(-x, -y);
+    const float az = -z;
+    const uint32_t slab = uint32_t(g.sy) * uint32_t(g.sz);
+    const uint32_t c0 = (uint32_t(bx) * uint32_t(g.sy) + uint32_t(by)) * uint32_t(g.sz) + uint32_t(bz);
+    const uint32_t mine = !valid || !plain ? 0u : g.near ? __ldg(&g.near[c0]) : (1u << 27) - 1u;
+    const ulonglong2* __restrict__ q2 = reinterpret_cast<const ulonglong2*>(pts);
+    uint32_t nf = 0;
+#pragma unroll 1
+    for (uint32_t mask = __reduce_or_sync(0xffffffffu, mine); mask; mask &= mask - 1u) {
+        const int t = __ffs(int(mask)) - 1;
+        uint32_t b = 0, e = 0;
+        if (mine >> t & 1u) {
+            const uint32_t c = c0 + uint32_t((t % 3 - 1) * int(slab) + (t / 3 % 3 - 1) * g.sz + t / 9 - 1);
+            b = __ldg(&g.start[c]);
+            e = __ldg(&g.start[c + 1]);
+        }
+        const uint32_t longest = __reduce_max_sync(0xffffffffu, e - b);
+#pragma unroll 1
+        for (uint32_t k = sub; k < longest + sub; k += uint32_t(kFlight * L)) {  // (every lane the same rounds)
+            ulonglong2 q[kFlight];
+#pragma unroll
+            for (int u = 0; u < kFlight; ++u) {
+                if (b + k + u * L < e) q[u] = __ldg(q2 + b + k + u * L);
+            }
+#pragma unroll
+            for (int u = 0; u < kFlight; ++u) {
+                const uint32_t j = b + k + u * L;
+                const f32x2 oxy = add2(f32x2{q[u].x}, axy);
+                const float oz = __uint_as_float(uint32_t(q[u].y)) + az;
+                float x2, y2;
+                unpack2(mul2(oxy, oxy), x2, y2);
+                const bool keep = j < e && (x2 + y2) + oz * oz < p.reach;
+                const uint32_t kept = __ballot_sync(0xffffffffu, keep);
+                const uint32_t at = nf + __popc(kept & below);
+                if (keep && at < cap) out[size_t(at) * R] = j;
+                nf += __popc(kept & own);
+            }
+        }
+    }
+    if (__any_sync(0xffffffffu, valid && !plain)) {  // tables that need checks: one lane a row
+        if (valid && !plain && sub == 0) nf = scan_checked(p, g, pts, cell, x, y, z, out, cap, R);
+        nf = __shfl_sync(0xffffffffu, nf, lane % R);
+    }
+    return nf;
+}
+
+// The 27 cells around each row of a warp, laid end to end: cell c's points are candidates
+// [upto[c - 1], upto[c]), point = candidate + shift[c].
+template <int L>
+struct GroupCells {
+    static constexpr int kRows = 32 / L;
+    uint32_t upto[kRows][28], shift[kRows][28];
+};
+
+// The same for cells of few points.  The lanes look the 27 cells up side by side, then test L candidates of the cells laid end
+// to end at a time (kFlight of them each in flight) and place the kept ones by a ballot.
+template <int L>
+__device__ __forceinline__ uint32_t scan_near_group(const Params& p, const GridDev& g, const float4* __restrict__ pts,
+                                                    bool valid, int3 cell, float x, float y, float z, uint32_t* out,
+                                                    uint32_t cap, uint32_t lane, GroupCells<L>& cells) {
+    constexpr uint32_t R = 32u / L;
+    constexpr int kPer = (27 + L - 1) / L;  // cells a lane
+    constexpr int kFlight = L <= 8 ? 4 : 2;
+    if (g.mode == 0) return 0u;
+    const uint32_t r = lane % R, sub = lane / R;
+    const uint32_t own = (L == 32 ? 0xffffffffu : L == 16 ? 0x55555555u : L == 8 ? 0x11111111u : 0x01010101u) << r;
+    const uint32_t below = own & ((1u << lane) - 1u);
+    const long long bx = (long long)cell.x - g.lx, by = (long long)cell.y - g.ly, bz = (long long)cell.z - g.lz;
+    const int edge = g.near ? 0 : 1;
+    const bool plain = g.mode == 1 && bx >= edge && bx + edge < g.sx && by >= edge && by + edge < g.sy && bz >= edge &&
+                       bz + edge < g.sz;
+    const uint32_t slab = uint32_t(g.sy) * uint32_t(g.sz);
+    const uint32_t c0 = (uint32_t(bx) * uint32_t(g.sy) + uint32_t(by)) * uint32_t(g.sz) + uint32_t(bz);
+    const uint32_t mask = !valid || !plain ? 0u : g.near ? __ldg(&g.near[c0]) : (1u << 27) - 1u;
+    uint32_t nf = 0;
+    if (__any_sync(0xffffffffu, mask != 0u)) {
+        uint32_t begin[kPer], len[kPer], total = 0;
+#pragma unroll
+        for (int c = 0; c < kPer; ++c) {
+            const int t = int(sub) * kPer + c;
+            begin[c] = len[c] = 0u;
+            if (t < 27 && (mask >> t & 1u)) {
+                const uint32_t at = c0 + uint32_t((t % 3 - 1) * int(slab) + (t / 3 % 3 - 1) * g.sz + t / 9 - 1);
+                begin[c] = __ldg(&g.start[at]);
+                len[c] = __ldg(&g.start[at + 1]) - begin[c];
+            }
+            total += len[c];
+        }
+        uint32_t upto = total;  // inclusive over the row's lanes
+#pragma unroll
+        for (int d = 1; d < L; d <<= 1) {
+            const uint32_t other = __shfl_up_sync(0xffffffffu, upto, d * int(R));
+            if (int(sub) >= d) upto += other;
+        }
+        const uint32_t all = __shfl_sync(0xffffffffu, upto, 32u - R + r);
+        upto -= total;
+#pragma unroll
+        for (int c = 0; c < kPer; ++c) {
+            const int t = int(sub) * kPer + c;
+            if (t < 27) {
+                cells.shift[r][t] = begin[c] - upto;
+                upto += len[c];
+                cells.upto[r][t] = upto;
+            }
+        }
+        __syncwarp();
+        const f32x2 axy = pack2(-x, -y);
+        const float az = -z;
+        const ulonglong2* __restrict__ q2 = reinterpret_cast<const ulonglong2*>(pts);
+        const uint32_t most = __reduce_max_sync(0xffffffffu, all);
+        uint32_t c = 0, end = cells.upto[r][0];
+#pragma unroll 1
+        for (uint32_t k = sub; k < most + sub; k += uint32_t(kFlight * L)) {  // (every lane the same rounds)
+            ulonglong2 q[kFlight];
+            uint32_t j[kFlight];
+#pragma unroll
+            for (int u = 0; u < kFlight; ++u) {
+                const uint32_t t = k + u * L;
+                if (t < all) {
+                    while (t >= end) end = cells.upto[r][++c];
+                    j[u] = t + cells.shift[r][c];
+                    q[u] = __ldg(q2 + j[u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kFlight; ++u) {
+                const f32x2 oxy = add2(f32x2{q[u].x}, axy);
+                const float oz = __uint_as_float(uint32_t(q[u].y)) + az;
+                float x2, y2;
+                unpack2(mul2(oxy, oxy), x2, y2);
+                const bool keep = k + u * L < all && (x2 + y2) + oz * oz < p.reach;
+                const uint32_t kept = __ballot_sync(0xffffffffu, keep);
+                const uint32_t at = nf + __popc(kept & below);
+                if (keep && at < cap) out[size_t(at) * R] = j[u];
+                nf += __popc(kept & own);
+            }
+        }
+        __syncwarp();
+    }
+    if (__any_sync(0xffffffffu, valid && !plain)) {  // tables that need checks: one lane a row
+        if (valid && !plain && sub == 0) nf = scan_checked(p, g, pts, cell, x, y, z, out, cap, R);
+        nf = __shfl_sync(0xffffffffu, nf, r);
+    }
+    return nf;
+}
+
+// k_density by L lanes a row.
+// BODIES: coupled bodies add their points.  (Terrain keeps a thread a row.)
+// FLIGHT: the scan a cell at a time with that many points a lane in flight (scan_cells_group); 0: the
+// cells end to end (scan_near_group).
+template <int SOLVER, bool BODIES, int L, int FLIGHT>
+__global__ void __launch_bounds__(kGroupBlock, kGroupBlocks)
+    k_density_group(const __grid_constant__ Params p, const __grid_constant__ DensityIn in, float* __restrict__ rho,
+                    float* __restrict__ press, float* __restrict__ scaled, float* __restrict__ alpha, Status* st,
+                    MoverDev M, uint32_t* scratch, PairRecords rec) {
+    // the sums: the kernel's value, and with DFSPH the gradients' x, y, z and squares
+    constexpr int NC = SOLVER == 1 ? 5 : 1, X = NC > 1 ? 1 : 0, Y = 2 * X, Z = 3 * X, Q = 4 * X;
+    using Sums = GroupSums<L, NC>;
+    constexpr uint32_t R = Sums::kRows;
+    __shared__ __align__(16) Sums shared[kGroupBlock / 32];
+    __shared__ GroupCells<L> cells[FLIGHT == 0 ? kGroupBlock / 32 : 1];
+    Sums& S = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, r = lane % R, sub = lane / R;
+    const uint32_t warp = blockIdx.x * (kGroupBlock / 32) + (threadIdx.x >> 5);
+    const float4* __restrict__ pos = in.pts[0];
+    uint32_t* const idx = scratch + size_t(warp) * R * in.list[0].cap + r;
     uint32_t compressed = 0, longest = 0;
-    if (row < p.n) {  // whole warps
-        const uint32_t i = fl.particle(row);
+    if (warp * R < p.n) {  // whole warps
+        const uint32_t row = warp * R + r;
+        const bool valid = row < p.n;
+        const uint32_t i = valid ? in.list[0].particle(row) : 0u;
         const float4 a = pos[i];
         const int3 cell = cell_of(p, a.x, a.y, a.z);
-        const uint32_t nf = warp_list_near(p, fg, pos, cell, a.x, a.y, a.z, fl, row, lane);
-        const uint32_t nw = warp_list_near(p, wg, walls, cell, a.x, a.y, a.z, wl, row, lane);
-        if (lane == 0) {
-            fl.count[row] = nf;
-            wl.count[row] = nw;
-        }
-        longest = nf > nw ? nf : nw;
-        __syncwarp();  // the entries other lanes wrote
-        float sum = 0.0f, wsum = 0.0f;
-        float sx = 0.0f, sy = 0.0f, sz = 0.0f, squares = 0.0f;
-        const uint32_t mf = nf < fl.cap ? nf : fl.cap, mw = nw < wl.cap ? nw : wl.cap;
-        for (uint32_t k0 = 0; k0 < mf; k0 += 32u) {
-            const uint32_t k = k0 + lane;
-            float v = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f, sq = 0.0f;
-            if (k < mf) {
-                uint2* ent = fl.e + fl.at(row, k);
-                const uint32_t j = ent->x;
-                const float4 q = __ldg(&pos[j]);
-                float ox = q.x - a.x, oy = q.y - a.y, oz = q.z - a.z;
-                float d = sqrtf(dot3(ox, oy, oz, ox, oy, oz));
-                v = kernel_value(p, d);
-                float g = d <= 0.0f ? 0.0f : kernel_slope(p, d) / d;
-                if (SOLVER == 1) {
-                    float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
-                    float gx = rx * g, gy = ry * g, gz = rz * g;
-                    if (fl.gv) fl.gv[fl.at(row, k)] = make_float4(gx, gy, gz, __uint_as_float(j));
-                    px = gx * p.mass, py = gy * p.mass, pz = gz * p.mass;
-                    sq = dot3(px, py, pz, px, py, pz);
+        float acc[Sums::kRounds], sums[2] = {0.0f, 0.0f}, out[NC];
+#pragma unroll
+        for (int q = 0; q < Sums::kRounds; ++q) acc[q] = 0.0f;
+#pragma unroll 1
+        for (int w = 0; w < 2; ++w) {  // the fluid, then the walls
+            const PairLists& l = in.list[w];
+            const float4* __restrict__ pts = in.pts[w];
+            uint32_t found;
+            if constexpr (FLIGHT == 0)
+                found = scan_near_group<L>(p, in.grid[w], pts, valid, cell, a.x, a.y, a.z, idx, l.cap, lane,
+                                           cells[threadIdx.x >> 5]);
+            else
+                found = scan_cells_group<L, FLIGHT>(p, in.grid[w], pts, valid, cell, a.x, a.y, a.z, idx, l.cap, lane);
+            if (valid && sub == 0) l.count[row] = found;
+            longest = max(longest, found);
+            const uint32_t m = valid ? min(found, l.cap) : 0u, most = __reduce_max_sync(0xffffffffu, m);
+            __syncwarp();  // the indices the row's other lanes wrote
+#pragma unroll 1
+            for (uint32_t k0 = 0; k0 < most; k0 += Sums::kChunk) {
+                // whole rounds of 2 L pairs, so every term that is added was put
+                const uint32_t here = min(most - k0, uint32_t(Sums::kChunk));
+#pragma unroll 1
+                for (uint32_t round = 0; round < here; round += 2u * L) {
+                    const uint32_t k = k0 + round + sub;
+                    uint32_t j[2];
+                    float4 q[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) j[u] = k + u * L < m ? idx[size_t(k + u * L) * R] : 0u;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) q[u] = k + u * L < m ? __ldg(&pts[j[u]]) : a;
+                    const f32x2 ox = pack2(q[0].x - a.x, q[1].x - a.x), oy = pack2(q[0].y - a.y, q[1].y - a.y),
+                                oz = pack2(q[0].z - a.z, q[1].z - a.z);
+                    f32x2 value;
+                    float g[2], v[2], gx[2] = {0.0f, 0.0f}, gy[2] = {0.0f, 0.0f}, gz[2] = {0.0f, 0.0f};
+                    kernel_pair(p, sum2(p, sum2(p, mul2(ox, ox), mul2(oy, oy)), mul2(oz, oz)), value, g[0], g[1]);
+                    unpack2(value, v[0], v[1]);
+                    if (SOLVER == 1) {
+                        const f32x2 ng = pack2(-g[0], -g[1]);  // (at - other) g, as pair_terms forms it
+                        unpack2(mul2(ox, ng), gx[0], gx[1]);
+                        unpack2(mul2(oy, ng), gy[0], gy[1]);
+                        unpack2(mul2(oz, ng), gz[0], gz[1]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const uint32_t ku = k + u * L;
+                        const bool there = ku < m;
+                        if (there) l.e[l.at(row, ku)] = make_uint2(j[u], __float_as_uint(g[u]));
+                        S.put(r, 0, ku - k0, there ? v[u] : 0.0f);
+                        if (SOLVER == 1) {
+                            if (there && l.gv)
+                                l.gv[l.at(row, ku)] =
+                                    make_float4(gx[u], gy[u], gz[u], w == 1 ? 0.0f : __uint_as_float(j[u]));
+                            // factors (dfsph.rs:149-153); walls add no squares
+                            const float px = there ? gx[u] * p.mass : 0.0f, py = there ? gy[u] * p.mass : 0.0f,
+                                        pz = there ? gz[u] * p.mass : 0.0f;
+                            S.put(r, X, ku - k0, px);
+                            S.put(r, Y, ku - k0, py);
+                            S.put(r, Z, ku - k0, pz);
+                            S.put(r, Q, ku - k0, w == 0 ? dot3(px, py, pz, px, py, pz) : 0.0f);
+                        }
+                    }
                 }
-                *ent = make_uint2(j, __float_as_uint(g));
+                S.template add<false>(acc, lane, here);
             }
-            const uint32_t here = mf - k0 < 32u ? mf - k0 : 32u;
-            for (uint32_t t = 0; t < here; ++t) {
-                sum += __shfl_sync(0xffffffffu, v, t);
-                if (SOLVER == 1) {
-                    sx = sx + __shfl_sync(0xffffffffu, px, t);
-                    sy = sy + __shfl_sync(0xffffffffu, py, t);
-                    sz = sz + __shfl_sync(0xffffffffu, pz, t);
-                    squares += __shfl_sync(0xffffffffu, sq, t);
-                }
-            }
-        }
-        for (uint32_t k0 = 0; k0 < mw; k0 += 32u) {
-            const uint32_t k = k0 + lane;
-            float v = 0.0f, px = 0.0f, py = 0.0f, pz = 0.0f;
-            if (k < mw) {
-                uint2* ent = wl.e + wl.at(row, k);
-                const uint32_t j = ent->x;
-                const float4 q = __ldg(&walls[j]);
-                float ox = q.x - a.x, oy = q.y - a.y, oz = q.z - a.z;
-                float d = sqrtf(dot3(ox, oy, oz, ox, oy, oz));
-                v = kernel_value(p, d);
-                float g = d <= 0.0f ? 0.0f : kernel_slope(p, d) / d;
-                if (SOLVER == 1) {
-                    float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
-                    float gx = rx * g, gy = ry * g, gz = rz * g;
-                    if (wl.gv) wl.gv[wl.at(row, k)] = make_float4(gx, gy, gz, 0.0f);
-                    px = gx * p.mass, py = gy * p.mass, pz = gz * p.mass;
-                }
-                *ent = make_uint2(j, __float_as_uint(g));
-            }
-            const uint32_t here = mw - k0 < 32u ? mw - k0 : 32u;
-            for (uint32_t t = 0; t < here; ++t) {
-                wsum += __shfl_sync(0xffffffffu, v, t);
-                if (SOLVER == 1) {
-                    sx = sx + __shfl_sync(0xffffffffu, px, t);
-                    sy = sy + __shfl_sync(0xffffffffu, py, t);
-                    sz = sz + __shfl_sync(0xffffffffu, pz, t);
-                }
-            }
+            S.spread(acc, lane, int(r), out);
+            sums[w] = out[0];
+#pragma unroll
+            for (int q = 0; q < Sums::kRounds; ++q)
+                if ((lane + 32u * q) % uint32_t(NC) == 0u) acc[q] = 0.0f;  // the walls' values sum on their own
         }
         // the coupled bodies' points, in their list order (mod.rs:648-656)
         float msum = 0.0f;
-        if (M.count)
+        if (BODIES && valid && sub == 0)
             each_near(p, M.grid, M.pos, cell, a.x, a.y, a.z, [&](uint32_t, float4 q) {
                 float ox = q.x - a.x, oy = q.y - a.y, oz = q.z - a.z;
                 msum += kernel_value(p, sqrtf(dot3(ox, oy, oz, ox, oy, oz)));
             });
-        float3 gslope;
-        float ground = T.regions ? ground_near(T, a.x, a.y, a.z, gslope) : 0.0f;
-        float density = p.mass * (sum + wsum + msum) + ground;
-        if (lane == 0) {
+        if (valid && sub == 0) {
+            float density = p.mass * (sums[0] + sums[1] + msum) + 0.0f;  // no ground
             rho[i] = density;
-            if (slope) slope[i] = make_float4(gslope.x, gslope.y, gslope.z, 0.0f);
             if (SOLVER == 0) {
                 float ratio = fminf(density / p.rest, 1.1f);
                 float pressure = fmaxf(p.stiffness * (pow7(ratio) - 1.0f), 0.0f);
                 press[i] = pressure;
-                scaled[i] = pressure / (density * density);
+                const float over = pressure > 0.0f ? pressure / (density * density) : 0.0f;
+                scaled[i] = over;
+                rec.pos_w[4 * size_t(i) + 3] = over;
             } else {
-                float total = dot3(sx, sy, sz, sx, sy, sz) + squares;
+                float total = dot3(out[X], out[Y], out[Z], out[X], out[Y], out[Z]) + out[Q];
                 alpha[i] = total > 0.0f ? 1.0f / total : 0.0f;
             }
+            rec.vel_w[4 * size_t(i) + 3] = density;
+            float c = density / p.rest - 1.0f;
+            if (c > 0.0f) compressed = max(compressed, __float_as_uint(c));
         }
-        float c = density / p.rest - 1.0f;
-        if (c > 0.0f) compressed = __float_as_uint(c);
     }
     compressed = block_reduce(compressed, MaxU(), 0u);
     longest = block_reduce(longest, MaxU(), 0u);
@@ -1236,124 +1437,141 @@ __global__ void k_cells_wet(GridDev g, int3 lo, int3 hi, uint32_t* wet) {
 
 // ---- WCSPH: forces, velocity update and advance in one pass (step.rs:159-223, 305-339) -----
 
-// Subtracts, in list order, every lane's (tx, ty, tz) of this round from (px, py, pz): lane t's
-// term after lane t - 1's, as the one-thread walk subtracts them.  A lane without a term holds
-// +0, whose subtraction leaves any value as it was.
-__device__ __forceinline__ void take_in_order(float& px, float& py, float& pz, float tx, float ty, float tz,
-                                              uint32_t here) {
-    for (uint32_t t = 0; t < here; ++t) {
-        px = px - __shfl_sync(0xffffffffu, tx, t);
-        py = py - __shfl_sync(0xffffffffu, ty, t);
-        pz = pz - __shfl_sync(0xffffffffu, tz, t);
-    }
-}
-
-// The WCSPH force and advance pass for scenes too small to fill the GPU a thread a particle
-// (k_density_warp made the lists): a warp a row, the pair terms a lane a neighbour, subtracted in
-// list order, so every sum is k_wcsph_force's bit for bit; lane 0 advances the particle.  Without
-// terrain or coupled bodies (their terms stay with k_wcsph_force).
-__global__ void __launch_bounds__(kBlock) k_wcsph_force_warp(Params p, const StepConsts* __restrict__ sc, PairLists fl,
-                                                             PairLists wl, const float4* __restrict__ pos,
-                                                             const float4* __restrict__ vel,
-                                                             const float* __restrict__ rho,
-                                                             const float* __restrict__ press,
-                                                             const float* __restrict__ scaled,
-                                                             const float4* __restrict__ walls,
-                                                             float4* __restrict__ pos_out, float4* __restrict__ vel_out,
-                                                             Status* st, float4* __restrict__ vel_pre) {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    const bool valid = row < p.n;  // whole warps
-    int3 nc = make_int3(0, 0, 0);
-    float speed = 0.0f;
+// k_wcsph_force by L lanes a row.
+template <bool BODIES, int L>
+__global__ void __launch_bounds__(kGroupBlock)
+    k_wcsph_force_group(Params p, const StepConsts* __restrict__ sc, PairLists fl, PairLists wl,
+                        const float4* __restrict__ pos, const float4* __restrict__ vel, const float* __restrict__ rho,
+                        const float* __restrict__ press, const float* __restrict__ scaled,
+                        const float4* __restrict__ walls, float4* __restrict__ pos_out, float4* __restrict__ vel_out,
+                        Status* st, float4* __restrict__ vel_pre, MoverDev M) {
+    using Sums = GroupSums<L, 3>;
+    constexpr uint32_t R = Sums::kRows;
+    __shared__ __align__(16) Sums shared[kGroupBlock / 32];
+    Sums& S = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, r = lane % R, sub = lane / R;
+    const uint32_t warp = blockIdx.x * (kGroupBlock / 32) + (threadIdx.x >> 5);
+    int3 lo = make_int3(INT_MAX, INT_MAX, INT_MAX), hi = make_int3(INT_MIN, INT_MIN, INT_MIN);
+    float fastest = 0.0f;
     uint32_t held = 0, bad = 0;
-    if (valid) {
-        const uint32_t i = fl.particle(row);
-        const float dt = sc->dt;
-        const float visc = sc->viscosity;
+    const float dt = sc->dt, visc = sc->viscosity, wall_visc = sc->wall_viscosity;
+    if (warp * R < p.n) {  // whole warps
+        const uint32_t row = warp * R + r;
+        const bool valid = row < p.n;
+        const uint32_t i = valid ? fl.particle(row) : 0u;
         float4 a = pos[i];
         float4 v = vel[i];
-        const float density = rho[i];
-        const float own = scaled[i];
-        float px = 0.0f, py = 0.0f, pz = 0.0f;
-        const uint32_t nf = fl.count[row], nw = wl.count[row];
-        const uint32_t mf = nf < fl.cap ? nf : fl.cap, mw = nw < wl.cap ? nw : wl.cap;
-        for (uint32_t k0 = 0; k0 < mf; k0 += 32u) {
-            const uint32_t k = k0 + lane;
-            float tx = 0.0f, ty = 0.0f, tz = 0.0f;
-            if (k < mf) {
-                const uint2 en = SLF_LIST_LOAD(fl.e + fl.at(row, k));
-                const uint32_t j = en.x;
-                const float g = __uint_as_float(en.y);
-                const float4 q = __ldg(&pos[j]), w = __ldg(&vel[j]);
-                float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
-                float squared = dot3(rx, ry, rz, rx, ry, rz);
-                if (squared > 0.0f) {
-                    float gx = rx * g, gy = ry * g, gz = rz * g;
-                    float toward = fminf(dot3(v.x - w.x, v.y - w.y, v.z - w.z, rx, ry, rz), 0.0f);
-                    float damp = -visc * toward / (squared + p.soften) * 2.0f / (density + __ldg(&rho[j]));
-                    float s = p.mass * (own + __ldg(&scaled[j]) + damp);
-                    tx = gx * s, ty = gy * s, tz = gz * s;
+        const float density = rho[i], own = scaled[i];
+        // every row's terms, in list order: term(k, entry, tx, ty, tz) for the row's k-th entry, and
+        // the chains take what this round put
+        auto walk = [&](const PairLists& l, auto negate, float(&acc)[Sums::kRounds], auto&& term) {
+            const uint32_t m = valid ? min(l.count[row], l.cap) : 0u, most = __reduce_max_sync(0xffffffffu, m);
+#pragma unroll 1
+            for (uint32_t k0 = 0; k0 < most; k0 += Sums::kChunk) {
+                const uint32_t here = min(most - k0, uint32_t(Sums::kChunk));
+#pragma unroll 1
+                for (uint32_t round = 0; round < here; round += 2u * L) {
+                    const uint32_t k = k0 + round + sub;
+                    uint2 en[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+                        en[u] = k + u * L < m ? SLF_LIST_LOAD(l.e + l.at(row, k + u * L)) : make_uint2(0u, 0u);
+                    float t[2][3];
+                    term(en, t);
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const bool there = k + u * L < m;
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) S.put(r, c, round + sub + u * L, there ? t[u][c] : 0.0f);
+                    }
                 }
+                S.template add<decltype(negate)::value>(acc, lane, here);
             }
-            take_in_order(px, py, pz, tx, ty, tz, mf - k0 < 32u ? mf - k0 : 32u);
-        }
-        const float mirrored = own + press[i] / p.rest_sq;
+            return most;
+        };
+        float push[Sums::kRounds] = {}, away[Sums::kRounds] = {}, damped[Sums::kRounds] = {};
+        walk(fl, std::true_type{}, push, [&](const uint2(&en)[2], float(&t)[2][3]) {
+            float4 q[2], w[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) q[u] = __ldg(&pos[en[u].x]), w[u] = __ldg(&vel[en[u].x]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float g = __uint_as_float(en[u].y);
+                float rx = a.x - q[u].x, ry = a.y - q[u].y, rz = a.z - q[u].z;
+                float squared = dot3(rx, ry, rz, rx, ry, rz);
+                float gx = rx * g, gy = ry * g, gz = rz * g;
+                float toward = dot3(v.x - w[u].x, v.y - w[u].y, v.z - w[u].z, rx, ry, rz);
+                float damp = 0.0f;  // a pair that parts is not damped: no division of a zero
+                if (toward < 0.0f) damp = -visc * toward / (squared + p.soften) * 2.0f / (density + w[u].w);
+                float s = p.mass * (own + q[u].w + damp);
+                const bool pair = squared > 0.0f;
+                t[u][0] = pair ? gx * s : 0.0f, t[u][1] = pair ? gy * s : 0.0f, t[u][2] = pair ? gz * s : 0.0f;
+            }
+        });
+        const float mirrored = own + (press[i] > 0.0f ? press[i] / p.rest_sq : 0.0f);
         // the walls' pressure, then wall_viscous's two walks (its normal, then its damping)
-        float awx = 0.0f, awy = 0.0f, awz = 0.0f;
-        for (uint32_t k0 = 0; k0 < mw; k0 += 32u) {
-            const uint32_t k = k0 + lane;
-            float tx = 0.0f, ty = 0.0f, tz = 0.0f, nx = 0.0f, ny = 0.0f, nz = 0.0f;
-            if (k < mw) {
-                const uint2 en = SLF_LIST_LOAD(wl.e + wl.at(row, k));
-                const float g = __uint_as_float(en.y);
-                const float4 q = __ldg(&walls[en.x]);
+        const uint32_t walled = walk(wl, std::true_type{}, push, [&](const uint2(&en)[2], float(&t)[2][3]) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float g = __uint_as_float(en[u].y);
+                const float4 q = __ldg(&walls[en[u].x]);
                 float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
                 float s = p.mass * mirrored;
-                tx = (rx * g) * s, ty = (ry * g) * s, tz = (rz * g) * s;
-                nx = -(rx * g), ny = -(ry * g), nz = -(rz * g);
+                t[u][0] = (rx * g) * s, t[u][1] = (ry * g) * s, t[u][2] = (rz * g) * s;
             }
-            const uint32_t here = mw - k0 < 32u ? mw - k0 : 32u;
-            take_in_order(px, py, pz, tx, ty, tz, here);
-            for (uint32_t t = 0; t < here; ++t) {
-                awx = awx + __shfl_sync(0xffffffffu, nx, t);
-                awy = awy + __shfl_sync(0xffffffffu, ny, t);
-                awz = awz + __shfl_sync(0xffffffffu, nz, t);
-            }
-        }
-        float wx = 0.0f, wy = 0.0f, wz = 0.0f;
-        if (nw != 0) {
+        });
+        float sum[3], wall[3] = {0.0f, 0.0f, 0.0f};
+        S.spread(push, lane, int(r), sum);
+        if (walled) {
+            walk(wl, std::false_type{}, away, [&](const uint2(&en)[2], float(&t)[2][3]) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float g = __uint_as_float(en[u].y);
+                    const float4 q = __ldg(&walls[en[u].x]);
+                    float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
+                    t[u][0] = -(rx * g), t[u][1] = -(ry * g), t[u][2] = -(rz * g);
+                }
+            });
+            float aw[3];
+            S.spread(away, lane, int(r), aw);
             // wall_viscous (step.rs:262-301): normalize_or(ZERO) dividing by the length
-            float len = sqrtf(dot3(awx, awy, awz, awx, awy, awz));
+            float len = sqrtf(dot3(aw[0], aw[1], aw[2], aw[0], aw[1], aw[2]));
             float ux = 0.0f, uy = 0.0f, uz = 0.0f;
             if (isfinite(len) && len > 0.0f) {
-                ux = awx / len;
-                uy = awy / len;
-                uz = awz / len;
+                ux = aw[0] / len;
+                uy = aw[1] / len;
+                uz = aw[2] / len;
             }
             float kk = fminf(dot3(v.x, v.y, v.z, ux, uy, uz), 0.0f);
             float ix = ux * kk, iy = uy * kk, iz = uz * kk;
-            const float wall_visc = sc->wall_viscosity;
-            for (uint32_t k0 = 0; k0 < mw; k0 += 32u) {
-                const uint32_t k = k0 + lane;
-                float tx = 0.0f, ty = 0.0f, tz = 0.0f;
-                if (k < mw) {
-                    const uint2 en = SLF_LIST_LOAD(wl.e + wl.at(row, k));
-                    const float g = __uint_as_float(en.y);
-                    const float4 q = __ldg(&walls[en.x]);
+            walk(wl, std::true_type{}, damped, [&](const uint2(&en)[2], float(&t)[2][3]) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float g = __uint_as_float(en[u].y);
+                    const float4 q = __ldg(&walls[en[u].x]);
                     float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
                     float toward = dot3(ix, iy, iz, rx, ry, rz);
+                    t[u][0] = t[u][1] = t[u][2] = 0.0f;
                     if (toward < 0.0f) {
                         float squeeze = toward / (dot3(rx, ry, rz, rx, ry, rz) + p.soften);
                         float damp = -wall_visc * squeeze / density;
                         float s = p.mass * damp;
-                        tx = (rx * g) * s, ty = (ry * g) * s, tz = (rz * g) * s;
+                        t[u][0] = (rx * g) * s, t[u][1] = (ry * g) * s, t[u][2] = (rz * g) * s;
                     }
                 }
-                take_in_order(wx, wy, wz, tx, ty, tz, mw - k0 < 32u ? mw - k0 : 32u);
-            }
+            });
+            S.spread(damped, lane, int(r), wall);
         }
-        if (lane == 0) {
-            float ax = (px + wx) + p.gravity.x, ay = (py + wy) + p.gravity.y, az = (pz + wz) + p.gravity.z;
+        if (valid && sub == 0) {
+            float px = sum[0], py = sum[1], pz = sum[2];
+            if (BODIES)
+                mover_pairs(p, M, sc->mover_damping, a, v, density, mirrored,
+                            [&](uint32_t, float gx, float gy, float gz, float s, float, float) {
+                                px = px - gx * s;
+                                py = py - gy * s;
+                                pz = pz - gz * s;
+                            });
+            float ax = (px + wall[0]) + p.gravity.x, ay = (py + wall[1]) + p.gravity.y, az = (pz + wall[2]) + p.gravity.z;
             v.x = v.x + ax * dt;
             v.y = v.y + ay * dt;
             v.z = v.z + az * dt;
@@ -1367,15 +1585,24 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_force_warp(Params p, const Ste
             }
             pos_out[i] = a;
             vel_out[i] = v;
-            nc = cell_of(p, a.x, a.y, a.z);
-            speed = sqrtf(dot3(v.x, v.y, v.z, v.x, v.y, v.z));
-            if (!(speed == speed)) speed = 0.0f;
+            const int3 nc = cell_of(p, a.x, a.y, a.z);
+            lo = make_int3(min(lo.x, nc.x), min(lo.y, nc.y), min(lo.z, nc.z));
+            hi = make_int3(max(hi.x, nc.x), max(hi.y, nc.y), max(hi.z, nc.z));
+            fastest = fmaxf(fastest, sqrtf(dot3(v.x, v.y, v.z, v.x, v.y, v.z)));
         }
     }
-    fold_advance_stats(st, valid && lane == 0, nc, speed, held, bad);
+    fold_advance_box(st, lo, hi, fastest, held, bad);
 }
 
-__global__ void __launch_bounds__(kBlock, SLF_PAIR_MIN_BLOCKS) k_wcsph_force(Params p, const StepConsts* __restrict__ sc, PairLists fl,
+// A thread a row, rows of the walk order a grid's width apart.  One 16-byte gather brings a
+// neighbour's position and p / rho^2, another its velocity and density (four gathers before), and a
+// pair that moves apart divides nothing: 157 -> 68 us at 262k particles (measured 157 -> 96 at 314k
+// by the gathers and three blocks of 80 registers a SM; four blocks spill, 108; two 124), then
+// 86 -> 68 at 262k and 249 -> 155 at 47k, support 4, by the division of zero (its slow path ran for
+// half of all pairs).  EXTRA: terrain regions or
+// coupled bodies add their terms.
+template <bool EXTRA>
+__global__ void __launch_bounds__(kBlock, 3) k_wcsph_force(Params p, const StepConsts* __restrict__ sc, PairLists fl,
                                                         PairLists wl, const float4* __restrict__ pos,
                                                         const float4* __restrict__ vel, const float* __restrict__ rho,
                                                         const float* __restrict__ press,
@@ -1384,13 +1611,11 @@ __global__ void __launch_bounds__(kBlock, SLF_PAIR_MIN_BLOCKS) k_wcsph_force(Par
                                                         float4* __restrict__ vel_out, Status* st,
                                                         float4* __restrict__ vel_pre, TerrainDev T,
                                                         const float4* __restrict__ slope, MoverDev M) {
-    uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t i = row < p.n ? fl.particle(row) : row;  // row of the walk order, its particle
-    bool valid = i < p.n;
-    int3 nc = make_int3(0, 0, 0);
-    float speed = 0.0f;
+    int3 lo = make_int3(INT_MAX, INT_MAX, INT_MAX), hi = make_int3(INT_MIN, INT_MIN, INT_MIN);
+    float fastest = 0.0f;
     uint32_t held = 0, bad = 0;
-    if (valid) {
+    for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < p.n; row += gridDim.x * blockDim.x) {
+        const uint32_t i = fl.particle(row);
         const float dt = sc->dt;
         const float visc = sc->viscosity;
         float4 a = pos[i];
@@ -1398,20 +1623,22 @@ __global__ void __launch_bounds__(kBlock, SLF_PAIR_MIN_BLOCKS) k_wcsph_force(Par
         float density = rho[i];
         float own = scaled[i];
         float px = 0.0f, py = 0.0f, pz = 0.0f;
-        each_listed2(fl, row, pos, vel, [&](uint32_t j, float g, float4 q, float4 w) {
+        each_listed2(fl, row, pos, vel, [&](uint32_t, float g, float4 q, float4 w) {
             float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
             float squared = dot3(rx, ry, rz, rx, ry, rz);
             if (squared <= 0.0f) return;
-            // g = slope(distance) / distance with distance = sqrt(squared) > 0
+            // g = slope(distance) / distance with distance = sqrt(squared) > 0; q.w is the
+            // neighbour's p / rho^2 and w.w its density (the density pass put them there)
             float gx = rx * g, gy = ry * g, gz = rz * g;
-            float toward = fminf(dot3(v.x - w.x, v.y - w.y, v.z - w.z, rx, ry, rz), 0.0f);
-            float damp = -visc * toward / (squared + p.soften) * 2.0f / (density + __ldg(&rho[j]));
-            float s = p.mass * (own + __ldg(&scaled[j]) + damp);
+            float toward = dot3(v.x - w.x, v.y - w.y, v.z - w.z, rx, ry, rz);
+            float damp = 0.0f;  // a pair that parts is not damped: no division of a zero
+            if (toward < 0.0f) damp = -visc * toward / (squared + p.soften) * 2.0f / (density + w.w);
+            float s = p.mass * (own + q.w + damp);
             px = px - gx * s;
             py = py - gy * s;
             pz = pz - gz * s;
         });
-        float mirrored = own + press[i] / p.rest_sq;
+        float mirrored = own + (press[i] > 0.0f ? press[i] / p.rest_sq : 0.0f);
         each_listed(wl, row, walls, [&](uint32_t, float g, float4 q) {
             float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
             float s = p.mass * mirrored;
@@ -1419,27 +1646,28 @@ __global__ void __launch_bounds__(kBlock, SLF_PAIR_MIN_BLOCKS) k_wcsph_force(Par
             py = py - (ry * g) * s;
             pz = pz - (rz * g) * s;
         });
-        if (slope) {  // the ground pushes back with this particle's own pressure (step.rs:203-205)
+        if (EXTRA && slope) {  // the ground pushes back with this particle's own pressure (step.rs:203-205)
             float4 sl = slope[i];
             px = px - sl.x * mirrored;
             py = py - sl.y * mirrored;
             pz = pz - sl.z * mirrored;
         }
-        if (M.count)
+        if (EXTRA && M.count)
             mover_pairs(p, M, sc->mover_damping, a, v, density, mirrored,
                         [&](uint32_t, float gx, float gy, float gz, float s, float, float) {
                             px = px - gx * s;
                             py = py - gy * s;
                             pz = pz - gz * s;
                         });
-        float3 wv = wall_viscous(p, sc->wall_viscosity, wl, walls, row, a, v, density, T);
+        TerrainDev none{};
+        float3 wv = wall_viscous(p, sc->wall_viscosity, wl, walls, row, a, v, density, EXTRA ? T : none);
         float ax = (px + wv.x) + p.gravity.x, ay = (py + wv.y) + p.gravity.y, az = (pz + wv.z) + p.gravity.z;
         v.x = v.x + ax * dt;
         v.y = v.y + ay * dt;
         v.z = v.z + az * dt;
         float4 pre = v;
         uint32_t flags = 0;
-        advance_one(p, dt, a, v, held, bad, T, &flags);
+        advance_one(p, dt, a, v, held, bad, EXTRA ? T : none, &flags);
         if (vel_pre) {
             // the velocity before the wall zeroed any component, and which ones it zeroed
             pre.w = __uint_as_float(flags);
@@ -1447,11 +1675,13 @@ __global__ void __launch_bounds__(kBlock, SLF_PAIR_MIN_BLOCKS) k_wcsph_force(Par
         }
         pos_out[i] = a;
         vel_out[i] = v;
-        nc = cell_of(p, a.x, a.y, a.z);
-        speed = sqrtf(dot3(v.x, v.y, v.z, v.x, v.y, v.z));
-        if (!(speed == speed)) speed = 0.0f;
+        const int3 nc = cell_of(p, a.x, a.y, a.z);
+        lo = make_int3(min(lo.x, nc.x), min(lo.y, nc.y), min(lo.z, nc.z));
+        hi = make_int3(max(hi.x, nc.x), max(hi.y, nc.y), max(hi.z, nc.z));
+        const float speed = sqrtf(dot3(v.x, v.y, v.z, v.x, v.y, v.z));
+        fastest = fmaxf(fastest, speed);  // (a NaN speed is ignored, as f32::max does)
     }
-    fold_advance_stats(st, valid, nc, speed, held, bad);
+    fold_advance_box(st, lo, hi, fastest, held, bad);
 }
 
 // ---- DFSPH ----------------------------------------------------------------------------------
@@ -1494,12 +1724,13 @@ __device__ __forceinline__ void rate_particle(const Params& p, const StepConsts*
     float target, error;
     if (WHICH == 1) {
         float over = fmaxf(rho[i] + dt * rate - p.rest, 0.0f);
-        target = over / sc->dt_sq;
-        error = over / p.rest;
+        // (a quotient of zero is zero, and its division would take the slow path)
+        target = over > 0.0f ? over / sc->dt_sq : 0.0f;
+        error = over > 0.0f ? over / p.rest : 0.0f;
     } else {
         float r = fl.count[row] + wl.count[row] < 20u ? 0.0f : fmaxf(rate, 0.0f);
-        target = r / dt;
-        error = dt * r / p.rest;
+        target = r > 0.0f ? r / dt : 0.0f;
+        error = r > 0.0f ? dt * r / p.rest : 0.0f;
     }
     // the stiffness rides in the spare lane of the position, where push_apart gathers it
     kappa_w[4 * (size_t)i + 3] = target * alpha[i];
@@ -1598,7 +1829,7 @@ __device__ __forceinline__ void viscous_particle(const Params& p, const StepCons
         float toward = dot3(v.x - w.x, v.y - w.y, v.z - w.z, rx, ry, rz);
         if (toward < 0.0f) {
             float squeeze = toward / (dot3(rx, ry, rz, rx, ry, rz) + p.soften);
-            float damp = -visc * squeeze * 2.0f / (density + __ldg(&rho[j]));
+            float damp = -visc * squeeze * 2.0f / (density + w.w);  // the neighbour's density (PairRecords)
             float s = p.mass * damp;
             px = px - (rx * g) * s;
             py = py - (ry * g) * s;
@@ -1905,23 +2136,28 @@ static inline uint32_t blocks_for(uint32_t n) {
 #ifndef SLF_SOLVER_RESIDENT
 #define SLF_SOLVER_RESIDENT 1
 #endif
-// resident blocks of k_rate<0>, k_rate<1>, k_push, k_density<0>, k_density<1>, k_viscous on the
+// resident blocks of k_rate<0>, k_rate<1>, k_push, k_density<0>, k_density<1>, k_viscous, k_wcsph_force on the
 // device (prepare_solver_grids; 0: not known yet, the grid then covers every row)
-static std::atomic<uint32_t> g_resident[6] = {0, 0, 0, 0, 0, 0};
+static std::atomic<uint32_t> g_resident[7] = {0, 0, 0, 0, 0, 0, 0};
+
+// blocks of the density pass up to which it runs wide: two a SM
+static std::atomic<uint32_t> g_wide_blocks{0};
 
 void prepare_solver_grids() {
     if (!SLF_SOLVER_RESIDENT || g_resident[2].load()) return;
-    int dev = 0, sms = 0, per[6] = {0, 0, 0, 0, 0, 0};
+    int dev = 0, sms = 0, per[7] = {0, 0, 0, 0, 0, 0, 0};
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0], k_rate<0>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1], k_rate<1>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[2], k_push, kBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[3], k_density<0, true>, kBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[4], k_density<1, false>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[3], k_density<0, true, false>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[4], k_density<1, false, false>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[5], k_viscous, kBlock, 0);
-    for (int k = 0; k < 6; ++k) g_resident[k].store(uint32_t(std::max(per[k], 0) * std::max(sms, 0)));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[6], k_wcsph_force<true>, kBlock, 0);
+    g_wide_blocks.store(2u * uint32_t(std::max(sms, 0)));
+    for (int k = 0; k < 7; ++k) g_resident[k].store(uint32_t(std::max(per[k], 0) * std::max(sms, 0)));
 }
 
 static uint32_t solver_blocks(uint32_t n, int kernel) {
@@ -1990,37 +2226,80 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
                                                         skip_begin, skip_end, st, dest, span, order);
 }
 
-size_t density_scratch_words(uint32_t n, uint32_t cap) {
+// blocks of a pass that gives each row `lanes` lanes
+static uint32_t group_blocks(uint32_t n, int lanes) {
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    const uint32_t rows = uint32_t(kGroupBlock / lanes);
+    return (n + rows - 1) / rows;
+}
+
+// calls f with the number of lanes as a constant; false for none (a thread a row)
+template <class F>
+static bool with_lanes(int lanes, F&& f) {
+    switch (lanes) {
+        case 4: f(std::integral_constant<int, 4>{}); return true;
+        case 8: f(std::integral_constant<int, 8>{}); return true;
+        case 16: f(std::integral_constant<int, 16>{}); return true;
+        case 32: f(std::integral_constant<int, 32>{}); return true;
+        default: return false;
+    }
+}
+
+size_t density_scratch_words(uint32_t n, uint32_t cap, float support) {
     // one list room a thread of the density pass's grid
     const uint32_t nb = (n + kBlock - 1) / kBlock, r0 = g_resident[3].load(), r1 = g_resident[4].load();
     const uint32_t resident = r0 && r1 ? std::max(r0, r1) : nb;
-    return size_t(std::min(resident, nb)) * kBlock * cap;
+    // (with lanes to share, a list room a row of the grid, whose last tile may be part empty)
+    const size_t group = group_lanes(n, support) ? size_t(n + kGroupBlock) : 0;
+    return std::max(size_t(std::min(resident, nb)) * kBlock, group) * cap;
 }
 
-void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, const float4* pos, const float4* walls,
+void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float4* pos, const float4* walls,
                     const PairLists& fl, const PairLists& wl, float* rho, float* press, float* scaled, float* alpha,
                     Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M,
-                    uint32_t* scratch) {
+                    uint32_t* scratch, float4* vel) {
     if (!p.n) return;
-    if (warp_rows(p.n, p.radius, p.spacing) && T.regions == 0 && M.count == 0) {
-        // a scene this small leaves most SMs idle a thread a particle: a warp a particle (terrain
-        // and body points, which every lane would take alike, stay a thread a particle)
-        if (p.solver == 0)
-            k_density_warp<0><<<blocks_for(p.n * 32u), kBlock, 0, s>>>(p, fg, wg, pos, walls, fl, wl, rho, press,
-                                                                       scaled, alpha, st, T, slope, M);
-        else
-            k_density_warp<1><<<blocks_for(p.n * 32u), kBlock, 0, s>>>(p, fg, wg, pos, walls, fl, wl, rho, press,
-                                                                       scaled, alpha, st, T, slope, M);
-        return;
-    }
-    const uint32_t nb = solver_blocks(p.n, p.solver == 0 ? 3 : 4);
+    const PairRecords rec{reinterpret_cast<float*>(pos), reinterpret_cast<float*>(vel)};
     const DensityIn in{{fg, wg}, {pos, walls}, {fl, wl}};
-    if (p.solver != 0)  // DFSPH takes neither terrain nor bodies
-        k_density<1, false><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch);
-    else if (T.regions || M.count || slope)
-        k_density<0, true><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch);
-    else
-        k_density<0, false><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch);
+    if (T.regions == 0 && slope == nullptr && with_lanes(group_lanes(p.n, p.radius / p.spacing), [&](auto lanes) {
+            constexpr int L = decltype(lanes)::value;
+            const uint32_t nb = group_blocks(p.n, L);
+            auto launch = [&](auto flight) {
+                constexpr int F = decltype(flight)::value;
+                if (p.solver != 0)  // DFSPH takes no bodies
+                    k_density_group<1, false, L, F><<<nb, kGroupBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, M,
+                                                                               scratch, rec);
+                else if (M.count)
+                    k_density_group<0, true, L, F><<<nb, kGroupBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, M,
+                                                                              scratch, rec);
+                else
+                    k_density_group<0, false, L, F><<<nb, kGroupBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, M,
+                                                                               scratch, rec);
+            };
+            // a cell's points at rest: few enough of them, L lanes test the 27 cells end to end (216
+            // candidates at support 2, L = 32, 1000 particles: 27 -> 15 us against a cell at a time);
+            // many, and a lane keeps four of a cell's in flight (64 at support 4, L = 4, 74k
+            // particles: 293 -> 273 us against two, at support 2 73 -> 90)
+            const float support = p.radius / p.spacing, points = support * support * support;
+            if constexpr (L >= 8) {
+                if (points <= 2.0f * L) return launch(std::integral_constant<int, 0>{});
+            }
+            if (points < 16.0f) launch(std::integral_constant<int, 2>{});
+            else launch(std::integral_constant<int, 4>{});
+        }))
+        return;
+    const uint32_t nb = solver_blocks(p.n, p.solver == 0 ? 3 : 4);
+    auto launch = [&](auto wide) {
+        constexpr bool W = decltype(wide)::value;
+        if (p.solver != 0)  // DFSPH takes neither terrain nor bodies
+            k_density<1, false, W><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch, rec);
+        else if (T.regions || M.count || slope)
+            k_density<0, true, W><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch, rec);
+        else
+            k_density<0, false, W><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch, rec);
+    };
+    if (nb <= g_wide_blocks.load()) launch(std::true_type{});
+    else launch(std::false_type{});
 }
 
 void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,
@@ -2029,13 +2308,24 @@ void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& 
                         float4* vel_pre, const TerrainDev& T, const float4* slope, cudaStream_t s,
                         const MoverDev& M) {
     if (!p.n) return;
-    if (warp_rows(p.n, p.radius, p.spacing) && T.regions == 0 && M.count == 0 && slope == nullptr) {
-        k_wcsph_force_warp<<<blocks_for(p.n * 32u), kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, press, scaled,
-                                                                    walls, pos_out, vel_out, st, vel_pre);
+    if (T.regions == 0 && slope == nullptr && with_lanes(group_lanes(p.n, p.radius / p.spacing), [&](auto lanes) {
+            constexpr int L = decltype(lanes)::value;
+            const uint32_t nb = group_blocks(p.n, L);
+            if (M.count)
+                k_wcsph_force_group<true, L><<<nb, kGroupBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, press, scaled,
+                                                                        walls, pos_out, vel_out, st, vel_pre, M);
+            else
+                k_wcsph_force_group<false, L><<<nb, kGroupBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, press, scaled,
+                                                                         walls, pos_out, vel_out, st, vel_pre, M);
+        }))
         return;
-    }
-    k_wcsph_force<<<blocks_for(p.n), kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, press, scaled, walls, pos_out,
-                                                     vel_out, st, vel_pre, T, slope, M);
+    const uint32_t nb = solver_blocks(p.n, 6);
+    if (T.regions || M.count || slope)
+        k_wcsph_force<true><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, press, scaled, walls, pos_out, vel_out,
+                                                  st, vel_pre, T, slope, M);
+    else
+        k_wcsph_force<false><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, press, scaled, walls, pos_out, vel_out,
+                                                   st, vel_pre, T, slope, M);
 }
 
 void launch_mover_count(const Params& p, const StepConsts* sc, const MoverDev& M, const float4* pos,
@@ -2136,7 +2426,8 @@ __global__ void k_warm_kappa(Params p, const StepConsts* __restrict__ sc, float 
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
     const float dt = sc->dt;
-    float kappa = share * applied[2 * (size_t)i] / dt;
+    const float impulse = share * applied[2 * (size_t)i];
+    float kappa = impulse != 0.0f ? impulse / dt : impulse;
     pos[i].w = kappa;
     applied[2 * (size_t)i] = kappa * dt;
 }

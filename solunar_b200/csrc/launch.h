@@ -39,31 +39,37 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
                          int4* cells_out, const float2* warm_in, float2* warm_out, uint32_t skip_begin,
                          uint32_t skip_end, Status* st, uint32_t* dest, int3 span, uint32_t* order, cudaStream_t s);
 
-// Particle counts up to which the EXACT density pass and the WCSPH force pass, without terrain or
-// coupled bodies, run a warp a particle (k_density_warp, k_wcsph_force_warp), which then needs no
-// walk order: below one 256-thread block per SM (148 on B200) a thread a particle leaves SMs idle
-// and each thread walks its candidates in one long chain of loads.  Measured: 8k particles at
-// support 4, density 392 -> 92 us and force 218 -> 67 us; 250k and 1M particles at support 2,
-// density 219 -> 547 us and 562 -> 2250 us, so larger scenes keep a thread a particle.
-constexpr uint32_t kWarpPassMax = 32768u;
-// Scenes at support 3 and more (hundreds of neighbours, thousands of candidates a particle) may
-// keep the warp passes up to this many particles.  Off: on the 64k-particle scene at support 4
-// the density pass gained (592 -> 548 us) but the force pass lost more (239 -> 358 us).
-#ifndef SLF_WARP_PASS_WIDE_MAX
-#define SLF_WARP_PASS_WIDE_MAX 0u
-#endif
-inline bool warp_rows(uint32_t n, float radius, float spacing) {
-    return n <= kWarpPassMax || (n <= SLF_WARP_PASS_WIDE_MAX && radius >= 3.0f * spacing);
+// Lanes a row of the EXACT density pass and the WCSPH force pass (k_density_group,
+// k_wcsph_force_group) in scenes without terrain; 0: a thread a row.  A row's lanes keep the SMs
+// busy where the rows alone would not, at the price of a few more instructions a pair, so the line
+// lies where the rows fill about half of the warps the SMs hold, and further out where a row has
+// hundreds of neighbours.  Measured, density + force in us (B200; - : not near):
+//            n   support 2: thread  L=4  L=8 L=16 L=32     support 4: thread  L=4  L=8 L=16 L=32
+//         1000              65   48   38   30   28                  328  141   87   64   50
+//         5832              68   50   39   33   45                  350  155   97   79   92
+//        10648              67   52   43   48   57                  355  159  111  124  131
+//        17576              70   53   49   56   77                  363  175  141  162  188
+//        27000              71   60   70   73    -                  380  200  200  223    -
+//        46656              75   88   97    -    -                  388  333  304  347    -
+//        74088              77  109    -    -    -                  469  431  436    -    -
+//       110592              96  149    -    -    -                  617  604  630    -    -
+// (a warp a row with shuffled sums, before: 8,000 particles at support 4 83 + 66.)
+inline int group_lanes(uint32_t n, float support) {
+    if (n <= 2048u) return 32;
+    if (n <= 8192u) return support >= 3.0f && n <= 4096u ? 32 : 16;
+    if (support >= 3.0f) return n <= 57344u ? 8 : n <= 114688u ? 4 : 0;
+    return n <= 20480u ? 8 : n <= 32768u ? 4 : 0;
 }
 
 // pair passes: the density pass builds the substep's neighbour lists, the others walk them
 // T: terrain regions (regions = 0: none); slope (optional): each particle's ground density gradient
-void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, const float4* pos, const float4* walls,
+// vel: the velocities at pos, whose spare lanes take the densities (and pos's WCSPH's p / rho^2)
+void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float4* pos, const float4* walls,
                     const PairLists& fl, const PairLists& wl, float* rho, float* press, float* scaled, float* alpha,
                     Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M,
-                    uint32_t* scratch);
+                    uint32_t* scratch, float4* vel);
 // words of launch_density's scratch for n particles and lists of cap slots
-size_t density_scratch_words(uint32_t n, uint32_t cap);
+size_t density_scratch_words(uint32_t n, uint32_t cap, float support);
 // vel_pre (optional): the velocity before the wall clamp, its w lane the bits of the components
 // the clamp zeroed (1 x, 2 y, 4 z), for the adjoint
 void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,

@@ -341,7 +341,7 @@ int32_t World::ensure_work_buffers() {
     SLF_TRY(cslot.ensure(n, 0, stream));
     SLF_TRY(members.ensure(n, 0, stream));
     SLF_TRY(partials.ensure(rate_partial_bytes(uint32_t(n)), 0, stream));
-    if (!fast()) SLF_TRY(dscratch.ensure(density_scratch_words(uint32_t(n), list_cap), 0, stream));
+    if (!fast()) SLF_TRY(dscratch.ensure(density_scratch_words(uint32_t(n), list_cap, radius / s.spacing), 0, stream));
     return SLF_OK;
 }
 
@@ -352,7 +352,7 @@ void World::density_pass(const Params& p, int a, const PairLists& fl, const Pair
                             alpha.p, d_status, on);
     else
         launch_density(p, fgrid, wgrid, pos[a].p, dwalls.p, fl, wl, rh, press.p, scaled.p, alpha.p, d_status,
-                       tdev, ground_slopes(), on, mover_dev(), dscratch.p);
+                       tdev, ground_slopes(), on, mover_dev(), dscratch.p, vel[a].p);
 }
 
 void World::force_pass(const Params& p, const PairLists& fl, const PairLists& wl, int a, int b, int nid, cudaStream_t on) {
@@ -498,11 +498,10 @@ int32_t World::plan_sort(SortPlan& sp, bool stable) {
     SLF_TRY(ensure_work_buffers());
     SLF_TRY(count.ensure(size_t(sp.volume) + 1, 0, stream));
     SLF_TRY(tiles.ensure(scan_tiles(sp.volume) + 1, 0, stream));
-    // the walk order of this sort's lists (none where every pass over the lists runs a warp a
-    // particle)
-    bool warp_passes = !fast() && s.solver == SLF_SOLVER_WCSPH && warp_rows(uint32_t(n), radius, s.spacing) &&
-                       terrains.empty() && m_pos.empty();
-    sp.ordered = !warp_passes;
+    // the walk order of this sort's lists (none where every pass over the lists gives a row
+    // several lanes)
+    bool shared_rows = !fast() && s.solver == SLF_SOLVER_WCSPH && group_lanes(uint32_t(n), radius / s.spacing) && terrains.empty();
+    sp.ordered = !shared_rows;
     if (sp.ordered) SLF_TRY(worder.ensure(n, 0, stream));
     worder_valid = sp.ordered;
     fgrid = GridDev{};
