@@ -142,10 +142,6 @@ struct Two {
 struct Three {
     float4 a, b, c;
 };
-struct FiveF {
-    float4 a, b, c;
-    float d, e;
-};
 
 // Adds three per-thread values into parameter-gradient slots: a block sum first, then one FP64
 // atomic per slot and block (every thread of the block calls it).
@@ -409,12 +405,47 @@ __global__ void k_adj_advance(Params p, const StepConsts* __restrict__ sc, const
 }
 
 // ---- forces (step.rs:173-211), wall viscosity (step.rs:262-301), Tait pressure (step.rs:147-172)
+// One fluid pair's share of the force adjoint, L = (a_i-bar - a_j-bar) . T(r, u, S, R), gathered by i.
+// q: the neighbour's position (p / rho^2 in w), its velocity (its density in w) and its a-bar.  A pair
+// that moves apart is not damped: half of all pairs, whose five divisions were of zero (the slow path).
+template <bool PRESSURE>
+__device__ __forceinline__ void force_pair(const Params& p, float nu, bool exact, float3 r, const Three& q, float3 vi,
+                                           float3 ai, float rho_i, float s_i, float3& xbar, float3& vbar, float& sbar,
+                                           float& rbar, double& nu_bar) {
+    const float m = p.mass, d2 = dotf(r, r), inv = inv_length(d2);
+    if (inv == 0.0f) return;
+    float g, gp;
+    grad_factor(p, d2 * inv, g, gp);
+    const float3 u = vi - f3(q.b), w = ai - f3(q.c);
+    const float S = PRESSURE ? s_i + q.a.w : 0.0f;
+    // EXACT lists: the forward's own dot product decides whether the pair approaches
+    const float ur = exact ? dot3(u.x, u.y, u.z, r.x, r.y, r.z) : dotf(u, r);
+    const float G = dotf(w, r), P = -m * g * G;  // P: dL/dPi and dL/dS
+    if (PRESSURE) sbar += P;
+    if (ur < 0.0f) {
+        const float ie = 1.0f / (d2 + p.soften), iR = 1.0f / (rho_i + q.b.w), k = 2.0f * ie * iR;
+        const float dPi_dt = -nu * k, Pi = dPi_dt * ur;
+        const float c1 = -m * (S + Pi);
+        xbar = xbar + w * (c1 * g) + r * (c1 * G * gp * inv - P * Pi * ie * 2.0f) + u * (P * dPi_dt);
+        vbar = vbar + r * (P * dPi_dt);
+        rbar -= P * Pi * iR;
+        // viscosity enters a_i's own term: a_i-bar . dT/dnu
+        nu_bar += (double)(m * g * ur * dotf(ai, r) * k);
+    } else if (PRESSURE) {
+        const float c1 = -m * S;
+        xbar = xbar + w * (c1 * g) + r * (c1 * G * gp * inv);
+    }
+}
+
 // PRESSURE = false: the DFSPH viscosity pass (dfsph.rs:90-99), the same pairs without pressure,
 // so the pressure records are neither gathered nor differentiated
 // TERRAIN: the ground's terms and the body points' as well (WCSPH worlds with terrain regions or
 // coupled bodies)
+// Three blocks a SM (80 registers; 111 uncapped, two blocks, the same time at 512k; four spill): the
+// gathers of three records a neighbour, where five were, and the divisions of zero bound it before:
+// the DFSPH viscosity's adjoint 388 -> 221 us at 512k particles, the WCSPH adjoint 362 -> 252 at 373k.
 template <bool PRESSURE, bool TERRAIN = false>
-__global__ void __launch_bounds__(kBlock) k_adj_force(Params p, const StepConsts* __restrict__ sc, PairLists fl,
+__global__ void __launch_bounds__(kBlock, 3) k_adj_force(Params p, const StepConsts* __restrict__ sc, PairLists fl,
                                                       PairLists wl, int form, const float4* __restrict__ pos,
                                                       const float4* __restrict__ vel, const float* __restrict__ rho,
                                                       const float* __restrict__ press,
@@ -434,42 +465,11 @@ __global__ void __launch_bounds__(kBlock) k_adj_force(Params p, const StepConsts
         float3 xbar = make_float3(0, 0, 0), vbar = make_float3(0, 0, 0);
         float sbar = 0.0f, pbar = 0.0f, rbar = 0.0f;
 
-        // fluid pairs: L = (a_i-bar - a_j-bar) . T(r, u, S, R)
-        walk4<FiveF>(fl, form, row,
-                     [&](uint32_t j) {
-                         return FiveF{__ldg(&pos[j]), __ldg(&vel[j]), __ldg(&ab[j]), __ldg(&rho[j]),
-                                      PRESSURE ? __ldg(&scaled[j]) : 0.0f};
-                     },
-                     [&](uint32_t, const FiveF& q, uint32_t e) {
-            float3 r = pair_off(p, form, xi, q.a, e);
-            float d2 = dotf(r, r), inv = inv_length(d2);
-            if (inv == 0.0f) return;
-            float g, gp;
-            grad_factor(p, d2 * inv, g, gp);
-            float3 u = vi - f3(q.b);
-            float3 w = ai - f3(q.c);
-            float R = rho_i + q.d;
-            float S = PRESSURE ? s_i + q.e : 0.0f;
-            // EXACT lists: the forward's own dot product decides whether the pair approaches
-            float ur = form == kFormExact ? dot3(u.x, u.y, u.z, r.x, r.y, r.z) : dotf(u, r);
-            bool act = ur < 0.0f;
-            float t = act ? ur : 0.0f;
-            float den = (d2 + p.soften) * R;
-            float Pi = -nu * t * 2.0f / den;
-            float G = dotf(w, r);
-            float P = -m * g * G;  // dL/dPi and dL/dS
-            float dPi_dt = -2.0f * nu / den;
-            float dPi_dd2 = -Pi / (d2 + p.soften);
-            float c1 = -m * (S + Pi);
-            float3 dr = w * (c1 * g) + r * (c1 * G * gp * inv + P * dPi_dd2 * 2.0f);
-            if (act) dr = dr + u * (P * dPi_dt);
-            xbar = xbar + dr;
-            if (act) vbar = vbar + r * (P * dPi_dt);
-            rbar += P * (-Pi / R);
-            if (PRESSURE) sbar += P;
-            // viscosity enters a_i's own term: a_i-bar . dT/dnu
-            nu_bar += (double)(2.0f * m * g * t * dotf(ai, r) / den);
-        });
+        walk4<Three>(fl, form, row, [&](uint32_t j) { return Three{__ldg(&pos[j]), __ldg(&vel[j]), __ldg(&ab[j])}; },
+                     [&](uint32_t, const Three& q, uint32_t e) {
+                         force_pair<PRESSURE>(p, nu, form == kFormExact, pair_off(p, form, xi, q.a, e), q, vi, ai, rho_i,
+                                              s_i, xbar, vbar, sbar, rbar, nu_bar);
+                     });
 
         // walls: pressure mirrored onto the wall (step.rs:197-202)
         uint32_t nw = listed_count(wl, row);
@@ -595,21 +595,25 @@ __global__ void __launch_bounds__(kBlock) k_adj_force(Params p, const StepConsts
     add_grads3(grads, kGradViscosity, kGradWallViscosity, kGradStiffness, nu_bar, nuw_bar, b_bar);
 }
 
-// ---- the same two adjoints a warp a row, for scenes too small to fill the GPU a thread a row ----
-// Each lane takes every 32nd entry of the row's lists; partial sums meet in butterfly sums, which
-// leave every lane with the same bits (each level adds x + y on one lane and y + x on its partner),
+// ---- the same two adjoints L lanes a row, for scenes too small to fill the GPU a thread a row ----
+// A warp takes 32 / L rows (lane = row + (32 / L) * sub, so that a step's list entries lie side by
+// side), each lane every L-th entry; partial sums meet in butterfly sums over the row's lanes, which
+// leave each of them with the same bits (each level adds x + y on one lane and y + x on its partner),
 // so the lanes agree on the wall normal they all form.  Run to run the sums are deterministic.
-__device__ __forceinline__ float warp_sum(float v) {
+template <int L>
+__device__ __forceinline__ float row_sum(float v) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = 16; o >= 32 / L; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ float3 warp_sum3(float3 v) { return make_float3(warp_sum(v.x), warp_sum(v.y), warp_sum(v.z)); }
+template <int L>
+__device__ __forceinline__ float3 row_sum3(float3 v) {
+    return make_float3(row_sum<L>(v.x), row_sum<L>(v.y), row_sum<L>(v.z));
+}
 
-constexpr uint32_t kAdjWarpMax = 262144u;  // rows a warp each up to this many particles
-
-// k_adj_force (WCSPH forces, wall viscosity, Tait pressure) a warp a row; no terrain.
-__global__ void __launch_bounds__(kBlock) k_adj_force_warp(Params p, const StepConsts* __restrict__ sc, PairLists fl,
+// k_adj_force (WCSPH forces, wall viscosity, Tait pressure) L lanes a row; no terrain.
+template <int L>
+__global__ void __launch_bounds__(kBlock) k_adj_force_group(Params p, const StepConsts* __restrict__ sc, PairLists fl,
                                                            PairLists wl, int form, const float4* __restrict__ pos,
                                                            const float4* __restrict__ vel, const float* __restrict__ rho,
                                                            const float* __restrict__ press,
@@ -618,56 +622,42 @@ __global__ void __launch_bounds__(kBlock) k_adj_force_warp(Params p, const StepC
                                                            const float4* __restrict__ ab, float4* __restrict__ xb,
                                                            float4* __restrict__ vb, float* __restrict__ rb,
                                                            double* __restrict__ grads) {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    constexpr uint32_t R = 32u / L;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane / R;
+    const uint32_t first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * R, row = first + lane % R;
     double nu_bar = 0.0, nuw_bar = 0.0, b_bar = 0.0;
-    if (row < p.n) {
-        const uint32_t i = fl.particle(row);
+    if (first < p.n) {  // whole warps; a row past the end lists nothing and writes nothing
+        const bool valid = row < p.n;
+        const uint32_t i = valid ? fl.particle(row) : 0u;
         const float nu = sc->viscosity, nuw = sc->wall_viscosity, m = p.mass;
         const float3 xi = f3(pos[i]), vi = f3(vel[i]), ai = f3(ab[i]);
         const float rho_i = rho[i], p_i = press[i], s_i = scaled[i];
         float3 xbar = make_float3(0, 0, 0), vbar = make_float3(0, 0, 0);
         float sbar = 0.0f, pbar = 0.0f, rbar = 0.0f;
 
-        // fluid pairs: L = (a_i-bar - a_j-bar) . T(r, u, S, R)
-        const uint32_t nf = listed_count(fl, row);
-        for (uint32_t k = lane; k < nf; k += 32u) {
-            const uint32_t e = listed_raw(fl, form, row, k), j = entry_index(e, form);
-            const float4 qa = __ldg(&pos[j]), qv = __ldg(&vel[j]), qb = __ldg(&ab[j]);
-            const float qr = __ldg(&rho[j]), qs = __ldg(&scaled[j]);
-            float3 r = pair_off(p, form, xi, qa, e);
-            float d2 = dotf(r, r), inv = inv_length(d2);
-            if (inv == 0.0f) continue;
-            float g, gp;
-            grad_factor(p, d2 * inv, g, gp);
-            float3 u = vi - f3(qv);
-            float3 w = ai - f3(qb);
-            float R = rho_i + qr;
-            float S = s_i + qs;
-            // EXACT lists: the forward's own dot product decides whether the pair approaches
-            float ur = form == kFormExact ? dot3(u.x, u.y, u.z, r.x, r.y, r.z) : dotf(u, r);
-            bool act = ur < 0.0f;
-            float t = act ? ur : 0.0f;
-            float den = (d2 + p.soften) * R;
-            float Pi = -nu * t * 2.0f / den;
-            float G = dotf(w, r);
-            float P = -m * g * G;
-            float dPi_dt = -2.0f * nu / den;
-            float dPi_dd2 = -Pi / (d2 + p.soften);
-            float c1 = -m * (S + Pi);
-            float3 dr = w * (c1 * g) + r * (c1 * G * gp * inv + P * dPi_dd2 * 2.0f);
-            if (act) dr = dr + u * (P * dPi_dt);
-            xbar = xbar + dr;
-            if (act) vbar = vbar + r * (P * dPi_dt);
-            rbar += P * (-Pi / R);
-            sbar += P;
-            nu_bar += (double)(2.0f * m * g * t * dotf(ai, r) / den);
+        const uint32_t nf = valid ? listed_count(fl, row) : 0u;
+        for (uint32_t k = sub; k < nf; k += 2u * L) {  // two neighbours' gathers in flight
+            uint32_t e[2];
+            Three q[2];
+#pragma unroll
+            for (int o = 0; o < 2; ++o) e[o] = listed_raw(fl, form, row, k + o * L < nf ? k + o * L : k);
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const uint32_t j = entry_index(e[o], form);
+                q[o] = Three{__ldg(&pos[j]), __ldg(&vel[j]), __ldg(&ab[j])};
+            }
+#pragma unroll
+            for (int o = 0; o < 2; ++o)
+                if (k + o * L < nf)
+                    force_pair<true>(p, nu, form == kFormExact, pair_off(p, form, xi, q[o].a, e[o]), q[o], vi, ai, rho_i,
+                                     s_i, xbar, vbar, sbar, rbar, nu_bar);
         }
 
         // walls: pressure mirrored onto the wall, and the wall normal's sum
-        const uint32_t nw = listed_count(wl, row);
+        const uint32_t nw = valid ? listed_count(wl, row) : 0u;
         const float M = s_i + p_i * p.inv_rest_sq;
         float3 A = make_float3(0, 0, 0);
-        for (uint32_t k = lane; k < nw; k += 32u) {
+        for (uint32_t k = sub; k < nw; k += L) {
             const uint32_t e = listed_raw(wl, form, row, k), j = entry_index(e, form);
             float3 r = pair_off(p, form, xi, __ldg(&walls[j]), e);
             float d2 = dotf(r, r), inv = inv_length(d2);
@@ -681,17 +671,20 @@ __global__ void __launch_bounds__(kBlock) k_adj_force_warp(Params p, const StepC
             xbar = xbar + (ai * g + r * (ar * gp * inv)) * (-m * M);
             A = A - r * g;
         }
-        A = warp_sum3(A);
+        const bool walled = __any_sync(0xffffffffu, nw > 0);
+        if (walled) A = row_sum3<L>(A);
 
-        // wall viscosity (every lane holds the same A, so the same normal and branch)
-        float alen = sqrtf(dotf(A, A));
-        if (nw > 0 && alen > 0.0f && isfinite(alen)) {
-            float3 nrm = A * (1.0f / alen);
+        // wall viscosity (every lane of a row holds the same A, so the same normal and branch; the
+        // warp's other rows only take part in the sums)
+        const float alen = sqrtf(dotf(A, A));
+        const bool on = nw > 0 && alen > 0.0f && isfinite(alen);
+        if (walled) {
+            float3 nrm = A * (on ? 1.0f / alen : 0.0f);
             float vn = dotf(vi, nrm);
             float kk = fminf(vn, 0.0f);
             float3 I = nrm * kk;
             float3 Ibar = make_float3(0, 0, 0);
-            for (uint32_t k = lane; k < nw; k += 32u) {
+            for (uint32_t k = sub; on && k < nw; k += L) {
                 const uint32_t e = listed_raw(wl, form, row, k), j = entry_index(e, form);
                 float3 r = pair_off(p, form, xi, __ldg(&walls[j]), e);
                 float tau = dotf(I, r);
@@ -711,15 +704,15 @@ __global__ void __launch_bounds__(kBlock) k_adj_force_warp(Params p, const StepC
                 xbar = xbar + dh * D + r * (h * (-D / e2) * 2.0f) + I * tb;
                 Ibar = Ibar + r * tb;
             }
-            Ibar = warp_sum3(Ibar);
+            Ibar = row_sum3<L>(Ibar);
             float3 nbar = Ibar * kk;
-            if (vn < 0.0f) {
+            if (on && vn < 0.0f) {
                 float kbar = dotf(Ibar, nrm);
-                if (lane == 0) vbar = vbar + nrm * kbar;
+                if (sub == 0) vbar = vbar + nrm * kbar;
                 nbar = nbar + vi * kbar;
             }
-            float3 Abar = (nbar - nrm * dotf(nrm, nbar)) * (1.0f / alen);
-            for (uint32_t k = lane; k < nw; k += 32u) {
+            float3 Abar = (nbar - nrm * dotf(nrm, nbar)) * (on ? 1.0f / alen : 0.0f);
+            for (uint32_t k = sub; on && k < nw; k += L) {
                 const uint32_t e = listed_raw(wl, form, row, k), j = entry_index(e, form);
                 float3 r = pair_off(p, form, xi, __ldg(&walls[j]), e);
                 float d = sqrtf(dotf(r, r));
@@ -730,12 +723,12 @@ __global__ void __launch_bounds__(kBlock) k_adj_force_warp(Params p, const StepC
             }
         }
 
-        xbar = warp_sum3(xbar);
-        vbar = warp_sum3(vbar);
-        sbar = warp_sum(sbar);
-        pbar = warp_sum(pbar);
-        rbar = warp_sum(rbar);
-        if (lane == 0) {
+        xbar = row_sum3<L>(xbar);
+        vbar = row_sum3<L>(vbar);
+        sbar = row_sum<L>(sbar);
+        pbar = row_sum<L>(pbar);
+        rbar = row_sum<L>(rbar);
+        if (valid && sub == 0) {
             // s = p / rho^2 and the Tait equation of state
             float ptot = pbar + sbar / (rho_i * rho_i);
             rbar += sbar * (-2.0f * p_i / (rho_i * rho_i * rho_i));
@@ -755,40 +748,51 @@ __global__ void __launch_bounds__(kBlock) k_adj_force_warp(Params p, const StepC
     add_grads3(grads, kGradViscosity, kGradWallViscosity, kGradStiffness, nu_bar, nuw_bar, b_bar);
 }
 
-// k_adj_density a warp a row.
-__global__ void __launch_bounds__(kBlock) k_adj_density_warp(Params p, PairLists fl, PairLists wl, int form,
+// k_adj_density L lanes a row.
+template <int L>
+__global__ void __launch_bounds__(kBlock) k_adj_density_group(Params p, PairLists fl, PairLists wl, int form,
                                                              const float4* __restrict__ pos,
                                                              const float4* __restrict__ walls,
                                                              const float* __restrict__ rb, float4* __restrict__ xb) {
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (row >= p.n) return;
-    const uint32_t i = fl.particle(row);
+    constexpr uint32_t R = 32u / L;
+    const uint32_t lane = threadIdx.x & 31u, sub = lane / R;
+    const uint32_t first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * R, row = first + lane % R;
+    if (first >= p.n) return;  // whole warps
+    const bool valid = row < p.n;
+    const uint32_t i = valid ? fl.particle(row) : 0u;
     const float3 xi = f3(pos[i]);
     const float rbi = rb[i];
     float3 xbar = make_float3(0, 0, 0);
-    const uint32_t nf = listed_count(fl, row);
-    for (uint32_t k = lane; k < nf; k += 32u) {
-        const uint32_t e = listed_raw(fl, form, row, k), j = entry_index(e, form);
-        const float4 q = __ldg(&pos[j]);
-        float3 r = pair_off(p, form, xi, q, e);
-        float d = sqrtf(dotf(r, r));
-        if (d <= 0.0f) continue;
+    auto pair = [&](float3 r, float share) {
+        const float d2 = dotf(r, r), inv = inv_length(d2);
+        if (inv == 0.0f) return;
         float g, gp;
-        grad_factor(p, d, g, gp);
-        xbar = xbar + r * (g * p.mass * (rbi + __ldg(&rb[j])));
+        grad_factor(p, d2 * inv, g, gp);
+        xbar = xbar + r * (g * p.mass * share);
+    };
+    const uint32_t nf = valid ? listed_count(fl, row) : 0u;
+    for (uint32_t k = sub; k < nf; k += 2u * L) {
+        uint32_t e[2];
+        float4 q[2];
+#pragma unroll
+        for (int o = 0; o < 2; ++o) e[o] = listed_raw(fl, form, row, k + o * L < nf ? k + o * L : k);
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+            const uint32_t j = entry_index(e[o], form);
+            q[o] = __ldg(&pos[j]);
+            q[o].w = __ldg(&rb[j]);
+        }
+#pragma unroll
+        for (int o = 0; o < 2; ++o)
+            if (k + o * L < nf) pair(pair_off(p, form, xi, q[o], e[o]), rbi + q[o].w);
     }
-    const uint32_t nw = listed_count(wl, row);
-    for (uint32_t k = lane; k < nw; k += 32u) {
-        const uint32_t e = listed_raw(wl, form, row, k), j = entry_index(e, form);
-        float3 r = pair_off(p, form, xi, __ldg(&walls[j]), e);
-        float d = sqrtf(dotf(r, r));
-        if (d <= 0.0f) continue;
-        float g, gp;
-        grad_factor(p, d, g, gp);
-        xbar = xbar + r * (g * p.mass * rbi);
+    const uint32_t nw = valid ? listed_count(wl, row) : 0u;
+    for (uint32_t k = sub; k < nw; k += L) {
+        const uint32_t e = listed_raw(wl, form, row, k);
+        pair(pair_off(p, form, xi, __ldg(&walls[entry_index(e, form)]), e), rbi);
     }
-    xbar = warp_sum3(xbar);
-    if (lane == 0) {
+    xbar = row_sum3<L>(xbar);
+    if (valid && sub == 0) {
         float4 x0 = xb[i];
         xb[i] = make_float4(x0.x + xbar.x, x0.y + xbar.y, x0.z + xbar.z, 0.0f);
     }
@@ -816,10 +820,10 @@ __global__ void __launch_bounds__(kBlock) k_adj_density(Params p, PairLists fl, 
                   },
                   [&](uint32_t, float4 q, uint32_t e) {
                       float3 r = pair_off(p, form, xi, q, e);
-                      float d = sqrtf(dotf(r, r));
-                      if (d <= 0.0f) return;
+                      float d2 = dotf(r, r), inv = inv_length(d2);
+                      if (inv == 0.0f) return;
                       float g, gp;
-                      grad_factor(p, d, g, gp);
+                      grad_factor(p, d2 * inv, g, gp);
                       xbar = xbar + r * (g * p.mass * (rbi + q.w));
                   });
     uint32_t nw = listed_count(wl, row);
@@ -1134,30 +1138,34 @@ __global__ void __launch_bounds__(kBlock) k_adj_alpha_prep(Params p, PairLists f
     float3 G = make_float3(0, 0, 0);
     walk4<float4>(fl, form, row, [&](uint32_t j) { return __ldg(&pos[j]); }, [&](uint32_t, float4 q, uint32_t e) {
         float3 r = pair_off(p, form, xi, q, e);
-        float d = sqrtf(dotf(r, r));
-        if (d <= 0.0f) return;
+        float d2 = dotf(r, r), inv = inv_length(d2);
+        if (inv == 0.0f) return;
         float g, gp;
-        grad_factor(p, d, g, gp);
+        grad_factor(p, d2 * inv, g, gp);
         G = G + r * (g * p.mass);
     });
     uint32_t nw = listed_count(wl, row);
     for (uint32_t k = 0; k < nw; ++k) {
         uint32_t e = listed_raw(wl, form, row, k), j = entry_index(e, form);
         float3 r = pair_off(p, form, xi, __ldg(&walls[j]), e);
-        float d = sqrtf(dotf(r, r));
-        if (d <= 0.0f) continue;
+        float d2 = dotf(r, r), inv = inv_length(d2);
+        if (inv == 0.0f) continue;
         float g, gp;
-        grad_factor(p, d, g, gp);
+        grad_factor(p, d2 * inv, g, gp);
         G = G + r * (g * p.mass);
     }
     float a = alpha[i];
     gt[i] = make_float4(G.x, G.y, G.z, -abar[i] * a * a);
 }
 
-__global__ void __launch_bounds__(kBlock) k_adj_alpha(Params p, PairLists fl, PairLists wl, int form,
-                                                      const float4* __restrict__ pos,
-                                                      const float4* __restrict__ walls,
-                                                      const float4* __restrict__ gt, float4* __restrict__ xb) {
+// Then both passes over the pairs that are left, in one walk: the factors' share, through grad W and
+// its transpose, and the densities' (k_adj_density's).  Two walks of the lists measured 68 us more at
+// 512k particles.
+__global__ void __launch_bounds__(kBlock, 4) k_adj_alpha_density(Params p, PairLists fl, PairLists wl, int form,
+                                                              const float4* __restrict__ pos,
+                                                              const float4* __restrict__ walls,
+                                                              const float4* __restrict__ gt,
+                                                              const float* __restrict__ rb, float4* __restrict__ xb) {
     uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t i = row < p.n ? fl.particle(row) : row;  // row of the walk order, its particle
     if (i >= p.n) return;
@@ -1165,30 +1173,35 @@ __global__ void __launch_bounds__(kBlock) k_adj_alpha(Params p, PairLists fl, Pa
     float3 xi = f3(pos[i]);
     float4 own = gt[i];
     float3 Gi = f3(own);
-    float tbi = own.w;
+    const float tbi = own.w, rbi = rb[i];
     float3 xacc = make_float3(0, 0, 0);
-    walk4<Two>(fl, form, row, [&](uint32_t j) { return Two{__ldg(&pos[j]), __ldg(&gt[j])}; },
+    walk4<Two>(fl, form, row,
+               [&](uint32_t j) {
+                   Two q{__ldg(&pos[j]), __ldg(&gt[j])};
+                   q.a.w = __ldg(&rb[j]);
+                   return q;
+               },
                [&](uint32_t, const Two& q, uint32_t e) {
                    float3 r = pair_off(p, form, xi, q.a, e);
-                   float d = sqrtf(dotf(r, r));
-                   if (d <= 0.0f) return;
+                   float d2 = dotf(r, r), inv = inv_length(d2);
+                   if (inv == 0.0f) return;
                    float g, gp;
-                   grad_factor(p, d, g, gp);
+                   grad_factor(p, d2 * inv, g, gp);
                    float3 gw = r * (g * m);
                    float4 oj = q.b;
                    float3 c = (Gi + gw) * (2.0f * m * tbi) - (f3(oj) - gw) * (2.0f * m * oj.w);
-                   xacc = xacc + c * g + r * (dotf(c, r) * gp / d);
+                   xacc = xacc + c * g + r * (dotf(c, r) * gp * inv + g * m * (rbi + q.a.w));
                });
     uint32_t nw = listed_count(wl, row);
     for (uint32_t k = 0; k < nw; ++k) {
         uint32_t e = listed_raw(wl, form, row, k), j = entry_index(e, form);
         float3 r = pair_off(p, form, xi, __ldg(&walls[j]), e);
-        float d = sqrtf(dotf(r, r));
-        if (d <= 0.0f) continue;
+        float d2 = dotf(r, r), inv = inv_length(d2);
+        if (inv == 0.0f) continue;
         float g, gp;
-        grad_factor(p, d, g, gp);
+        grad_factor(p, d2 * inv, g, gp);
         float3 c = Gi * (2.0f * m * tbi);
-        xacc = xacc + c * g + r * (dotf(c, r) * gp / d);
+        xacc = xacc + c * g + r * (dotf(c, r) * gp * inv + g * m * rbi);
     }
     float4 x0 = xb[i];
     xb[i] = make_float4(x0.x + xacc.x, x0.y + xacc.y, x0.z + xacc.z, 0.0f);
@@ -1234,11 +1247,12 @@ void launch_adjoint_wcsph(const Params& p, const StepConsts* sc, const PairLists
                                                                    walls, ab, xb, vb, rb, grads, 0, T, slope, bodies);
         k_adj_density<<<adj_blocks(p.n), kBlock, 0, s>>>(p, fl, wl, form, pos, walls, rb, xb, T.regions ? slope : nullptr,
                                                          bodies);
-    } else if (p.n <= kAdjWarpMax) {
-        // few rows: a warp each, so that the GPU fills
-        k_adj_force_warp<<<adj_blocks(p.n * 32u), kBlock, 0, s>>>(p, sc, fl, wl, form, pos, vel, rho, press, scaled,
-                                                                  walls, ab, xb, vb, rb, grads);
-        k_adj_density_warp<<<adj_blocks(p.n * 32u), kBlock, 0, s>>>(p, fl, wl, form, pos, walls, rb, xb);
+    } else if (with_lanes(adjoint_lanes(p.n, p.radius / p.spacing), [&](auto lanes) {
+                   constexpr int L = decltype(lanes)::value;
+                   k_adj_force_group<L><<<adj_blocks(p.n * L), kBlock, 0, s>>>(p, sc, fl, wl, form, pos, vel, rho, press,
+                                                                               scaled, walls, ab, xb, vb, rb, grads);
+                   k_adj_density_group<L><<<adj_blocks(p.n * L), kBlock, 0, s>>>(p, fl, wl, form, pos, walls, rb, xb);
+               })) {
     } else {
         k_adj_force<true><<<adj_blocks(p.n), kBlock, 0, s>>>(p, sc, fl, wl, form, pos, vel, rho, press, scaled,
                                                              walls, ab, xb, vb, rb, grads, 0, T, slope, MoverDev{});
@@ -1307,8 +1321,7 @@ void launch_adj_factors_density(const Params& p, const PairLists& fl, const Pair
                                 float4* gt, const float* rb, float4* xb, cudaStream_t s) {
     if (!p.n) return;
     k_adj_alpha_prep<<<adj_blocks(p.n), kBlock, 0, s>>>(p, fl, wl, form, pos, walls, alpha, abar, gt);
-    k_adj_alpha<<<adj_blocks(p.n), kBlock, 0, s>>>(p, fl, wl, form, pos, walls, gt, xb);
-    k_adj_density<<<adj_blocks(p.n), kBlock, 0, s>>>(p, fl, wl, form, pos, walls, rb, xb, nullptr, MoverDev{});
+    k_adj_alpha_density<<<adj_blocks(p.n), kBlock, 0, s>>>(p, fl, wl, form, pos, walls, gt, rb, xb);
 }
 
 void launch_adj_unsort(uint32_t n, const uint32_t* dest, const float4* xb, const float4* vb, float4* xp, float4* vp,

@@ -117,6 +117,14 @@ struct PairLists {
 #endif
 };
 
+// Where the density pass leaves what the later passes gather of a neighbour beside its position and
+// velocity, so that one 16-byte gather brings both: p / rho^2 in the position's spare lane (WCSPH;
+// DFSPH's checks put the stiffness there), the density in the velocity's.
+struct PairRecords {
+    float* pos_w;
+    float* vel_w;
+};
+
 // Terrain regions (src/fluid/terrain.rs): signed distances at nodes `step` apart from `low`, index
 // (y * nz + z) * nx + x, `offset` into the shared distance array; and the ground sites, the
 // water's lattice within the kernel around a particle with the density each site adds.

@@ -582,14 +582,6 @@ __device__ __forceinline__ void pair_terms(const Params& p, const PairLists& l, 
 // (step.rs:147-172) or the DFSPH factors (dfsph.rs:108-163) --------------------------------
 
 // four blocks a SM (64 registers), as the pass compiled before it strode over rows
-// Where the density pass leaves what the later passes gather of a neighbour beside its position and
-// velocity, so that one 16-byte gather brings both: p / rho^2 in the position's spare lane (WCSPH;
-// DFSPH's checks put the stiffness there), the density in the velocity's.
-struct PairRecords {
-    float* pos_w;
-    float* vel_w;
-};
-
 // What the pass lists: the fluid (0), then the walls (1).
 struct DensityIn {
     GridDev grid[2];
@@ -2231,18 +2223,6 @@ static uint32_t group_blocks(uint32_t n, int lanes) {
     g_launches.fetch_add(1, std::memory_order_relaxed);
     const uint32_t rows = uint32_t(kGroupBlock / lanes);
     return (n + rows - 1) / rows;
-}
-
-// calls f with the number of lanes as a constant; false for none (a thread a row)
-template <class F>
-static bool with_lanes(int lanes, F&& f) {
-    switch (lanes) {
-        case 4: f(std::integral_constant<int, 4>{}); return true;
-        case 8: f(std::integral_constant<int, 8>{}); return true;
-        case 16: f(std::integral_constant<int, 16>{}); return true;
-        case 32: f(std::integral_constant<int, 32>{}); return true;
-        default: return false;
-    }
 }
 
 size_t density_scratch_words(uint32_t n, uint32_t cap, float support) {

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kBlock) k_density_fast(Params p, GridDev fg, G
                                                          const float4* __restrict__ walls, PairLists fpl,
                                                          PairLists wpl, float* __restrict__ rho,
                                                          float* __restrict__ press, float* __restrict__ scaled,
-                                                         float* __restrict__ alpha, Status* st) {
+                                                         float* __restrict__ alpha, Status* st, PairRecords rec) {
     IndexLists fl = index_lists(fpl), wl = index_lists(wpl);
     uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t i = row < p.n ? fpl.particle(row) : row;  // row of the walk order, its particle
@@ -291,11 +291,14 @@ __global__ void __launch_bounds__(kBlock) k_density_fast(Params p, GridDev fg, G
             float r2 = ratio * ratio, r4 = r2 * r2;
             float pressure = fmaxf(p.stiffness * (ratio * r2 * r4 - 1.0f), 0.0f);
             press[i] = pressure;
-            scaled[i] = pressure / (density * density);
+            const float over = pressure > 0.0f ? pressure / (density * density) : 0.0f;
+            scaled[i] = over;
+            rec.pos_w[4 * size_t(i) + 3] = over;
         } else {
             float total = fl2(sx, sy, sz) + squares;
             alpha[i] = total > 0.0f ? 1.0f / total : 0.0f;
         }
+        rec.vel_w[4 * size_t(i) + 3] = density;
         float c = density * p.inv_rest - 1.0f;
         if (c > 0.0f) compressed = __float_as_uint(c);
     }
@@ -508,9 +511,12 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_force_fast(Params p, const Ste
             float squared = fl2(r.x, r.y, r.z);
             if (squared <= 0.0f) return;
             float g = fast_factor(p, squared);
-            float toward = fminf(fmaf(v.x - w.x, r.x, fmaf(v.y - w.y, r.y, (v.z - w.z) * r.z)), 0.0f);
-            float damp = visc2 * toward / ((squared + p.soften) * (density + __ldg(&rho[e & kIndexMask])));
-            float s = g * p.mass * (own + __ldg(&scaled[e & kIndexMask]) + damp);
+            float toward = fmaf(v.x - w.x, r.x, fmaf(v.y - w.y, r.y, (v.z - w.z) * r.z));
+            // the neighbour's density and p / rho^2 ride in the spare lanes (PairRecords); a pair that
+            // parts is not damped, and divides no zero (the division's slow path)
+            float damp = 0.0f;
+            if (toward < 0.0f) damp = visc2 * toward / ((squared + p.soften) * (density + w.w));
+            float s = g * p.mass * (own + q.w + damp);
             px = fmaf(-r.x, s, px);
             py = fmaf(-r.y, s, py);
             pz = fmaf(-r.z, s, pz);
@@ -579,11 +585,11 @@ __device__ __forceinline__ void rate_particle_fast(const Params& p, const StepCo
     float target, error;
     if (WHICH == 1) {
         float over = fmaxf(fmaf(dt, rate, rho[i]) - p.rest, 0.0f);
-        target = over / sc->dt_sq;
+        target = over > 0.0f ? over / sc->dt_sq : 0.0f;  // (no division of a zero: its slow path)
         error = over * p.inv_rest;
     } else {
         float r = fl.count[row] + wl.count[row] < 20u ? 0.0f : fmaxf(rate, 0.0f);
-        target = r / dt;
+        target = r > 0.0f ? r / dt : 0.0f;
         error = dt * r * p.inv_rest;
     }
     // the stiffness goes into the position's spare lane
@@ -690,7 +696,7 @@ __global__ void __launch_bounds__(kBlock) k_viscous_fast(Params p, const StepCon
         float toward = fmaf(v.x - w.x, r.x, fmaf(v.y - w.y, r.y, (v.z - w.z) * r.z));
         if (toward < 0.0f) {
             float l2 = fl2(r.x, r.y, r.z);
-            float s = visc2 * toward / ((l2 + p.soften) * (density + __ldg(&rho[j]))) * fast_factor(p, l2);
+            float s = visc2 * toward / ((l2 + p.soften) * (density + w.w)) * fast_factor(p, l2);
             px = fmaf(-r.x, s, px);
             py = fmaf(-r.y, s, py);
             pz = fmaf(-r.z, s, pz);
@@ -830,25 +836,26 @@ void prepare_fast_grids() {
     for (int k = 0; k < 4; ++k) g_fast_resident[k].store(uint32_t(std::max(per[k], 0) * std::max(sms, 0)));
 }
 
-void launch_density_fast(const Params& p, const GridDev& fg, const GridDev& wg, const float4* pos, const int4* cells,
+void launch_density_fast(const Params& p, const GridDev& fg, const GridDev& wg, float4* pos, const int4* cells,
                          const float4* walls, const PairLists& fl, const PairLists& wl, float* rho, float* press,
-                         float* scaled, float* alpha, Status* st, cudaStream_t s) {
+                         float* scaled, float* alpha, Status* st, cudaStream_t s, float4* vel) {
     if (!p.n) return;
+    const PairRecords rec{reinterpret_cast<float*>(pos), reinterpret_cast<float*>(vel)};
     uint32_t nb = fast_blocks(p.n);
     if (cells) {
         if (p.solver == 0)
             k_density_fast<0, true><<<nb, kBlock, 0, s>>>(p, fg, wg, pos, cells, walls, fl, wl, rho, press, scaled,
-                                                           alpha, st);
+                                                           alpha, st, rec);
         else
             k_density_fast<1, true><<<nb, kBlock, 0, s>>>(p, fg, wg, pos, cells, walls, fl, wl, rho, press, scaled,
-                                                           alpha, st);
+                                                           alpha, st, rec);
     } else {
         if (p.solver == 0)
             k_density_fast<0, false><<<nb, kBlock, 0, s>>>(p, fg, wg, pos, cells, walls, fl, wl, rho, press, scaled,
-                                                            alpha, st);
+                                                            alpha, st, rec);
         else
             k_density_fast<1, false><<<nb, kBlock, 0, s>>>(p, fg, wg, pos, cells, walls, fl, wl, rho, press, scaled,
-                                                            alpha, st);
+                                                            alpha, st, rec);
     }
 }
 

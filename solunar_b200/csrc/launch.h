@@ -61,6 +61,21 @@ inline int group_lanes(uint32_t n, float support) {
     return n <= 20480u ? 8 : n <= 32768u ? 4 : 0;
 }
 
+// Lanes a row of the WCSPH adjoint (k_adj_force_group, k_adj_density_group) in scenes without terrain
+// or bodies; 0: a thread a row, whose wall normals are summed as the forward sums them.  Measured, us
+// (before: a warp a row, every entry of a row in another sector):
+//            n   support 2: before thread  L=4  L=8 L=16     support 4: before thread  L=4  L=8 L=16
+//         1000                  27     79   38   31   28                  40    555  130   76   50
+//        17576                  57     80   41   41   43                 135    580  158  113  100
+//        46656                 111     88   55   59   71                 331    685  261  217  216
+//       110592                 227    106   90  103  136                 729    792  452  415  451
+//       262144                 523    200  174  212  292
+inline int adjoint_lanes(uint32_t n, float support) {
+    if (n > 262144u) return 0;
+    if (support >= 3.0f) return n <= 4096u ? 32 : n <= 20480u ? 16 : 8;
+    return n <= 8192u ? 16 : n <= 24576u ? 8 : 4;
+}
+
 // pair passes: the density pass builds the substep's neighbour lists, the others walk them
 // T: terrain regions (regions = 0: none); slope (optional): each particle's ground density gradient
 // vel: the velocities at pos, whose spare lanes take the densities (and pos's WCSPH's p / rho^2)
@@ -166,9 +181,9 @@ void launch_unpack3(uint32_t n, const float* in, float4* out, cudaStream_t s, ui
 // lists hold indexes only (with the cell step in their top bits) and each pass recomputes the
 // kernel gradient from the positions.  `cells` non-null (or `rel`) selects cell-relative
 // positions: pos holds offsets in [0, r) from the cell corner, cells the integer cells.
-void launch_density_fast(const Params& p, const GridDev& fg, const GridDev& wg, const float4* pos, const int4* cells,
+void launch_density_fast(const Params& p, const GridDev& fg, const GridDev& wg, float4* pos, const int4* cells,
                          const float4* walls, const PairLists& fl, const PairLists& wl, float* rho, float* press,
-                         float* scaled, float* alpha, Status* st, cudaStream_t s);
+                         float* scaled, float* alpha, Status* st, cudaStream_t s, float4* vel);
 void launch_wcsph_force_fast(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,
                              const float4* pos, const int4* cells, const float4* vel, const float* rho,
                              const float* press, const float* scaled, const float4* walls, float4* pos_out,

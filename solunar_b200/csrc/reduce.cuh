@@ -4,10 +4,23 @@
 
 #include <climits>
 #include <cstdint>
+#include <type_traits>
 
 #include "fluid_device.cuh"
 
 namespace slf {
+
+// calls f with the number of lanes as a constant; false for none (a thread a row)
+template <class F>
+bool with_lanes(int lanes, F&& f) {
+    switch (lanes) {
+        case 4: f(std::integral_constant<int, 4>{}); return true;
+        case 8: f(std::integral_constant<int, 8>{}); return true;
+        case 16: f(std::integral_constant<int, 16>{}); return true;
+        case 32: f(std::integral_constant<int, 32>{}); return true;
+        default: return false;
+    }
+}
 
 // ---- block reductions ---------------------------------------------------------------------
 

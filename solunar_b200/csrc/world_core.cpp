@@ -349,7 +349,7 @@ void World::density_pass(const Params& p, int a, const PairLists& fl, const Pair
     if (!on) on = stream;
     if (fast())
         launch_density_fast(p, fgrid, wgrid, pos[a].p, cells_of(a), dwalls.p, fl, wl, rh, press.p, scaled.p,
-                            alpha.p, d_status, on);
+                            alpha.p, d_status, on, vel[a].p);
     else
         launch_density(p, fgrid, wgrid, pos[a].p, dwalls.p, fl, wl, rh, press.p, scaled.p, alpha.p, d_status,
                        tdev, ground_slopes(), on, mover_dev(), dscratch.p, vel[a].p);
