@@ -20,7 +20,7 @@
 namespace slf {
 
 // How a world's lists hold a neighbour: EXACT lists {index, g} pairs; FAST lists the index in
-// the low 26 bits with the cell step to the neighbour in the top six (zero steps for absolute
+// the low 26 bits with the cell step to the neighbour in the top six (nothing there for absolute
 // positions); cell-relative positions are FAST lists whose steps matter.
 enum ListForm : int { kFormFast = 0, kFormExact = 1, kFormCellRelative = 2 };
 constexpr uint32_t kEntryIndexMask = (1u << 26) - 1u;

@@ -14,6 +14,7 @@
 #include "fluid_device.cuh"
 #include "launch.h"
 #include "reduce.cuh"
+#include "scan.cuh"
 
 namespace slf {
 
@@ -390,77 +391,6 @@ __device__ __forceinline__ float ground_near(const TerrainDev& T, float px, floa
 // instead (eight candidates and four pairs in flight, up to 128 registers): it has no other warps
 // to hide behind.  74k particles: 57 -> 48 us, at support 4 378 -> 302; 111k, three blocks a SM,
 // stay.
-
-// Lists the points of cells [b, e) within reach of `at`, in array order: each kept index goes to
-// out[nf * 32] (room for `cap`; the count goes on past it).  Four candidates' gathers are in flight
-// at a time, and a kept one costs a predicated store and an add: no branch, so the lanes of a warp
-// that keep nothing do not wait for those that do.  axy, az: the negated position; x and y of the
-// test run packed, each operation rounded as each_in_cell's.
-template <int kScanUnroll>
-__device__ __forceinline__ void scan_range(const Params& p, const float4* __restrict__ pts, uint32_t b, uint32_t e,
-                                           f32x2 axy, float az, uint32_t* out, uint32_t cap,
-                                           uint32_t& nf) {
-    const ulonglong2* __restrict__ q2 = reinterpret_cast<const ulonglong2*>(pts);
-#pragma unroll 1
-    for (uint32_t j = b; j < e; j += kScanUnroll) {
-        ulonglong2 q[kScanUnroll];
-#pragma unroll
-        for (int u = 0; u < kScanUnroll; ++u) {
-            if (j + u < e) q[u] = __ldg(q2 + j + u);
-        }
-#pragma unroll
-        for (int u = 0; u < kScanUnroll; ++u) {
-            const f32x2 oxy = add2(f32x2{q[u].x}, axy);
-            const float oz = __uint_as_float(uint32_t(q[u].y)) + az;
-            float x2, y2;
-            unpack2(mul2(oxy, oxy), x2, y2);
-            const bool keep = j + u < e && (x2 + y2) + oz * oz < p.reach;
-            if (keep && nf < cap) out[size_t(nf) * 32u] = j + u;
-            nf += keep ? 1u : 0u;
-        }
-    }
-}
-
-// The scan through tables that need bounds checks or a search, out of line: what it would hold in
-// registers stays out of the density pass.
-__device__ __noinline__ uint32_t scan_checked(const Params& p, const GridDev& g, const float4* __restrict__ pts,
-                                              int3 cell, float x, float y, float z, uint32_t* out,
-                                              uint32_t cap, uint32_t stride) {
-    uint32_t nf = 0;
-    each_near(p, g, pts, cell, x, y, z, [&](uint32_t j, float4) {
-        if (nf < cap) out[size_t(nf) * stride] = j;
-        ++nf;
-    });
-    return nf;
-}
-
-// Lists the points of `g` within reach of (x, y, z) in the reference's list order (each_near's).
-// Where the table knows which of a cell's 27 cells hold points (GridDev::near, the walls), only those
-// are visited; a cell with its 26 neighbours inside a dense table needs no bounds checks (the world
-// pads the fluid's table so that every particle's has).
-template <int kScanUnroll>
-__device__ __forceinline__ uint32_t scan_near(const Params& p, const GridDev& g, const float4* __restrict__ pts,
-                                              int3 cell, float x, float y, float z, uint32_t* out,
-                                              uint32_t cap) {
-    if (g.mode == 0) return 0u;
-    const long long bx = (long long)cell.x - g.lx, by = (long long)cell.y - g.ly, bz = (long long)cell.z - g.lz;
-    const int edge = g.near ? 0 : 1;  // cells that a walk without checks keeps away from the box's faces
-    if (g.mode != 1 || bx < edge || bx + edge >= g.sx || by < edge || by + edge >= g.sy || bz < edge ||
-        bz + edge >= g.sz)
-        return scan_checked(p, g, pts, cell, x, y, z, out, cap, 32u);
-    const f32x2 axy = pack2(-x, -y);
-    const float az = -z;
-    const uint32_t slab = uint32_t(g.sy) * uint32_t(g.sz);
-    const uint32_t c0 = (uint32_t(bx) * uint32_t(g.sy) + uint32_t(by)) * uint32_t(g.sz) + uint32_t(bz);
-    uint32_t nf = 0;
-#pragma unroll 1
-    for (uint32_t mask = g.near ? __ldg(&g.near[c0]) : (1u << 27) - 1u; mask; mask &= mask - 1u) {
-        const int t = __ffs(int(mask)) - 1;
-        const uint32_t c = c0 + uint32_t((t % 3 - 1) * int(slab) + (t / 3 % 3 - 1) * g.sz + t / 9 - 1);
-        scan_range<kScanUnroll>(p, pts, __ldg(&g.start[c]), __ldg(&g.start[c + 1]), axy, az, out, cap, nf);
-    }
-    return nf;
-}
 
 // a / radius, rounded as the IEEE division rounds it, without one: with y = RN(1 / r),
 // q = RN(a y), the remainder a - q r is exact in one fma and RN(q + remainder y) is RN(a / r)

@@ -22,6 +22,7 @@
 #include "fluid_device.cuh"
 #include "launch.h"
 #include "reduce.cuh"
+#include "scan.cuh"
 
 namespace slf {
 
@@ -219,14 +220,30 @@ __device__ __forceinline__ void each_near_rel(const Params& p, const GridDev& g,
 
 // ---- densities and lists (mod.rs:621-675; step.rs:147-172; dfsph.rs:108-163) ---------------
 
+// The checked scan in cell-relative form (scan_near's, for tables that need bounds checks).
+static __device__ __noinline__ uint32_t scan_checked_rel(const Params& p, const GridDev& g,
+                                                         const float4* __restrict__ pts, int3 cell, float x, float y,
+                                                         float z, uint32_t* out, uint32_t cap) {
+    uint32_t nf = 0;
+    each_near_rel(p, g, pts, cell, make_float4(x, y, z, 0.0f),
+                  [&](uint32_t j, float4, int dx, int dy, int dz, float, float, float) {
+                      if (nf < cap) out[size_t(nf) * 32u] = encode_entry(j, dx, dy, dz);
+                      ++nf;
+                  });
+    return nf;
+}
+
+// The candidates are scanned into the row's list first (scan_near: a kept one costs a predicated
+// store), then the sums run over the list, four gathers in flight, with every lane at work; the list
+// is the final one, read back from the L1.  Against sums inside the candidate loop: 443 -> 335 us at
+// 1M particles, 132 -> 114 at 241k cell-relative (three blocks a SM 374, five spill, 660).
 template <int SOLVER, bool REL>
-__global__ void __launch_bounds__(kBlock) k_density_fast(Params p, GridDev fg, GridDev wg,
-                                                         const float4* __restrict__ pos,
-                                                         const int4* __restrict__ cells,
-                                                         const float4* __restrict__ walls, PairLists fpl,
-                                                         PairLists wpl, float* __restrict__ rho,
-                                                         float* __restrict__ press, float* __restrict__ scaled,
-                                                         float* __restrict__ alpha, Status* st, PairRecords rec) {
+__global__ void __launch_bounds__(kBlock, 4)
+    k_density_fast(const __grid_constant__ Params p, const __grid_constant__ GridDev fg,
+                   const __grid_constant__ GridDev wg, const float4* __restrict__ pos, const int4* __restrict__ cells,
+                   const float4* __restrict__ walls, PairLists fpl, PairLists wpl, float* __restrict__ rho,
+                   float* __restrict__ press, float* __restrict__ scaled, float* __restrict__ alpha, Status* st,
+                   PairRecords rec) {
     IndexLists fl = index_lists(fpl), wl = index_lists(wpl);
     uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t i = row < p.n ? fpl.particle(row) : row;  // row of the walk order, its particle
@@ -241,50 +258,52 @@ __global__ void __launch_bounds__(kBlock) k_density_fast(Params p, GridDev fg, G
         } else {
             cell = cell_of(p, a.x, a.y, a.z);
         }
-        float sum = 0.0f, wsum = 0.0f;
-        float sx = 0.0f, sy = 0.0f, sz = 0.0f, squares = 0.0f;
-        uint32_t nf = 0, nw = 0;
-        auto fluid = [&](uint32_t j, int dx, int dy, int dz, float rx, float ry, float rz) {
-            float l2 = fl2(rx, ry, rz);
-            sum += fast_value(p, l2);
-            if (nf < fl.cap) fl.idx[fl.at(row, nf)] = encode_entry(j, dx, dy, dz);
-            ++nf;
-            if (SOLVER == 1) {
-                float g = fast_factor(p, l2) * p.mass;
-                float px = rx * g, py = ry * g, pz = rz * g;
-                sx += px;
-                sy += py;
-                sz += pz;
-                squares = fmaf(px, px, fmaf(py, py, fmaf(pz, pz, squares)));
+        float sums[2], sx = 0.0f, sy = 0.0f, sz = 0.0f, squares = 0.0f;
+#pragma unroll 1
+        for (int w = 0; w < 2; ++w) {  // the fluid, then the walls
+            const IndexLists& l = w ? wl : fl;
+            const float4* __restrict__ pts = w ? walls : pos;
+            uint32_t* const out = l.idx + l.at(row, 0);
+            uint32_t found;
+            if (REL)
+                found = scan_near<4, true>(p, w ? wg : fg, pts, cell, a.x, a.y, a.z, out, l.cap,
+                                           [](const Params& p_, const GridDev& g_, const float4* pts_, int3 c_, float x_,
+                                              float y_, float z_, uint32_t* out_, uint32_t cap_) {
+                                               return scan_checked_rel(p_, g_, pts_, c_, x_, y_, z_, out_, cap_);
+                                           });
+            else
+                found = scan_near<4>(p, w ? wg : fg, pts, cell, a.x, a.y, a.z, out, l.cap);
+            l.count[row] = found;
+            longest = max(longest, found);
+            float sum = 0.0f;
+            const uint32_t m = found < l.cap ? found : l.cap;
+#pragma unroll 1
+            for (uint32_t k = 0; k < m; k += 4) {
+                uint32_t e[4];
+                float4 q[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) e[u] = out[size_t(k + u < m ? k + u : m - 1) * 32u];  // (written above: no read-only load)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) q[u] = __ldg(&pts[e[u] & kIndexMask]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (k + u >= m) continue;
+                    const float3 r = pair_offset<REL>(p, a, q[u], e[u]);
+                    const float l2 = fl2(r.x, r.y, r.z);
+                    sum += fast_value(p, l2);
+                    if (SOLVER == 1) {
+                        const float g = fast_factor(p, l2) * p.mass, px = r.x * g, py = r.y * g, pz = r.z * g;
+                        sx += px;
+                        sy += py;
+                        sz += pz;
+                        if (w == 0) squares = fmaf(px, px, fmaf(py, py, fmaf(pz, pz, squares)));
+                    }
+                }
             }
-        };
-        auto wall = [&](uint32_t j, int dx, int dy, int dz, float rx, float ry, float rz) {
-            float l2 = fl2(rx, ry, rz);
-            wsum += fast_value(p, l2);
-            if (nw < wl.cap) wl.idx[wl.at(row, nw)] = encode_entry(j, dx, dy, dz);
-            ++nw;
-            if (SOLVER == 1) {
-                float g = fast_factor(p, l2) * p.mass;
-                sx = fmaf(rx, g, sx);
-                sy = fmaf(ry, g, sy);
-                sz = fmaf(rz, g, sz);
-            }
-        };
-        if (REL) {
-            each_near_rel(p, fg, pos, cell, a, [&](uint32_t j, float4, int dx, int dy, int dz, float rx, float ry,
-                                                   float rz) { fluid(j, dx, dy, dz, rx, ry, rz); });
-            each_near_rel(p, wg, walls, cell, a, [&](uint32_t j, float4, int dx, int dy, int dz, float rx, float ry,
-                                                     float rz) { wall(j, dx, dy, dz, rx, ry, rz); });
-        } else {
-            each_near(p, fg, pos, cell, a.x, a.y, a.z,
-                      [&](uint32_t j, float4 q) { fluid(j, 0, 0, 0, a.x - q.x, a.y - q.y, a.z - q.z); });
-            each_near(p, wg, walls, cell, a.x, a.y, a.z,
-                      [&](uint32_t j, float4 q) { wall(j, 0, 0, 0, a.x - q.x, a.y - q.y, a.z - q.z); });
+            sums[1] = sum;
+            if (w == 0) sums[0] = sum;
         }
-        fl.count[row] = nf;
-        wl.count[row] = nw;
-        longest = nf > nw ? nf : nw;
-        float density = p.mass * (sum + wsum);
+        float density = p.mass * (sums[0] + sums[1]);
         rho[i] = density;
         if (SOLVER == 0) {
             float ratio = fminf(density * p.inv_rest, 1.1f);
@@ -599,7 +618,7 @@ __device__ __forceinline__ void rate_particle_fast(const Params& p, const StepCo
 }
 
 template <int WHICH, bool REL>
-__global__ void __launch_bounds__(kBlock) k_rate_fast(Params p, const StepConsts* __restrict__ sc, PairLists fpl,
+__global__ void __launch_bounds__(kBlock, 4) k_rate_fast(Params p, const StepConsts* __restrict__ sc, PairLists fpl,
                                                       PairLists wpl, const float4* __restrict__ pos,
                                                       const float4* __restrict__ vel, const float* __restrict__ rho,
                                                       const float* __restrict__ alpha,

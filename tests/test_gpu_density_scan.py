@@ -7,7 +7,7 @@ particle runs (smaller scenes take a warp a particle).
 import numpy as np
 import pytest
 
-from solunar_b200.abi import FluidSettings, FluidSolver
+from solunar_b200.abi import Arithmetic, FluidSettings, FluidSolver, Positions
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +41,25 @@ def test_scan_and_pair_terms_are_the_restatements(gpu_lib, oracle_lib, solver, s
     assert np.array_equal(bits(g.positions()), bits(o.positions()))
     assert np.array_equal(bits(g.velocities()), bits(o.velocities()))
     assert np.array_equal(bits(g.densities()), bits(o.densities()))
+
+
+@pytest.mark.parametrize("positions", [Positions.ABSOLUTE, Positions.CELL_RELATIVE])
+@pytest.mark.parametrize("solver", [FluidSolver.WCSPH, FluidSolver.DFSPH])
+def test_fast_scan_finds_the_restatements_neighbours(gpu_lib, oracle_lib, solver, positions):
+    # a pair found or lost changes a density by far more than the rounding of the up to 64 terms both
+    # sums hold: 64 x 2^-24 each, twice that apart.  Pairs at the very radius (which cell-relative
+    # offsets may round to the other side) weigh nothing.
+    rng = np.random.default_rng(9)
+    settings = FluidSettings(solver=solver, spacing=0.02, arithmetic=Arithmetic.FAST, positions=positions)
+    pts = (rng.uniform(-0.5, 0.5, (33000, 3)) * 0.64).astype(np.float32)
+    pts[600:605] = 1.3
+    pts[600:605] += (rng.uniform(0.0, 0.3, (5, 3)) * 0.02).astype(np.float32)
+    worlds = gpu_lib.FluidWorld(settings), oracle_lib.OracleWorld(settings, residual_sum=1)
+    for w in worlds:
+        w.add_wall((0.0, 0.0, 0.0), (0.1, 0.14, 0.12))
+        w.add_particles(pts)
+        w.update_neighbors()
+        w.compute_densities()
+    g, o = worlds
+    assert np.array_equal(g.ids(), o.ids())
+    np.testing.assert_allclose(g.densities(), o.densities(), rtol=2 * 64 * 2.0 ** -24)
