@@ -1276,69 +1276,102 @@ __device__ __forceinline__ void mover_pairs(const Params& p, const MoverDev& M, 
     });
 }
 
-// What the body points took from the water this substep: one thread per (512-particle chunk,
-// body) walks the chunk's particles in order and sums, for the points of its body, the damping
-// force and its torque about the body's centre (couple.rs:401-414, step.rs:173-221).  Pairs
-// below the settling speed give nothing.  centre[b] = centre + moved; felt[c * bodies + b] =
-// (force, torque).
-// What the body points take (couple.rs:401-414) in three passes that keep the reference's order:
-// each particle counts its pairs above the settling speed, a scan places them, each particle
-// writes its pairs' force and torque about the owner's centre (in pair order) at its place, and
-// one thread per (512-particle chunk, body) adds its body's records over the chunk's range in
-// order (step.rs:173-221: chunk sums, in particle then pair order).
-template <bool WRITE>
-__global__ void k_mover_pairs(Params p, const StepConsts* __restrict__ sc, MoverDev M, const float4* __restrict__ pos,
-                              const float4* __restrict__ vel, const float* __restrict__ rho,
-                              const float* __restrict__ press, const float* __restrict__ scaled,
-                              const float4* __restrict__ centre, uint32_t* __restrict__ count,
-                              const uint32_t* __restrict__ offset, float4* __restrict__ pair) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
-    float4 a = pos[i], v = vel[i];
-    float density = rho[i];
-    float mirrored = scaled[i] + press[i] / p.rest_sq;
-    uint32_t k = WRITE ? offset[i] : 0u;
-    mover_pairs(p, M, sc->mover_damping, a, v, density, mirrored,
-                [&](uint32_t j, float gx, float gy, float gz, float, float damp, float toward) {
-                    float4 q = __ldg(&M.pos[j]);
-                    float ox = a.x - q.x, oy = a.y - q.y, oz = a.z - q.z;
-                    if (toward * toward < p.settles * dot3(ox, oy, oz, ox, oy, oz)) return;
-                    if (WRITE) {
-                        uint32_t b = __float_as_uint(q.w);
-                        float4 o = centre[b];
-                        float s = damp * p.mass;
-                        float ex = gx * s, ey = gy * s, ez = gz * s;
-                        float rx = q.x - o.x, ry = q.y - o.y, rz = q.z - o.z;
-                        pair[2 * size_t(k)] = make_float4(ex, ey, ez, q.w);
-                        pair[2 * size_t(k) + 1] =
-                            make_float4(ry * ez - ey * rz, rz * ex - ez * rx, rx * ey - ex * ry, 0.0f);
-                    }
-                    ++k;
-                });
-    if (!WRITE) count[i] = k;
-}
+// What the body points took from the water this substep (couple.rs:401-414): per 512-particle chunk
+// and body, the damping force and its torque about the body's centre, summed over the chunk's pairs in
+// particle then pair order (step.rs:173-221).  Pairs below the settling speed give nothing.  A block a
+// chunk: its threads count their particles' pairs, a scan places them, and the pairs go through shared
+// memory kFeltPairs at a time, where one thread per (body, component) adds them in order.  Most chunks
+// touch no body and end after the count.  felt[c * bodies + b] = (force, torque).
+// (As counts, a scan, a host wait for their total, pair records in memory and a thread per chunk and
+// body over them, before: five launches and a wait a substep.)
+constexpr int kFeltBlock = 512, kFeltPairs = 256;
 
-__global__ void k_mover_felt(uint32_t n, uint32_t bodies, const uint32_t* __restrict__ offset,
-                             const float4* __restrict__ pair, float4* __restrict__ felt) {
-    uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t chunks = (n + 511u) / 512u;
-    if (t >= chunks * bodies) return;
-    uint32_t c = t / bodies, b = t % bodies;
-    uint32_t from = offset[c * 512u], to = offset[min(n, (c + 1u) * 512u)];
-    float fx = 0.0f, fy = 0.0f, fz = 0.0f, tx = 0.0f, ty = 0.0f, tz = 0.0f;
-    for (uint32_t k = from; k < to; ++k) {
-        float4 f = pair[2 * size_t(k)];
-        if (__float_as_uint(f.w) != b) continue;
-        float4 q = pair[2 * size_t(k) + 1];
-        fx = fx + f.x;
-        fy = fy + f.y;
-        fz = fz + f.z;
-        tx = tx + q.x;
-        ty = ty + q.y;
-        tz = tz + q.z;
+__global__ void __launch_bounds__(kFeltBlock) k_mover_felt(const __grid_constant__ Params p,
+                                                           const StepConsts* __restrict__ sc,
+                                                           const __grid_constant__ MoverDev M,
+                                                           const float4* __restrict__ pos, const float4* __restrict__ vel,
+                                                           const float* __restrict__ rho, const float* __restrict__ press,
+                                                           const float* __restrict__ scaled,
+                                                           const float4* __restrict__ centre, float elapsed,
+                                                           uint32_t bodies, float4* __restrict__ felt) {
+    __shared__ float term[6][kFeltPairs];
+    __shared__ uint32_t owner[kFeltPairs];
+    __shared__ uint32_t warp_sums[kFeltBlock / 32];
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    float* const sums = reinterpret_cast<float*>(felt + 2 * size_t(blockIdx.x) * bodies);  // [b][8], 3 and 7 unused
+    for (uint32_t q = t; q < 8u * bodies; q += kFeltBlock) sums[q] = 0.0f;
+    const uint32_t i = blockIdx.x * uint32_t(kFeltBlock) + t;
+    const bool valid = i < p.n;
+    float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), v = a;
+    float density = 1.0f, mirrored = 0.0f;
+    if (valid) {
+        a = pos[i];
+        v = vel[i];
+        density = rho[i];
+        mirrored = scaled[i] + (press[i] > 0.0f ? press[i] / p.rest_sq : 0.0f);
     }
-    felt[2 * size_t(t)] = make_float4(fx, fy, fz, 0.0f);
-    felt[2 * size_t(t) + 1] = make_float4(tx, ty, tz, 0.0f);
+    // f(k, j, point, gradient * mass, damp) for the particle's k-th pair above the settling speed
+    auto pairs = [&](auto&& f) {
+        uint32_t k = 0;
+        mover_pairs(p, M, sc->mover_damping, a, v, density, mirrored,
+                    [&](uint32_t j, float gx, float gy, float gz, float, float damp, float toward) {
+                        const float4 q = __ldg(&M.pos[j]);
+                        const float ox = a.x - q.x, oy = a.y - q.y, oz = a.z - q.z;
+                        if (toward * toward < p.settles * dot3(ox, oy, oz, ox, oy, oz)) return;
+                        f(k, q, gx, gy, gz, damp);
+                        ++k;
+                    });
+        return k;
+    };
+    const uint32_t mine = valid ? pairs([](uint32_t, float4, float, float, float, float) {}) : 0u;
+    // where the particle's pairs stand among the chunk's
+    uint32_t upto = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t other = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= uint32_t(d)) upto += other;
+    }
+    __syncthreads();
+    if (lane == 31) warp_sums[warp] = upto;
+    __syncthreads();
+    uint32_t before = upto - mine, total = 0;
+#pragma unroll
+    for (int w = 0; w < kFeltBlock / 32; ++w) {
+        if (uint32_t(w) < warp) before += warp_sums[w];
+        total += warp_sums[w];
+    }
+    for (uint32_t base = 0; base < total; base += kFeltPairs) {
+        const uint32_t here = min(total - base, uint32_t(kFeltPairs));
+        if (mine && before < base + here && before + mine > base)
+            pairs([&](uint32_t k, float4 q, float gx, float gy, float gz, float damp) {
+                const uint32_t at = before + k - base;  // (wraps past `here` before the window)
+                if (at >= here) return;
+                const uint32_t b = __float_as_uint(q.w);
+                const float4 c = centre[2 * size_t(b)], u = centre[2 * size_t(b) + 1];
+                const float cx = c.x + u.x * elapsed, cy = c.y + u.y * elapsed, cz = c.z + u.z * elapsed;
+                const float s = damp * p.mass;
+                const float ex = gx * s, ey = gy * s, ez = gz * s;
+                const float rx = q.x - cx, ry = q.y - cy, rz = q.z - cz;
+                term[0][at] = ex;
+                term[1][at] = ey;
+                term[2][at] = ez;
+                term[3][at] = ry * ez - ey * rz;
+                term[4][at] = rz * ex - ez * rx;
+                term[5][at] = rx * ey - ex * ry;
+                owner[at] = b;
+            });
+        __syncthreads();
+        for (uint32_t q = t; q < 6u * bodies; q += kFeltBlock) {
+            const uint32_t b = q / 6u, c = q % 6u;
+            float* const to = sums + 8 * size_t(b) + c + (c >= 3u ? 1u : 0u);
+            float sum = *to;
+#pragma unroll 4
+            for (uint32_t k = 0; k < here; ++k)
+                if (owner[k] == b) sum = sum + term[c][k];
+            *to = sum;
+        }
+        __syncthreads();
+    }
 }
 
 // Whether any cell of the box [lo, hi] (cell keys) holds fluid in the last sort's dense table
@@ -1973,6 +2006,72 @@ __global__ void k_mover_order(uint32_t k, const uint32_t* __restrict__ lin, cons
     pos_out[d] = make_float4(s0.x + v.x * elapsed, s0.y + v.y * elapsed, s0.z + v.z * elapsed, s0.w);
 }
 
+// k_mover_cells, the scan and both phases of k_mover_order in one block, for the few thousand points and
+// cells of most scenes: the table is counted and scanned in shared memory.
+constexpr int kCarryBlock = 1024;
+constexpr uint32_t kCarryPoints = 16384, kCarryCells = 12000;  // 47 KB of table
+
+__global__ void __launch_bounds__(kCarryBlock) k_mover_carry(const __grid_constant__ Params p, uint32_t k,
+                                                             const float4* __restrict__ start,
+                                                             const float4* __restrict__ vel, float elapsed, int3 low,
+                                                             int3 span, uint32_t volume, uint32_t* lin, uint32_t* slot,
+                                                             uint32_t* __restrict__ table_out, uint32_t* members,
+                                                             float4* __restrict__ start_out, float4* __restrict__ vel_out,
+                                                             float4* __restrict__ pos_out) {
+    extern __shared__ uint32_t table[];  // volume words
+    __shared__ uint32_t warp_sums[kCarryBlock / 32];
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    for (uint32_t c = t; c < volume; c += kCarryBlock) table[c] = 0u;
+    __syncthreads();
+    for (uint32_t i = t; i < k; i += kCarryBlock) {
+        const float4 s0 = start[i], v = vel[i];
+        const float x = s0.x + v.x * elapsed, y = s0.y + v.y * elapsed, z = s0.z + v.z * elapsed;
+        const int3 c = cell_of(p, x, y, z);
+        const uint32_t l = uint32_t(((long long)(c.x - low.x) * span.y + (c.y - low.y)) * span.z + (c.z - low.z));
+        lin[i] = l;
+        slot[i] = atomicAdd(&table[l], 1u);
+    }
+    __syncthreads();
+    // exclusive scan: a run of cells a thread
+    const uint32_t per = (volume + kCarryBlock - 1) / kCarryBlock, c0 = min(t * per, volume), c1 = min(c0 + per, volume);
+    uint32_t sum = 0;
+    for (uint32_t c = c0; c < c1; ++c) sum += table[c];
+    uint32_t upto = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t other = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= uint32_t(d)) upto += other;
+    }
+    if (lane == 31) warp_sums[warp] = upto;
+    __syncthreads();
+    uint32_t at = upto - sum;
+    for (uint32_t w = 0; w < warp; ++w) at += warp_sums[w];
+    for (uint32_t c = c0; c < c1; ++c) {
+        const uint32_t here = table[c];
+        table[c] = at;
+        table_out[c] = at;
+        at += here;
+    }
+    if (t == 0) table_out[volume] = k;
+    __syncthreads();
+    for (uint32_t i = t; i < k; i += kCarryBlock) members[table[lin[i]] + slot[i]] = i;
+    __syncthreads();
+    for (uint32_t i = t; i < k; i += kCarryBlock) {
+        const uint32_t l = lin[i], b = table[l], e = l + 1u < volume ? table[l + 1u] : k;
+        const float4 s0 = start[i], v = vel[i];
+        const uint32_t own = __float_as_uint(s0.w);
+        uint32_t rank = 0;
+        for (uint32_t q = b; q < e; ++q) {
+            const uint32_t m = members[q], om = __float_as_uint(__ldg(&start[m].w));
+            rank += (om < own || (om == own && m < i)) ? 1u : 0u;
+        }
+        const uint32_t d = b + rank;
+        start_out[d] = s0;
+        vel_out[d] = v;
+        pos_out[d] = make_float4(s0.x + v.x * elapsed, s0.y + v.y * elapsed, s0.z + v.z * elapsed, s0.w);
+    }
+}
+
 // ---- the particles a coupled body's lift reads (lift.rs:29-60) -----------------------------------
 
 // keep[i] = 1 for a particle inside any of the boxes (low, high pairs, bounds inclusive, NaN
@@ -2238,22 +2337,13 @@ void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& 
                                                    st, vel_pre, T, slope, M);
 }
 
-void launch_mover_count(const Params& p, const StepConsts* sc, const MoverDev& M, const float4* pos,
-                        const float4* vel, const float* rho, const float* press, const float* scaled,
-                        uint32_t* count, cudaStream_t s) {
-    if (p.n)
-        k_mover_pairs<false><<<blocks_for(p.n), kBlock, 0, s>>>(p, sc, M, pos, vel, rho, press, scaled, nullptr, count,
-                                                                nullptr, nullptr);
-}
-
 void launch_mover_felt(const Params& p, const StepConsts* sc, const MoverDev& M, const float4* pos, const float4* vel,
-                       const float* rho, const float* press, const float* scaled, const float4* centre,
-                       uint32_t bodies, const uint32_t* offset, float4* pair, float4* felt, cudaStream_t s) {
+                       const float* rho, const float* press, const float* scaled, const float4* centre, float elapsed,
+                       uint32_t bodies, float4* felt, cudaStream_t s) {
     if (!p.n) return;
-    k_mover_pairs<true><<<blocks_for(p.n), kBlock, 0, s>>>(p, sc, M, pos, vel, rho, press, scaled, centre, nullptr,
-                                                           offset, pair);
-    uint32_t threads = (p.n + 511u) / 512u * bodies;
-    if (threads) k_mover_felt<<<(threads + 63u) / 64u, 64, 0, s>>>(p.n, bodies, offset, pair, felt);
+    static_assert(kFeltBlock == 512, "a block a chunk, a thread a particle");
+    k_mover_felt<<<(p.n + 511u) / 512u, kFeltBlock, 0, s>>>(p, sc, M, pos, vel, rho, press, scaled, centre, elapsed,
+                                                            bodies, felt);
     note_launch();
 }
 
@@ -2383,6 +2473,12 @@ void launch_carry_movers(const Params& p, uint32_t k, const float4* start, const
                          int3 span, uint32_t volume, uint32_t* lin, uint32_t* slot, uint32_t* table, uint32_t* tiles,
                          uint32_t* members, float4* start_out, float4* vel_out, float4* pos_out, cudaStream_t s) {
     if (!k) return;
+    if (k <= kCarryPoints && volume <= kCarryCells) {
+        k_mover_carry<<<1, kCarryBlock, volume * 4, s>>>(p, k, start, vel, elapsed, low, span, volume, lin, slot, table,
+                                                         members, start_out, vel_out, pos_out);
+        note_launch();
+        return;
+    }
     cudaMemsetAsync(table, 0, (size_t(volume) + 1) * 4, s);
     k_mover_cells<<<blocks_for(k), kBlock, 0, s>>>(p, k, start, vel, elapsed, low, span, lin, slot, table);
     launch_exclusive_scan(table, volume, tiles, s);

@@ -92,16 +92,12 @@ void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& 
                         const float* scaled, const float4* walls, float4* pos_out, float4* vel_out, Status* st,
                         float4* vel_pre, const TerrainDev& T, const float4* slope, cudaStream_t s,
                         const MoverDev& M = MoverDev{});
-// coupled bodies: each particle's count of pairs whose damping a body takes (count[i]); then,
-// with their exclusive scan in `offset` (n + 1 entries), the pairs' force and torque records and
-// per (512-particle chunk, body) their sums in order (felt: chunks x bodies pairs of float4); and
+// what the body points took this substep: per (512-particle chunk, body) their sums in order (felt:
+// chunks x bodies pairs of float4), about the centres centre[2 b] + centre[2 b + 1] elapsed; and
 // whether the last sort's table holds fluid in the cell box [lo, hi] (*wet set to 1, else left)
-void launch_mover_count(const Params& p, const StepConsts* sc, const MoverDev& M, const float4* pos,
-                        const float4* vel, const float* rho, const float* press, const float* scaled,
-                        uint32_t* count, cudaStream_t s);
 void launch_mover_felt(const Params& p, const StepConsts* sc, const MoverDev& M, const float4* pos, const float4* vel,
-                       const float* rho, const float* press, const float* scaled, const float4* centre,
-                       uint32_t bodies, const uint32_t* offset, float4* pair, float4* felt, cudaStream_t s);
+                       const float* rho, const float* press, const float* scaled, const float4* centre, float elapsed,
+                       uint32_t bodies, float4* felt, cudaStream_t s);
 // the bodies' felt records of a substep (launch_mover_felt) added into impulse[2 b] (force x dt)
 // and impulse[2 b + 1] (torque x dt), chunk by chunk in order
 void launch_mover_fold(uint32_t n, uint32_t bodies, const float4* felt, float dt, float4* impulse, cudaStream_t s);

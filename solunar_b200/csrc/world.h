@@ -582,9 +582,6 @@ struct World {
             for (auto* b : {&dmpos, &dmvel, &dcentre, &dfelt}) b->release(stream);
             dmstart.release(stream);
             dwet.release(stream);
-            dmcount.release(stream);
-            dmtiles.release(stream);
-            dmpair.release(stream);
             dmkeys.release(stream);
             rec_rate.release(stream);
             rec_vel.release(stream);
@@ -737,8 +734,7 @@ struct World {
     uint32_t mvolume = 0;
     DevBuf<float4> dmcur_start, dmcur_vel, dmnext_start, dmnext_vel;
     DevBuf<uint32_t> dmlin, dmslot, dmmembers, dmtable, dmtable_tiles;
-    DevBuf<uint32_t> dmcount, dmtiles;
-    DevBuf<float4> dmpair;
+    float melapsed = 0.0f;  // how far into the step the points stand
     DevBuf<int4> dmkeys;
     GridDev mgrid{};
 

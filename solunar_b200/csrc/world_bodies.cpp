@@ -175,13 +175,28 @@ int32_t World::plan_movers(float last) {
 }
 
 int32_t World::carry_movers(float elapsed, float last) {
-    if (elapsed == 0.0f) SLF_TRY(plan_movers(last));
+    melapsed = elapsed;
+    if (elapsed == 0.0f) {
+        SLF_TRY(plan_movers(last));
+        // each body's centre and velocity as the step begins, for what its points take (mover_felt)
+        std::vector<float4> centres;
+        for (const Coupled& known : coupled) {
+            centres.push_back(make_float4(known.center.x, known.center.y, known.center.z, 0.0f));
+            centres.push_back(make_float4(known.velocity.x, known.velocity.y, known.velocity.z, 0.0f));
+        }
+        SLF_TRY(dcentre.ensure(std::max<size_t>(centres.size(), 1), 0, stream));
+        SLF_CUDA(cudaMemcpyAsync(dcentre.p, centres.data(), centres.size() * sizeof(float4), cudaMemcpyHostToDevice,
+                                 stream));
+        SLF_CUDA(cudaStreamSynchronize(stream));  // the staging vector is pageable and freed next
+    }
     size_t k = m_start.size();
     if (k && mdevice) {
         for (auto& known : coupled) known.moved = known.velocity * elapsed;
-        launch_carry_movers(params(), uint32_t(k), dmcur_start.p, dmcur_vel.p, elapsed, mlow, mspan, mvolume, dmlin.p,
-                            dmslot.p, dmtable.p, dmtable_tiles.p, dmmembers.p, dmnext_start.p, dmnext_vel.p, dmpos.p,
-                            stream);
+        timed("bodies_carry", 0.0, [&] {
+            launch_carry_movers(params(), uint32_t(k), dmcur_start.p, dmcur_vel.p, elapsed, mlow, mspan, mvolume,
+                                dmlin.p, dmslot.p, dmtable.p, dmtable_tiles.p, dmmembers.p, dmnext_start.p,
+                                dmnext_vel.p, dmpos.p, stream);
+        });
         std::swap(dmcur_start, dmnext_start);
         std::swap(dmcur_vel, dmnext_vel);
         // the sorted velocities: dmcur_vel now; the grid: the dense table over the step's box
@@ -287,28 +302,15 @@ int32_t World::fastest_near_water(float dt, float slow, float& most) {
 
 int32_t World::mover_felt(float dt, const Params& p, int a, int nid) {
     if (coupled.empty() || m_pos.empty() || n == 0) return SLF_OK;
-    size_t bodies = coupled.size(), chunks = (n + 511) / 512;
-    std::vector<float4> centres(bodies);
-    for (size_t b = 0; b < bodies; ++b) {
-        F3 o = coupled[b].center + coupled[b].moved;
-        centres[b] = make_float4(o.x, o.y, o.z, 0.0f);
-    }
-    SLF_TRY(dcentre.ensure(bodies, 0, stream));
+    const size_t bodies = coupled.size(), chunks = (n + 511) / 512;
     SLF_TRY(dfelt.ensure(2 * chunks * bodies, 0, stream));
-    SLF_TRY(dmcount.ensure(n + 1, 0, stream));
-    SLF_TRY(dmtiles.ensure(scan_tiles(uint32_t(n)) + 1, 0, stream));
-    SLF_CUDA(cudaMemcpyAsync(dcentre.p, centres.data(), bodies * sizeof(float4), cudaMemcpyHostToDevice, stream));
-    launch_mover_count(p, d_consts, mover_dev(), pos[a].p, vel[a].p, rho[nid].p, press.p, scaled.p, dmcount.p,
-                       stream);
-    launch_exclusive_scan(dmcount.p, uint32_t(n), dmtiles.p, stream);
-    uint32_t total = 0;
-    SLF_CUDA(cudaMemcpyAsync(&total, dmcount.p + n, 4, cudaMemcpyDeviceToHost, stream));
-    SLF_TRY(sync());
-    SLF_TRY(dmpair.ensure(2 * size_t(std::max<uint32_t>(total, 1)), 0, stream));
-    launch_mover_felt(p, d_consts, mover_dev(), pos[a].p, vel[a].p, rho[nid].p, press.p, scaled.p, dcentre.p,
-                      uint32_t(bodies), dmcount.p, dmpair.p, dfelt.p, stream);
+    timed("bodies_felt", 0.0, [&] {
+        launch_mover_felt(p, d_consts, mover_dev(), pos[a].p, vel[a].p, rho[nid].p, press.p, scaled.p, dcentre.p,
+                          melapsed, uint32_t(bodies), dfelt.p, stream);
+    });
     // folded on the device into the step's impulses, read once when the step ends
-    launch_mover_fold(uint32_t(n), uint32_t(bodies), dfelt.p, dt, dimpulse.p, stream);
+    timed("bodies_fold", 0.0,
+          [&] { launch_mover_fold(uint32_t(n), uint32_t(bodies), dfelt.p, dt, dimpulse.p, stream); });
     return SLF_OK;
 }
 

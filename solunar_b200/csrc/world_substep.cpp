@@ -12,9 +12,8 @@ int32_t World::wcsph_substep(float dt, uint32_t& held) {
     SLF_TRY(plan_sort(sp, whole));
     if (whole) SLF_TRY(substep_graph(dt, p, a, b, nid, sp, whole));
     if (!whole) {
-        SLF_TRY(enqueue_sort(a, sp, stream));
-        SLF_TRY(reset_status());
-        launch_set_consts(consts(dt), d_consts, stream);
+        *h_consts = consts(dt);  // (the last launch that read them was waited for)
+        SLF_TRY(enqueue_sort(a, sp, stream, SubstepBegin{d_status, d_consts, h_consts}));
         PairLists fl = fluid_lists(), wl = wall_lists();
         timed("density", bytes_per_particle::density_wcsph,
               [&] { density_pass(p, a, fl, wl, rho[nid].p); });
