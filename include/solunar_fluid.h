@@ -350,7 +350,7 @@ int32_t slf_step_backward(slf_world* world, const float* dpositions, const float
 /* No counterpart in the reference: the cell sort of slf_update_neighbors for callers that
  * cannot allocate device memory (an engine that hands out all GPU memory from its own pool, a
  * plugin that only receives buffers from its host).  It allocates nothing: its scratch is one
- * fixed array in device memory, about 7.4 MB, that every GPU which loads this library holds
+ * fixed array in device memory, about 5.3 MB, that every GPU which loads this library holds
  * until the process exits.
  *
  * positions: n packed xyz float triples and ids: n ids, both in device memory; radius: the

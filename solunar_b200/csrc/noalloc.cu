@@ -13,6 +13,7 @@
 // the array and it keeps what the last call left in it; the kernels clear what must start at
 // zero.  Two calls whose work overlaps on the GPU (different streams, or different host threads)
 // race on it.
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstdint>
@@ -29,29 +30,21 @@ namespace slf {
 
 constexpr uint32_t kNoAllocMaxParticles = 1u << 18;  // 262,144 particles
 constexpr uint32_t kNoAllocMaxCells = 1u << 20;      // 1,048,576 cells in the bounding box
-constexpr uint32_t kNoAllocHeader = 64;               // bounding box, flags (u32 words)
-constexpr uint32_t kNoAllocTiles = (kNoAllocMaxCells + kBlock * 8 - 1) / (kBlock * 8) + 1;
+constexpr uint32_t kNoAllocHeader = 64;               // error flag, arrivals (u32 words)
+constexpr uint32_t kNoAllocBlocks = 256;  // most blocks of the sort's grid
 
 // word offsets inside the scratch array
-constexpr size_t kOffLin = kNoAllocHeader;
-constexpr size_t kOffSlot = kOffLin + kNoAllocMaxParticles;
-constexpr size_t kOffMembers = kOffSlot + kNoAllocMaxParticles;
+constexpr size_t kOffBounds = kNoAllocHeader;                  // each block's box (6 words)
+constexpr size_t kOffSums = kOffBounds + 6 * kNoAllocBlocks;   // each block's share of the counts
+constexpr size_t kOffMembers = kOffSums + kNoAllocBlocks;
 constexpr size_t kOffCount = kOffMembers + kNoAllocMaxParticles;
-constexpr size_t kOffTiles = kOffCount + kNoAllocMaxCells + 1;
-constexpr size_t kNoAllocWords = kOffTiles + kNoAllocTiles + 64;  // about 7.4 MB
+constexpr size_t kNoAllocWords = kOffCount + kNoAllocMaxCells + 1;  // about 5.3 MB
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
 
-// header words: cell box low (3), high (3), error flag
-enum { kHdrLo = 0, kHdrHi = 3, kHdrError = 6 };
-
-__global__ void k_na_reset(uint32_t* hdr) {
-    if (threadIdx.x < 3) {
-        reinterpret_cast<int*>(hdr)[kHdrLo + threadIdx.x] = INT_MAX;
-        reinterpret_cast<int*>(hdr)[kHdrHi + threadIdx.x] = INT_MIN;
-    }
-    if (threadIdx.x == 0) hdr[kHdrError] = 0;
-}
+// header words: error flag, the grid barrier's count of arrivals
+enum { kHdrError = 0, kHdrArrived = 1 };
+enum { kErrorBox = 1, kErrorWait = 2 };
 
 __device__ __forceinline__ int3 na_cell(const float* pos, uint32_t i, float radius) {
     // cell_of (src/fluid/mod.rs:526-533)
@@ -59,97 +52,173 @@ __device__ __forceinline__ int3 na_cell(const float* pos, uint32_t i, float radi
                      __float2int_rz(floorf(pos[3 * i + 2] / radius)));
 }
 
-__global__ void k_na_bounds(const float* __restrict__ pos, uint32_t n, float radius, uint32_t* hdr) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    // whether the warp holds a particle is its own flag: a particle's cell may itself saturate
-    // to INT_MAX or INT_MIN (a position of 1e30 at a small radius), so no cell value can
-    // stand for "none"
-    const bool any = __any_sync(0xffffffffu, i < n);
+// All blocks of the grid (a cooperative launch: they are on the GPU together) meet; `round` counts the
+// meetings.  A wait that runs out of patience reports itself and lets every block leave.
+__device__ __forceinline__ bool na_meet(uint32_t* hdr, uint32_t round) {
+    __shared__ bool met;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&hdr[kHdrArrived], 1u);
+        const uint32_t all = round * gridDim.x;
+        bool there = false;
+        for (uint32_t spin = 0; spin < (1u << 22) && !there; ++spin)
+            there = *reinterpret_cast<volatile uint32_t*>(&hdr[kHdrArrived]) >= all;
+        if (!there) atomicMax(&hdr[kHdrError], uint32_t(kErrorWait));
+        __threadfence();
+        met = there;
+    }
+    __syncthreads();
+    return met;
+}
+
+constexpr int kNoAllocThreads = 512;
+constexpr int kNoAllocItems = 4;  // particles a thread keeps in registers from pass to pass
+
+// The whole sort in one launch: the box of the cells, a count a cell, their scan, ids by cell, ranks.
+// The grid meets between the passes, each pass touches only the box's cells, and a thread's particles
+// (their cells, slots and ids) stay in its registers.  As eight launches over a table of every cell the
+// scratch holds, before: 95 -> 60 us a call at 201,544 particles (the call ends with a host wait).
+__global__ void __launch_bounds__(kNoAllocThreads) k_na_sort(const float* __restrict__ pos,
+                                                             const uint32_t* __restrict__ ids, uint32_t n, float radius,
+                                                             uint32_t* scratch, uint32_t* __restrict__ order) {
+    uint32_t* const hdr = scratch;
+    uint32_t* const count = scratch + kOffCount;
+    uint32_t* const members = scratch + kOffMembers;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, width = gridDim.x * kNoAllocThreads;
+    __shared__ int part[6][kNoAllocThreads / 32];
+    __shared__ uint32_t sums[kNoAllocThreads / 32];
+    int3 cell[kNoAllocItems];
+    uint32_t id[kNoAllocItems], lin[kNoAllocItems], slot[kNoAllocItems];
+    // (a thread without a particle takes part with an empty box)
     int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
-    if (i < n) {
-        int3 c = na_cell(pos, i, radius);
-        lo[0] = hi[0] = c.x;
-        lo[1] = hi[1] = c.y;
-        lo[2] = hi[2] = c.z;
+#pragma unroll
+    for (int k = 0; k < kNoAllocItems; ++k) {
+        const uint32_t i = blockIdx.x * kNoAllocThreads + t + k * width;
+        cell[k] = make_int3(0, 0, 0);
+        id[k] = lin[k] = slot[k] = 0u;
+        if (i >= n) continue;
+        cell[k] = na_cell(pos, i, radius);
+        id[k] = ids[i];
+        lo[0] = min(lo[0], cell[k].x), lo[1] = min(lo[1], cell[k].y), lo[2] = min(lo[2], cell[k].z);
+        hi[0] = max(hi[0], cell[k].x), hi[1] = max(hi[1], cell[k].y), hi[2] = max(hi[2], cell[k].z);
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = min(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = max(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
+        lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
+        hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
+        if (lane == 0) part[a][warp] = lo[a], part[3 + a][warp] = hi[a];
     }
-    if ((threadIdx.x & 31) == 0 && any) {
-        int* h = reinterpret_cast<int*>(hdr);
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(&h[kHdrLo + a], lo[a]);
-            atomicMax(&h[kHdrHi + a], hi[a]);
-        }
+    __syncthreads();
+    if (warp < 6) {  // a warp a bound
+        const int v = part[warp][lane % (kNoAllocThreads / 32)];
+        const int r = warp < 3 ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+        if (lane == 0) scratch[kOffBounds + 6 * blockIdx.x + warp] = uint32_t(r);
     }
-}
-
-__device__ __forceinline__ bool na_box(const uint32_t* hdr, int3& lo, int3& span) {
-    const int* h = reinterpret_cast<const int*>(hdr);
-    lo = make_int3(h[kHdrLo], h[kHdrLo + 1], h[kHdrLo + 2]);
-    long long sx = (long long)h[kHdrHi] - lo.x + 1, sy = (long long)h[kHdrHi + 1] - lo.y + 1,
-              sz = (long long)h[kHdrHi + 2] - lo.z + 1;
-    if (sx <= 0 || sy <= 0 || sz <= 0) return false;
+    if (!na_meet(hdr, 1)) return;
+    // every block takes the box from all blocks' bounds
+    __shared__ int box[6];
+    if (warp < 6) {
+        int v = warp < 3 ? INT_MAX : INT_MIN;
+        for (uint32_t b = lane; b < gridDim.x; b += 32) {
+            const int w = int(__ldcg(&scratch[kOffBounds + 6 * b + warp]));
+            v = warp < 3 ? min(v, w) : max(v, w);
+        }
+        v = warp < 3 ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+        if (lane == 0) box[warp] = v;
+    }
+    __syncthreads();
+    const long long sx = (long long)box[3] - box[0] + 1, sy = (long long)box[4] - box[1] + 1,
+                    sz = (long long)box[5] - box[2] + 1;
     // each side is at most 2^32 cells: bounding them first keeps the products inside 64 bits
     const long long cap = (long long)kNoAllocMaxCells;
-    if (sx > cap || sy > cap || sz > cap || sx * sy > cap || sx * sy * sz > cap) return false;
-    span = make_int3(int(sx), int(sy), int(sz));
-    return true;
-}
-
-__global__ void k_na_count(const float* __restrict__ pos, uint32_t n, float radius, uint32_t* scratch) {
-    uint32_t* hdr = scratch;
-    int3 lo, span;
-    if (!na_box(hdr, lo, span)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) hdr[kHdrError] = 1;
-        return;
+    if (sx <= 0 || sy <= 0 || sz <= 0 || sx > cap || sy > cap || sz > cap || sx * sy > cap || sx * sy * sz > cap) {
+        if (blockIdx.x == 0 && t == 0) atomicMax(&hdr[kHdrError], uint32_t(kErrorBox));
+        return;  // every block alike
     }
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int3 c = na_cell(pos, i, radius);
-    // offsets in 64 bits (a cell minus the box's low corner can pass the i32 range), and every
-    // particle checked against the box before it touches the count table: a cell outside it
-    // fails the call instead of writing outside the scratch array
-    const long long x = (long long)c.x - lo.x, y = (long long)c.y - lo.y, z = (long long)c.z - lo.z;
-    if (x < 0 || x >= span.x || y < 0 || y >= span.y || z < 0 || z >= span.z) {
-        hdr[kHdrError] = 1;
-        return;
+    const uint32_t volume = uint32_t(sx * sy * sz);
+    for (uint32_t c = blockIdx.x * kNoAllocThreads + t; c < volume; c += width) count[c] = 0u;
+    if (!na_meet(hdr, 2)) return;
+#pragma unroll
+    for (int k = 0; k < kNoAllocItems; ++k) {
+        if (blockIdx.x * kNoAllocThreads + t + k * width >= n) continue;
+        // offsets in 64 bits (a cell minus the box's low corner can pass the i32 range), and every
+        // particle checked against the box before it touches the count table: a cell outside it
+        // (another call's work on the scratch) fails the call instead of writing outside the array
+        const long long x = (long long)cell[k].x - box[0], y = (long long)cell[k].y - box[1],
+                        z = (long long)cell[k].z - box[2];
+        lin[k] = uint32_t((x * sy + y) * sz + z);
+        if (x < 0 || x >= sx || y < 0 || y >= sy || z < 0 || z >= sz) {
+            atomicMax(&hdr[kHdrError], uint32_t(kErrorBox));
+            lin[k] = 0u;
+        }
+        slot[k] = atomicAdd(&count[lin[k]], 1u);
     }
-    uint32_t l = uint32_t((x * span.y + y) * span.z + z);
-    scratch[kOffLin + i] = l;
-    scratch[kOffSlot + i] = atomicAdd(&scratch[kOffCount + l], 1u);
-}
-
-__global__ void k_na_members(uint32_t n, const uint32_t* __restrict__ ids, uint32_t* scratch) {
-    if (scratch[kHdrError]) return;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t l = scratch[kOffLin + i];
-    scratch[kOffMembers + scratch[kOffCount + l] + scratch[kOffSlot + i]] = ids[i];
-}
-
-// order[cell start + rank of the id in its cell] = i: the (cell, id) order of mod.rs:541-550.
-// A cell of k particles costs k comparisons a particle (k^2 for the cell).  Equal ids (a world's
-// ids are distinct; a caller's arrays need not be) are ranked by the slot each took in its cell,
-// so order is always a permutation, with repeated ids in no particular order among themselves.
-__global__ void k_na_order(uint32_t n, const uint32_t* __restrict__ ids, const uint32_t* __restrict__ scratch,
-                           uint32_t* __restrict__ order) {
-    if (scratch[kHdrError]) return;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t l = scratch[kOffLin + i];
-    uint32_t b = scratch[kOffCount + l], e = scratch[kOffCount + l + 1];
-    uint32_t id = ids[i], own = b + scratch[kOffSlot + i], rank = 0;
-    for (uint32_t k = b; k < e; ++k) {
-        uint32_t m = scratch[kOffMembers + k];
-        rank += (m < id || (m == id && k < own)) ? 1u : 0u;
+    if (!na_meet(hdr, 3)) return;
+    // exclusive scan: a run of cells a block, a run of those a thread (whole warps read side by side)
+    const uint32_t per = ((volume + gridDim.x - 1) / gridDim.x + 31u) & ~31u;
+    const uint32_t c0 = min(blockIdx.x * per, volume), c1 = min(c0 + per, volume);
+    uint32_t sum = 0;
+    for (uint32_t c = c0 + t; c < c1; c += kNoAllocThreads) sum += __ldcg(&count[c]);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) sums[warp] = sum;
+    __syncthreads();
+    if (t == 0) {
+        uint32_t all = 0;
+        for (int w = 0; w < kNoAllocThreads / 32; ++w) all += sums[w];
+        scratch[kOffSums + blockIdx.x] = all;
     }
-    order[b + rank] = i;
+    if (!na_meet(hdr, 4)) return;
+    uint32_t carry = 0;
+    for (uint32_t b = lane; b < blockIdx.x; b += 32) carry += __ldcg(&scratch[kOffSums + b]);
+    carry = __reduce_add_sync(0xffffffffu, carry);  // (every warp alike)
+    for (uint32_t base = c0; base < c1; base += kNoAllocThreads) {
+        const uint32_t c = base + t, v = c < c1 ? __ldcg(&count[c]) : 0u;
+        uint32_t upto = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t other = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= uint32_t(d)) upto += other;
+        }
+        __syncthreads();
+        if (lane == 31) sums[warp] = upto;
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < kNoAllocThreads / 32; ++w) {
+            if (uint32_t(w) < warp) before += sums[w];
+            all += sums[w];
+        }
+        if (c < c1) count[c] = carry + before + upto - v;
+        carry += all;
+    }
+    if (blockIdx.x == 0 && t == 0) count[volume] = n;
+    if (!na_meet(hdr, 5)) return;
+    uint32_t first[kNoAllocItems];
+#pragma unroll
+    for (int k = 0; k < kNoAllocItems; ++k) {
+        first[k] = 0u;
+        if (blockIdx.x * kNoAllocThreads + t + k * width >= n) continue;
+        first[k] = __ldcg(&count[lin[k]]);
+        if (first[k] < n && slot[k] < n - first[k]) members[first[k] + slot[k]] = id[k];
+    }
+    if (!na_meet(hdr, 6)) return;
+    // order[cell start + rank of the id in its cell] = i: the (cell, id) order of mod.rs:541-550.
+    // A cell of k particles costs k comparisons a particle (k^2 for the cell).  Equal ids (a world's
+    // ids are distinct; a caller's arrays need not be) are ranked by the slot each took in its cell,
+    // so order is always a permutation, with repeated ids in no particular order among themselves.
+#pragma unroll
+    for (int k = 0; k < kNoAllocItems; ++k) {
+        const uint32_t i = blockIdx.x * kNoAllocThreads + t + k * width;
+        if (i >= n) continue;
+        const uint32_t e = min(__ldcg(&count[lin[k] + 1]), n), own = first[k] + slot[k];
+        uint32_t rank = 0;
+        for (uint32_t q = first[k]; q < e; ++q) {
+            const uint32_t m = __ldcg(&members[q]);
+            rank += (m < id[k] || (m == id[k] && q < own)) ? 1u : 0u;
+        }
+        if (first[k] < n && rank < n - first[k]) order[first[k] + rank] = i;
+    }
 }
 
 namespace {
@@ -198,20 +267,26 @@ extern "C" int32_t slf_sort_by_cell_noalloc(const float* positions, const uint32
     if (st != SLF_OK) return st;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint32_t m = uint32_t(n);
-    uint32_t blocks = (m + kBlock - 1) / kBlock;
-    k_na_reset<<<1, 32, 0, s>>>(scratch);
-    cudaError_t e = cudaMemsetAsync(scratch + kOffCount, 0, (size_t(kNoAllocMaxCells) + 1) * 4, s);
-    if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "clearing the cell counts", e);
-    k_na_bounds<<<blocks, kBlock, 0, s>>>(positions, m, radius, scratch);
-    k_na_count<<<blocks, kBlock, 0, s>>>(positions, m, radius, scratch);
-    launch_exclusive_scan(scratch + kOffCount, kNoAllocMaxCells, scratch + kOffTiles, s);
-    k_na_members<<<blocks, kBlock, 0, s>>>(m, ids, scratch);
-    k_na_order<<<blocks, kBlock, 0, s>>>(m, ids, scratch, order);
-    e = cudaGetLastError();
+    // a block a SM at most, and no more than there are particles for: they all run at once
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "cudaDeviceGetAttribute", e);
+    uint32_t blocks = std::min<uint32_t>(uint32_t(sms), kNoAllocBlocks);
+    if (uint64_t(blocks) * kNoAllocThreads * kNoAllocItems < kNoAllocMaxParticles)
+        return na_fail(SLF_ERR_CUDA, "the device has too few SMs for the cell sort");
+    blocks = std::min(blocks, (m + 255u) / 256u);
+    blocks = std::max(blocks, (m + kNoAllocThreads * kNoAllocItems - 1u) / (kNoAllocThreads * kNoAllocItems));
+    e = cudaMemsetAsync(scratch, 0, 2 * 4, s);
+    if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "clearing the header", e);
+    void* args[] = {&positions, &ids, &m, &radius, &scratch, &order};
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_na_sort), dim3(blocks), dim3(kNoAllocThreads), args, 0, s);
+    note_launch();
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "launching the cell sort", e);
     e = cudaMemcpyAsync(&h_noalloc_error, scratch + kHdrError, 4, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "finishing the cell sort", e);
+    if (h_noalloc_error == kErrorWait) return na_fail(SLF_ERR_TIMEOUT, "the cell sort's blocks did not meet");
     if (h_noalloc_error) return na_fail(SLF_ERR_OUT_OF_RANGE, "particles spread over more cells than the scratch holds");
     return SLF_OK;
 }
