@@ -977,21 +977,8 @@ constexpr int kListUnroll = SLF_LIST_UNROLL;
 #define SLF_PUSH_MIN_BLOCKS 5
 #endif
 
-
-
-// Where a walk finds its neighbours (the global arrays, read through the L1).
-struct FromGlobal {
-    const float4* __restrict__ p;
-    const float4* __restrict__ v;
-    __device__ __forceinline__ void get(uint32_t j, float4& q) const { q = __ldg(&p[j]); }
-    __device__ __forceinline__ void get(uint32_t j, float4& q, float4& w) const {
-        q = __ldg(&p[j]);
-        w = __ldg(&v[j]);
-    }
-};
-
-template <class Src, class F>
-__device__ __forceinline__ void each_listed_from(const PairLists& l, uint32_t i, const Src& src, F&& f) {
+template <class F>
+__device__ __forceinline__ void each_listed(const PairLists& l, uint32_t i, const float4* __restrict__ pts, F&& f) {
     uint32_t n = l.count[i];
     if (n > l.cap) n = l.cap;
     if (n == 0) return;
@@ -1002,7 +989,7 @@ __device__ __forceinline__ void each_listed_from(const PairLists& l, uint32_t i,
     for (uint32_t k = 0; k < n; k += kListUnroll) {
         float4 q[kListUnroll];
 #pragma unroll
-        for (int u = 0; u < kListUnroll; ++u) src.get(e[u].x, q[u]);
+        for (int u = 0; u < kListUnroll; ++u) q[u] = __ldg(&pts[e[u].x]);
         uint2 next[kListUnroll];
 #pragma unroll
         for (int u = 0; u < kListUnroll; ++u) {
@@ -1017,14 +1004,10 @@ __device__ __forceinline__ void each_listed_from(const PairLists& l, uint32_t i,
     }
 }
 
-template <class F>
-__device__ __forceinline__ void each_listed(const PairLists& l, uint32_t i, const float4* __restrict__ pts, F&& f) {
-    each_listed_from(l, i, FromGlobal{pts, nullptr}, f);
-}
-
 // The same walk with a second array gathered alongside (velocities).
-template <class Src, class F>
-__device__ __forceinline__ void each_listed2_from(const PairLists& l, uint32_t i, const Src& src, F&& f) {
+template <class F>
+__device__ __forceinline__ void each_listed2(const PairLists& l, uint32_t i, const float4* __restrict__ pts,
+                                             const float4* __restrict__ more, F&& f) {
     uint32_t n = l.count[i];
     if (n > l.cap) n = l.cap;
     if (n == 0) return;
@@ -1035,7 +1018,10 @@ __device__ __forceinline__ void each_listed2_from(const PairLists& l, uint32_t i
     for (uint32_t k = 0; k < n; k += kListUnroll) {
         float4 q[kListUnroll], w[kListUnroll];
 #pragma unroll
-        for (int u = 0; u < kListUnroll; ++u) src.get(e[u].x, q[u], w[u]);
+        for (int u = 0; u < kListUnroll; ++u) {
+            q[u] = __ldg(&pts[e[u].x]);
+            w[u] = __ldg(&more[e[u].x]);
+        }
         uint2 next[kListUnroll];
 #pragma unroll
         for (int u = 0; u < kListUnroll; ++u) {
@@ -1050,47 +1036,8 @@ __device__ __forceinline__ void each_listed2_from(const PairLists& l, uint32_t i
     }
 }
 
-template <class F>
-__device__ __forceinline__ void each_listed2(const PairLists& l, uint32_t i, const float4* __restrict__ pts,
-                                             const float4* __restrict__ more, F&& f) {
-    each_listed2_from(l, i, FromGlobal{pts, more}, f);
-}
-
-// The solver check's walk over gradient entries (PairLists::gv): f(G, w) for each fluid neighbour
-// in list order, G the pair's kernel gradient and w = vel[index].  Entries stream evict-first,
-// kListUnroll at a time, the group's velocity gathers issued before any is used and the next
-// group's entries requested before this group is used; past the end of the list the last entry
-// is loaded again but not used.
-template <class F>
-__device__ __forceinline__ void each_gradient(const PairLists& l, uint32_t row, const float4* __restrict__ vel,
-                                              F&& f) {
-    uint32_t n = l.count[row];
-    if (n > l.cap) n = l.cap;
-    if (n == 0) return;
-    const float4* __restrict__ base = l.gv + l.at(row, 0);
-    float4 e[kListUnroll];
-#pragma unroll
-    for (int u = 0; u < kListUnroll; ++u) e[u] = SLF_LIST_LOAD(base + size_t(u < (int)n ? u : n - 1) * 32u);
-    for (uint32_t k = 0; k < n; k += kListUnroll) {
-        float4 w[kListUnroll];
-#pragma unroll
-        for (int u = 0; u < kListUnroll; ++u) w[u] = __ldg(&vel[__float_as_uint(e[u].w)]);
-        float4 next[kListUnroll];
-#pragma unroll
-        for (int u = 0; u < kListUnroll; ++u) {
-            uint32_t kk = k + kListUnroll + u;
-            next[u] = SLF_LIST_LOAD(base + size_t(kk < n ? kk : n - 1) * 32u);
-        }
-#pragma unroll
-        for (int u = 0; u < kListUnroll; ++u)
-            if (k + u < n) f(e[u], w[u]);
-#pragma unroll
-        for (int u = 0; u < kListUnroll; ++u) e[u] = next[u];
-    }
-}
-
-// The check's walk taking each slot in one of its two forms: slot k reads its kept gradient (16
-// bytes, then one gather: the neighbour's velocity) when bit k % 4 of GV_SLOTS is set, and its
+// The solver check's walk, w = vel[index], the entries streamed evict-first and requested a group
+// ahead.  Each slot takes one of two forms: slot k reads its kept gradient (PairLists::gv; 16 bytes, then one gather: the neighbour's velocity) when bit k % 4 of GV_SLOTS is set, and its
 // {index, g} entry (8 bytes, then two gathers: position and velocity, G = (a - q) g as the
 // density pass formed it) when not.  The first form moves more list bytes, the second gathers
 // more: mixing them balances the pass's DRAM stream against its gathers.  f(G, w) in list order.
@@ -1642,34 +1589,26 @@ __global__ void __launch_bounds__(kBlock, 3) k_wcsph_force(Params p, const StepC
 // ---- DFSPH ----------------------------------------------------------------------------------
 
 // density_rate (dfsph.rs:166-181), then the solve's stiffness and error (dfsph.rs:241-259) of
-// particle i, its neighbours taken from src.
-template <int WHICH, class Src>
+// particle i.  The lists always carry the kept gradients here, the walls' too: with no walk over
+// {index, g} entries beside this one the pass keeps its registers (76 -> 4 bytes spilled at 64
+// registers) and takes 106.2 us a launch at 1M, 37.9 at 250k, from 108.6 and 39.4.  Three blocks
+// a SM take 107.3 and 41.4, five (100 bytes spilled) 129.7 and 48.9.
+template <int WHICH>
 __device__ __forceinline__ void rate_particle(const Params& p, const StepConsts* __restrict__ sc,
-                                              const PairLists& fl, const PairLists& wl, uint32_t i, uint32_t row, const Src& src,
+                                              const PairLists& fl, const PairLists& wl, uint32_t i, uint32_t row,
                                               const float4* __restrict__ pos, const float4* __restrict__ vel,
                                               const float* __restrict__ rho, const float* __restrict__ alpha,
-                                              const float4* __restrict__ walls, float* __restrict__ kappa_w,
+                                              float* __restrict__ kappa_w,
                                               SolveRec rec, uint32_t slot, double& err, uint32_t& loaded) {
     const float dt = sc->dt;
     float4 a = pos[i];
     float4 v = vel[i];
     float rate = 0.0f;
-    if (fl.gv && wl.gv) {
-        // the gradients the density pass kept, for the slots that read them
-        each_gradient_mixed<SLF_RATE_GV_SLOTS>(fl, row, pos, vel, a, [&](float4 G, float4 w) {
-            rate += dot3(v.x - w.x, v.y - w.y, v.z - w.z, G.x, G.y, G.z);
-        });
-        each_wall_gradient(wl, row, [&](float4 G) { rate += dot3(v.x, v.y, v.z, G.x, G.y, G.z); });
-    } else {
-        each_listed2_from(fl, row, src, [&](uint32_t, float g, float4 q, float4 w) {
-            float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
-            rate += dot3(v.x - w.x, v.y - w.y, v.z - w.z, rx * g, ry * g, rz * g);
-        });
-        each_listed(wl, row, walls, [&](uint32_t, float g, float4 q) {
-            float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
-            rate += dot3(v.x, v.y, v.z, rx * g, ry * g, rz * g);
-        });
-    }
+    // the gradients the density pass kept, for the slots that read them
+    each_gradient_mixed<SLF_RATE_GV_SLOTS>(fl, row, pos, vel, a, [&](float4 G, float4 w) {
+        rate += dot3(v.x - w.x, v.y - w.y, v.z - w.z, G.x, G.y, G.z);
+    });
+    each_wall_gradient(wl, row, [&](float4 G) { rate += dot3(v.x, v.y, v.z, G.x, G.y, G.z); });
     rate = rate * p.mass;
     if (rec.rate) {  // recorded for the adjoint
         size_t at = size_t(slot) * p.n + i;
@@ -1699,8 +1638,8 @@ template <int WHICH>
 __global__ void __launch_bounds__(kBlock, SLF_RATE_MIN_BLOCKS) k_rate(Params p, const StepConsts* __restrict__ sc, PairLists fl,
                                                  PairLists wl, const float4* __restrict__ pos,
                                                  const float4* __restrict__ vel, const float* __restrict__ rho,
-                                                 const float* __restrict__ alpha, const float4* __restrict__ walls,
-                                                 float* __restrict__ kappa_w, DD* __restrict__ partial,
+                                                 const float* __restrict__ alpha, float* __restrict__ kappa_w,
+                                                 DD* __restrict__ partial,
                                                  uint32_t* __restrict__ partial_loaded, Status* st,
                                                  SolveRec rec, unsigned long long loop) {
     // a solve that already stopped leaves the rest of its batch of launches idle
@@ -1714,8 +1653,7 @@ __global__ void __launch_bounds__(kBlock, SLF_RATE_MIN_BLOCKS) k_rate(Params p, 
         const uint32_t i = fl.particle(row);
         double err = 0.0;
         uint32_t one = 0;
-        rate_particle<WHICH>(p, sc, fl, wl, i, row, FromGlobal{pos, vel}, pos, vel, rho, alpha, walls, kappa_w, rec, slot,
-                             err, one);
+        rate_particle<WHICH>(p, sc, fl, wl, i, row, pos, vel, rho, alpha, kappa_w, rec, slot, err, one);
         acc = dd_add(acc, DD{err, 0.0});
         loaded += one;
     }
@@ -1723,29 +1661,30 @@ __global__ void __launch_bounds__(kBlock, SLF_RATE_MIN_BLOCKS) k_rate(Params p, 
 }
 
 // push_apart (dfsph.rs:184-216) of particle i: the velocity change from each particle's
-// stiffness, which the rate pass left in the w lane of each position.
-template <class Src>
+// stiffness, which the rate pass left in the w lane of each position.  Fluid pairs read {index, g}
+// and gather that record: a kept gradient in the entry's place moves 8 bytes more for nothing,
+// with the stiffness alone gathered too (1 to 4 slots in four: 78 to 100 us at 1M against 72).
+// Wall pairs need no gather at all from their kept gradients: 72 -> 69 us.
 __device__ __forceinline__ void push_particle(const Params& p, const StepConsts* __restrict__ sc, const PairLists& fl,
-                                              const PairLists& wl, uint32_t i, uint32_t row, const Src& src,
+                                              const PairLists& wl, uint32_t i, uint32_t row,
                                               const float4* __restrict__ pos, float4* __restrict__ vel,
-                                              const float4* __restrict__ walls, float* __restrict__ applied) {
+                                              float* __restrict__ applied) {
     const float dt = sc->dt;
     float4 a = pos[i];
     float own = a.w;
     float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-    each_listed_from(fl, row, src, [&](uint32_t, float g, float4 q) {
+    each_listed(fl, row, pos, [&](uint32_t, float g, float4 q) {
         float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
         float s = p.mass * (own + q.w);
         cx = cx - (rx * g) * s;
         cy = cy - (ry * g) * s;
         cz = cz - (rz * g) * s;
     });
-    each_listed(wl, row, walls, [&](uint32_t, float g, float4 q) {
-        float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
-        float s = p.mass * own;
-        cx = cx - (rx * g) * s;
-        cy = cy - (ry * g) * s;
-        cz = cz - (rz * g) * s;
+    const float ws = p.mass * own;
+    each_wall_gradient(wl, row, [&](float4 G) {
+        cx = cx - G.x * ws;
+        cy = cy - G.y * ws;
+        cz = cz - G.z * ws;
     });
     float4 v = vel[i];
     v.x = v.x + cx * dt;
@@ -1758,12 +1697,12 @@ __device__ __forceinline__ void push_particle(const Params& p, const StepConsts*
 
 __global__ void __launch_bounds__(kBlock, SLF_PUSH_MIN_BLOCKS) k_push(Params p, const StepConsts* __restrict__ sc, PairLists fl,
                                                  PairLists wl, const float4* __restrict__ pos,
-                                                 float4* __restrict__ vel, const float4* __restrict__ walls,
-                                                 Status* st, float* __restrict__ applied, unsigned long long loop) {
+                                                 float4* __restrict__ vel, Status* st,
+                                                 float* __restrict__ applied, unsigned long long loop) {
     loop_bound(p, st, loop);
     if (__ldcg(&st->settled)) return;
     for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < p.n; row += gridDim.x * blockDim.x)
-        push_particle(p, sc, fl, wl, fl.particle(row), row, FromGlobal{pos, nullptr}, pos, vel, walls, applied);
+        push_particle(p, sc, fl, wl, fl.particle(row), row, pos, vel, applied);
 }
 
 // viscous (step.rs:229-251) + gravity of particle i (row `row` of the walk order)
@@ -2398,24 +2337,24 @@ size_t rate_partial_bytes(uint32_t n) { return (n + kBlock - 1) / kBlock * (size
 
 
 void launch_rate(int which, const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,
-                 float4* pos, const float4* vel, const float* rho, const float* alpha, const float4* walls,
-                 void* partials, Status* st, SolveRec rec, cudaStream_t s, unsigned long long loop) {
+                 float4* pos, const float4* vel, const float* rho, const float* alpha, void* partials,
+                 Status* st, SolveRec rec, cudaStream_t s, unsigned long long loop) {
     if (!p.n) return;
     // the partials' room is for one block a 256 rows; the grid takes at most that many
     uint32_t nb = solver_blocks(p.n, which == 0 ? 0 : 1);
     DD* part = static_cast<DD*>(partials);
     uint32_t* loaded = reinterpret_cast<uint32_t*>(part + (p.n + kBlock - 1) / kBlock);
     if (which == 0)
-        k_rate<0><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, alpha, walls, reinterpret_cast<float*>(pos),
-                                        part, loaded, st, rec, loop);
+        k_rate<0><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, alpha, reinterpret_cast<float*>(pos), part,
+                                        loaded, st, rec, loop);
     else
-        k_rate<1><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, alpha, walls, reinterpret_cast<float*>(pos),
-                                        part, loaded, st, rec, loop);
+        k_rate<1><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, alpha, reinterpret_cast<float*>(pos), part,
+                                        loaded, st, rec, loop);
 }
 
 void launch_push(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl, const float4* pos,
-                 float4* vel, const float4* walls, Status* st, float* applied, cudaStream_t s, unsigned long long loop) {
-    if (p.n) k_push<<<solver_blocks(p.n, 2), kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, walls, st, applied, loop);
+                 float4* vel, Status* st, float* applied, cudaStream_t s, unsigned long long loop) {
+    if (p.n) k_push<<<solver_blocks(p.n, 2), kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, st, applied, loop);
 }
 
 // Warm start of a solve: the stiffness that applies `share` of the impulse S the particle's last

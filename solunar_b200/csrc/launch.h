@@ -116,12 +116,11 @@ void prepare_fast_grids();
 // loop (optional): the while-node handle of a solve captured as a CUDA graph; the check that
 // stops the solve ends that loop, and the push bounds it at max_iterations + 1 bodies.
 void launch_rate(int which, const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,
-                 float4* pos, const float4* vel, const float* rho, const float* alpha, const float4* walls,
-                 void* partials, Status* st, SolveRec rec, cudaStream_t s, unsigned long long loop = 0);
+                 float4* pos, const float4* vel, const float* rho, const float* alpha, void* partials, Status* st,
+                 SolveRec rec, cudaStream_t s, unsigned long long loop = 0);
 // applied (optional, stride 2): each particle's stiffness impulse sum, for warm starts
 void launch_push(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl, const float4* pos,
-                 float4* vel, const float4* walls, Status* st, float* applied, cudaStream_t s,
-                 unsigned long long loop = 0);
+                 float4* vel, Status* st, float* applied, cudaStream_t s, unsigned long long loop = 0);
 // warm start: pos.w = share * applied / dt, applied = that stiffness * dt
 void launch_warm_kappa(const Params& p, const StepConsts* sc, float share, float* applied, float4* pos, cudaStream_t s);
 void launch_viscous(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl, const float4* pos,

@@ -27,10 +27,6 @@
 
 #include "../../include/solunar_fluid.h"
 
-// EXACT DFSPH keeps each pair's gradient for the solver check (0: the check gathers positions)
-#ifndef SLF_KEEP_GRADIENTS
-#define SLF_KEEP_GRADIENTS 1
-#endif
 #include "launch.h"
 
 namespace slf {
@@ -691,7 +687,8 @@ struct World {
     const uint32_t* walk_order() const { return worder_valid ? worder.p : nullptr; }
     // EXACT DFSPH keeps each pair's gradient for the solver check (16 bytes a slot, fluid and
     // walls): the check then gathers a neighbour's velocity only, not its position too
-    bool keeps_gradients() const { return SLF_KEEP_GRADIENTS && !fast() && s.solver == SLF_SOLVER_DFSPH; }
+    // EXACT DFSPH keeps each pair's gradient for the solver check, and the walls' for the push
+    bool keeps_gradients() const { return !fast() && s.solver == SLF_SOLVER_DFSPH; }
     PairLists fluid_lists() const {
         return PairLists{list_cap, fent.p, fcnt.p, walk_order(), keeps_gradients() ? fgv.p : nullptr};
     }

@@ -373,15 +373,15 @@ void World::rate_pass(int which, const Params& p, const PairLists& fl, const Pai
         launch_rate_fast(which, rel(), p, d_consts, fl, wl, pos[a].p, v, rho[nid].p, alpha.p, dwalls.p,
                          partials.p, d_status, rec, on, loop);
     else
-        launch_rate(which, p, d_consts, fl, wl, pos[a].p, v, rho[nid].p, alpha.p, dwalls.p, partials.p, d_status,
-                    rec, on, loop);
+        launch_rate(which, p, d_consts, fl, wl, pos[a].p, v, rho[nid].p, alpha.p, partials.p, d_status, rec,
+                    on, loop);
 }
 
 void World::push_pass(const Params& p, const PairLists& fl, const PairLists& wl, int a, float4* v, float* applied,
                       cudaStream_t cs, unsigned long long loop) {
     cudaStream_t on = cs ? cs : stream;
     if (fast()) launch_push_fast(rel(), p, d_consts, fl, wl, pos[a].p, v, dwalls.p, d_status, applied, on, loop);
-    else launch_push(p, d_consts, fl, wl, pos[a].p, v, dwalls.p, d_status, applied, on, loop);
+    else launch_push(p, d_consts, fl, wl, pos[a].p, v, d_status, applied, on, loop);
 }
 
 void World::advance_pass(const Params& p, int a, int b, float4* pre, cudaStream_t on) {
