@@ -395,7 +395,9 @@ struct World {
     TerrainDev tdev{};
 
     Status* d_status = nullptr;
-    Status* h_status = nullptr;
+    Status* h_status = nullptr;     // pinned
+    uint32_t* h_posted = nullptr;   // pinned: nonzero once the status asked for is in h_status
+    bool polls = true;              // waits for it by polling (unless the device is set to block)
     StepConsts* d_consts = nullptr;
     StepConsts* h_consts = nullptr;  // pinned: the constants of the next substep run as a graph
 
@@ -595,6 +597,7 @@ struct World {
             if (d_status) cudaFree(d_status);
             if (d_consts) cudaFree(d_consts);
             if (h_status) cudaFreeHost(h_status);
+            if (h_posted) cudaFreeHost(h_posted);
             if (h_consts) cudaFreeHost(h_consts);
             cudaStreamDestroy(stream);
         }
@@ -846,9 +849,17 @@ struct World {
         return SLF_OK;
     }
 
+    // The status into h_status: post_status queues the kernel that writes it there (a recorded substep
+    // ends with that kernel itself), await_status waits for it.  Every post is waited for before the next.
+    void expect_status() { *static_cast<volatile uint32_t*>(h_posted) = 0; }
+    void post_status() {
+        expect_status();
+        launch_post_status(d_status, h_status, h_posted, stream);
+    }
+    int32_t await_status();
     int32_t read_status() {
-        SLF_CUDA(cudaMemcpyAsync(h_status, d_status, sizeof(Status), cudaMemcpyDeviceToHost, stream));
-        return sync();
+        post_status();
+        return await_status();
     }
 
     // Clears the per-substep fields; the box starts empty.

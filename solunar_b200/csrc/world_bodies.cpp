@@ -310,7 +310,7 @@ int32_t World::mover_felt(float dt, const Params& p, int a, int nid) {
     });
     // folded on the device into the step's impulses, read once when the step ends
     timed("bodies_fold", 0.0,
-          [&] { launch_mover_fold(uint32_t(n), uint32_t(bodies), dfelt.p, dt, dimpulse.p, stream); });
+          [&] { launch_mover_fold(uint32_t(n), uint32_t(bodies), dfelt.p, dt, dimpulse.p, d_status, list_cap, stream); });
     return SLF_OK;
 }
 

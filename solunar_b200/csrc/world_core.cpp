@@ -1,4 +1,7 @@
 // world_core.cpp -- World's settings, particles, status, the spatial hash and read-outs of the world.
+#include <atomic>
+#include <chrono>
+
 #include "world.h"
 
 namespace slf {
@@ -49,6 +52,11 @@ int32_t World::init(const slf_settings& settings) {
     SLF_CUDA(cudaMalloc(&d_consts, sizeof(StepConsts)));
     SLF_CUDA(cudaMallocHost(&h_status, sizeof(Status)));
     std::memset(h_status, 0, sizeof(Status));
+    SLF_CUDA(cudaMallocHost(&h_posted, sizeof(uint32_t)));
+    *h_posted = 0;
+    unsigned int flags = 0;
+    SLF_CUDA(cudaGetDeviceFlags(&flags));
+    polls = (flags & cudaDeviceScheduleMask) != cudaDeviceScheduleBlockingSync;
     SLF_CUDA(cudaMallocHost(&h_consts, sizeof(StepConsts)));
     SLF_CUDA(cudaMemsetAsync(d_status, 0, sizeof(Status), stream));
     build_ground_sites();
@@ -420,6 +428,27 @@ Status World::fresh_status() {
 int32_t World::reset_status() {
     *h_status = fresh_status();
     SLF_CUDA(cudaMemcpyAsync(d_status, h_status, sizeof(Status), cudaMemcpyHostToDevice, stream));
+    return SLF_OK;
+}
+
+int32_t World::await_status() {
+    // (a profile needs its events finished; work that takes longer, or failed, the stream's wait sees)
+    if (polls && !prof.on) {
+        const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(20);
+        do {
+            for (int k = 0; k < 64; ++k) {
+                if (*static_cast<volatile uint32_t*>(h_posted)) {
+                    std::atomic_thread_fence(std::memory_order_acquire);
+                    return SLF_OK;
+                }
+#if defined(__x86_64__)
+                __builtin_ia32_pause();
+#endif
+            }
+        } while (std::chrono::steady_clock::now() < until);
+    }
+    SLF_TRY(sync());
+    if (!*static_cast<volatile uint32_t*>(h_posted)) return fail(SLF_ERR_CUDA, "the status was not written");
     return SLF_OK;
 }
 

@@ -20,10 +20,13 @@ int32_t World::wcsph_substep(float dt, uint32_t& held) {
         timed("wcsph_force_advance", bytes_per_particle::wcsph_force,
               [&] { force_pass(p, fl, wl, a, b, nid); });
     }
-    SLF_TRY(read_status());
+    if (!whole) post_status();
+    // what the bodies' points take is queued behind the status: it runs while the host reads that
+    const int32_t felt = mover_felt(dt, p, a, nid);
+    SLF_TRY(await_status());
     SLF_TRY(lists_fit());
     SLF_TRY(check_state());
-    SLF_TRY(mover_felt(dt, p, a, nid));
+    SLF_TRY(felt);
     held = h_status->held;
     cpos = b;
     cid = nid;
@@ -269,6 +272,7 @@ int32_t World::capture_substep(const Params& p, int a, int b, int nid, const Sor
         density_pass(p, a, fl, wl, rho[nid].p, cs);
         if (s.solver == SLF_SOLVER_WCSPH) {
             force_pass(p, fl, wl, a, b, nid, cs);
+            launch_post_status(d_status, h_status, h_posted, cs);
             return SLF_OK;
         }
         uint32_t pre = 0;
@@ -276,6 +280,7 @@ int32_t World::capture_substep(const Params& p, int a, int b, int nid, const Sor
         viscous_pass(p, fl, wl, a, b, nid, cs);
         SLF_TRY(capture_solve(1, p, a, vel[b].p, nid, fl, wl, SolveRec{nullptr, nullptr}, pre));
         advance_pass(p, a, b, vel_pre, cs);
+        launch_post_status(d_status, h_status, h_posted, cs);
         return SLF_OK;
     };
     int32_t st = record();
@@ -329,6 +334,7 @@ int32_t World::substep_graph(float dt, const Params& p, int a, int b, int nid, c
     hit->used = ++graph_clock;
     ++hit->runs;
     *h_consts = consts(dt);  // (the last launch that read them was waited for)
+    expect_status();
     SLF_CUDA(cudaGraphLaunch(hit->exec, stream));
     note_launches(hit->outside);
     graph_solves = s.solver == SLF_SOLVER_DFSPH ? 3u : 0u;
@@ -424,7 +430,8 @@ int32_t World::dfsph_substep(float dt, uint32_t& held, uint32_t& iterations, Dfs
         }
         timed("advance", bytes_per_particle::advance, [&] { advance_pass(p, a, b, pre); });
     }
-    SLF_TRY(read_status());
+    if (!whole) post_status();
+    SLF_TRY(await_status());
     if (graph_solves) {
         uint32_t its[2] = {div_it, den_it};
         SLF_TRY(finish_graph_solves(its));
