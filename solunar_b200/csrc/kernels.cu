@@ -87,12 +87,15 @@ __global__ void k_max_compression(Params p, const float* __restrict__ rho, Statu
 
 // The status into the host's pinned copy, then the word the host polls.  A copy and a stream
 // synchronisation in its place take about 6 us more a wait: 44 -> 38 us a substep of 720 particles.
-__global__ void __launch_bounds__(32) k_post_status(const Status* st, Status* out, uint32_t* posted) {
+// spoiled (optional): whether the substep's lists outgrew cap or its values are non-finite.
+__global__ void __launch_bounds__(32) k_post_status(const Status* st, Status* out, uint32_t* posted, uint32_t cap,
+                                                    uint32_t* spoiled) {
     constexpr uint32_t words = sizeof(Status) / 4;
     static_assert(sizeof(Status) % 4 == 0 && words <= 32, "a word a lane");
     const uint32_t t = threadIdx.x;
     if (t < words)
         reinterpret_cast<volatile uint32_t*>(out)[t] = reinterpret_cast<const volatile uint32_t*>(st)[t];
+    if (t == 0 && spoiled) *spoiled = st->list_max > cap || st->nonfinite ? 1u : 0u;
     __threadfence_system();
     __syncwarp();
     if (t == 0) *reinterpret_cast<volatile uint32_t*>(posted) = 1u;
@@ -1247,7 +1250,7 @@ __device__ __forceinline__ void mover_pairs(const Params& p, const MoverDev& M, 
 constexpr int kFeltBlock = 512, kFeltPairs = 256;
 
 __global__ void __launch_bounds__(kFeltBlock) k_mover_felt(const __grid_constant__ Params p,
-                                                           const StepConsts* __restrict__ sc,
+                                                           float mover_damping,
                                                            const __grid_constant__ MoverDev M,
                                                            const float4* __restrict__ pos, const float4* __restrict__ vel,
                                                            const float* __restrict__ rho, const float* __restrict__ press,
@@ -1273,7 +1276,7 @@ __global__ void __launch_bounds__(kFeltBlock) k_mover_felt(const __grid_constant
     // f(k, j, point, gradient * mass, damp) for the particle's k-th pair above the settling speed
     auto pairs = [&](auto&& f) {
         uint32_t k = 0;
-        mover_pairs(p, M, sc->mover_damping, a, v, density, mirrored,
+        mover_pairs(p, M, mover_damping, a, v, density, mirrored,
                     [&](uint32_t j, float gx, float gy, float gz, float, float damp, float toward) {
                         const float4 q = __ldg(&M.pos[j]);
                         const float ox = a.x - q.x, oy = a.y - q.y, oz = a.z - q.z;
@@ -2155,9 +2158,10 @@ void launch_max_compression(const Params& p, const float* rho, Status* st, cudaS
     if (p.n) k_max_compression<<<blocks_for(p.n), kBlock, 0, s>>>(p, rho, st);
 }
 
-void launch_post_status(const Status* st, Status* out, uint32_t* posted, cudaStream_t s) {
+void launch_post_status(const Status* st, Status* out, uint32_t* posted, cudaStream_t s, uint32_t cap,
+                        uint32_t* spoiled) {
     note_launch();
-    k_post_status<<<1, 32, 0, s>>>(st, out, posted);
+    k_post_status<<<1, 32, 0, s>>>(st, out, posted, cap, spoiled);
 }
 
 void launch_count_cells(const Params& p, const float4* pos, const int4* cells, int3 low, int3 span, uint32_t* count,
@@ -2294,12 +2298,12 @@ void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& 
                                                    st, vel_pre, T, slope, M);
 }
 
-void launch_mover_felt(const Params& p, const StepConsts* sc, const MoverDev& M, const float4* pos, const float4* vel,
+void launch_mover_felt(const Params& p, float mover_damping, const MoverDev& M, const float4* pos, const float4* vel,
                        const float* rho, const float* press, const float* scaled, const float4* centre, float elapsed,
                        uint32_t bodies, float4* felt, cudaStream_t s) {
     if (!p.n) return;
     static_assert(kFeltBlock == 512, "a block a chunk, a thread a particle");
-    k_mover_felt<<<(p.n + 511u) / 512u, kFeltBlock, 0, s>>>(p, sc, M, pos, vel, rho, press, scaled, centre, elapsed,
+    k_mover_felt<<<(p.n + 511u) / 512u, kFeltBlock, 0, s>>>(p, mover_damping, M, pos, vel, rho, press, scaled, centre, elapsed,
                                                             bodies, felt);
     note_launch();
 }
@@ -2311,8 +2315,8 @@ void launch_mover_felt(const Params& p, const StepConsts* sc, const MoverDev& M,
 // A substep that will run again or fails (its lists outgrew cap, or it left non-finite values) adds
 // nothing: its chunks are queued before the host has read its status.
 __global__ void k_mover_fold(uint32_t chunks, uint32_t bodies, const float4* __restrict__ felt, float dt,
-                             float4* __restrict__ impulse, const Status* __restrict__ st, uint32_t cap) {
-    if (st->list_max > cap || st->nonfinite) return;
+                             float4* __restrict__ impulse, const uint32_t* __restrict__ spoiled) {
+    if (*spoiled) return;
     __shared__ float4 force[kBlock], torque[kBlock];
     const uint32_t b = blockIdx.x, t = threadIdx.x;
     float4 imp = impulse[2 * size_t(b)], ang = impulse[2 * size_t(b) + 1];
@@ -2340,10 +2344,10 @@ __global__ void k_mover_fold(uint32_t chunks, uint32_t bodies, const float4* __r
     }
 }
 
-void launch_mover_fold(uint32_t n, uint32_t bodies, const float4* felt, float dt, float4* impulse, const Status* st,
-                       uint32_t cap, cudaStream_t s) {
+void launch_mover_fold(uint32_t n, uint32_t bodies, const float4* felt, float dt, float4* impulse,
+                       const uint32_t* spoiled, cudaStream_t s) {
     if (!n || !bodies) return;
-    k_mover_fold<<<bodies, kBlock, 0, s>>>((n + 511u) / 512u, bodies, felt, dt, impulse, st, cap);
+    k_mover_fold<<<bodies, kBlock, 0, s>>>((n + 511u) / 512u, bodies, felt, dt, impulse, spoiled);
     note_launch();
 }
 

@@ -22,8 +22,10 @@ struct SubstepBegin {
     const StepConsts* from;
 };
 
-// the status into the host's pinned copy, then 1 into the word beside it
-void launch_post_status(const Status* st, Status* out, uint32_t* posted, cudaStream_t s);
+// the status into the host's pinned copy, then 1 into the word beside it; spoiled (optional): whether
+// the substep will run again or fails
+void launch_post_status(const Status* st, Status* out, uint32_t* posted, cudaStream_t s, uint32_t cap = 0,
+                        uint32_t* spoiled = nullptr);
 
 // counting sort by dense cell index; cells (cell-relative positions) optional
 void launch_count_cells(const Params& p, const float4* pos, const int4* cells, int3 low, int3 span, uint32_t* count,
@@ -98,13 +100,13 @@ void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& 
 // what the body points took this substep: per (512-particle chunk, body) their sums in order (felt:
 // chunks x bodies pairs of float4), about the centres centre[2 b] + centre[2 b + 1] elapsed; and
 // whether the last sort's table holds fluid in the cell box [lo, hi] (*wet set to 1, else left)
-void launch_mover_felt(const Params& p, const StepConsts* sc, const MoverDev& M, const float4* pos, const float4* vel,
+void launch_mover_felt(const Params& p, float mover_damping, const MoverDev& M, const float4* pos, const float4* vel,
                        const float* rho, const float* press, const float* scaled, const float4* centre, float elapsed,
                        uint32_t bodies, float4* felt, cudaStream_t s);
 // the bodies' felt records of a substep (launch_mover_felt) added into impulse[2 b] (force x dt)
 // and impulse[2 b + 1] (torque x dt), chunk by chunk in order
-void launch_mover_fold(uint32_t n, uint32_t bodies, const float4* felt, float dt, float4* impulse, const Status* st,
-                       uint32_t cap, cudaStream_t s);
+void launch_mover_fold(uint32_t n, uint32_t bodies, const float4* felt, float dt, float4* impulse,
+                       const uint32_t* spoiled, cudaStream_t s);
 void launch_cells_wet(const GridDev& g, int3 lo, int3 hi, uint32_t* wet, cudaStream_t s);
 size_t rate_partial_bytes(uint32_t n);
 // Looks up, once per process, how many blocks of the solver passes the device holds at once (not

@@ -616,6 +616,7 @@ int32_t World::step_untaped(float dt, slf_report* out) {
                 SLF_TRY(st);
                 r.held_back += held;
             }
+            SLF_TRY(join_bodies());
             r.substeps = substeps;
         } else {
             // dfsph.rs:52-55: ground pushes through the weakly compressible solver's pressure only

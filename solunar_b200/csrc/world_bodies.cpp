@@ -192,11 +192,14 @@ int32_t World::carry_movers(float elapsed, float last) {
     size_t k = m_start.size();
     if (k && mdevice) {
         for (auto& known : coupled) known.moved = known.velocity * elapsed;
+        cudaStream_t on;
+        SLF_TRY(fork_bodies(on));
         timed("bodies_carry", 0.0, [&] {
             launch_carry_movers(params(), uint32_t(k), dmcur_start.p, dmcur_vel.p, elapsed, mlow, mspan, mvolume,
                                 dmlin.p, dmslot.p, dmtable.p, dmtable_tiles.p, dmmembers.p, dmnext_start.p,
-                                dmnext_vel.p, dmpos.p, stream);
+                                dmnext_vel.p, dmpos.p, on);
         });
+        SLF_TRY(mark_bodies(on));
         std::swap(dmcur_start, dmnext_start);
         std::swap(dmcur_vel, dmnext_vel);
         // the sorted velocities: dmcur_vel now; the grid: the dense table over the step's box
@@ -211,6 +214,7 @@ int32_t World::carry_movers(float elapsed, float last) {
         mgrid.start = dmtable.p;
         return SLF_OK;
     }
+    SLF_TRY(join_bodies());
     struct MK {
         Key3 cell;
         uint32_t owner;
@@ -304,13 +308,42 @@ int32_t World::mover_felt(float dt, const Params& p, int a, int nid) {
     if (coupled.empty() || m_pos.empty() || n == 0) return SLF_OK;
     const size_t bodies = coupled.size(), chunks = (n + 511) / 512;
     SLF_TRY(dfelt.ensure(2 * chunks * bodies, 0, stream));
+    cudaStream_t on;
+    SLF_TRY(fork_bodies(on));
     timed("bodies_felt", 0.0, [&] {
-        launch_mover_felt(p, d_consts, mover_dev(), pos[a].p, vel[a].p, rho[nid].p, press.p, scaled.p, dcentre.p,
-                          melapsed, uint32_t(bodies), dfelt.p, stream);
+        launch_mover_felt(p, consts(dt).mover_damping, mover_dev(), pos[a].p, vel[a].p, rho[nid].p, press.p, scaled.p, dcentre.p,
+                          melapsed, uint32_t(bodies), dfelt.p, on);
     });
     // folded on the device into the step's impulses, read once when the step ends
     timed("bodies_fold", 0.0,
-          [&] { launch_mover_fold(uint32_t(n), uint32_t(bodies), dfelt.p, dt, dimpulse.p, d_status, list_cap, stream); });
+          [&] { launch_mover_fold(uint32_t(n), uint32_t(bodies), dfelt.p, dt, dimpulse.p, d_spoiled, on); });
+    return mark_bodies(on);
+}
+
+int32_t World::fork_bodies(cudaStream_t& on) {
+    on = stream;
+    if (prof.on) return SLF_OK;
+    if (!mstream) {
+        SLF_CUDA(cudaStreamCreateWithFlags(&mstream, cudaStreamNonBlocking));
+        SLF_CUDA(cudaEventCreateWithFlags(&mfork, cudaEventDisableTiming));
+        SLF_CUDA(cudaEventCreateWithFlags(&mdone, cudaEventDisableTiming));
+    }
+    SLF_CUDA(cudaEventRecord(mfork, stream));
+    SLF_CUDA(cudaStreamWaitEvent(mstream, mfork, 0));
+    on = mstream;
+    mapart = true;
+    return SLF_OK;
+}
+
+int32_t World::mark_bodies(cudaStream_t on) {
+    if (on != stream) SLF_CUDA(cudaEventRecord(mdone, on));
+    return SLF_OK;
+}
+
+int32_t World::join_bodies() {
+    if (!mapart) return SLF_OK;
+    mapart = false;
+    SLF_CUDA(cudaStreamWaitEvent(stream, mdone, 0));
     return SLF_OK;
 }
 
@@ -501,6 +534,7 @@ int32_t World::step_with_bodies(float dt, const slf_body_pose* poses, uint64_t n
         SLF_CUDA(cudaMemsetAsync(dimpulse.p, 0, 2 * coupled.size() * sizeof(float4), stream));
     }
     int32_t st = step(dt, out);
+    SLF_TRY(join_bodies());  // (a step that failed in mid-substep)
     if (st == SLF_OK && !coupled.empty()) {  // the damping the bodies took, as the substeps folded it
         std::vector<float4> imp(2 * coupled.size());
         SLF_CUDA(cudaMemcpyAsync(imp.data(), dimpulse.p, imp.size() * sizeof(float4), cudaMemcpyDeviceToHost, stream));

@@ -54,6 +54,7 @@ int32_t World::init(const slf_settings& settings) {
     std::memset(h_status, 0, sizeof(Status));
     SLF_CUDA(cudaMallocHost(&h_posted, sizeof(uint32_t)));
     *h_posted = 0;
+    SLF_CUDA(cudaMalloc(&d_spoiled, sizeof(uint32_t)));
     unsigned int flags = 0;
     SLF_CUDA(cudaGetDeviceFlags(&flags));
     polls = (flags & cudaDeviceScheduleMask) != cudaDeviceScheduleBlockingSync;

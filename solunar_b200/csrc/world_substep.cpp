@@ -14,13 +14,14 @@ int32_t World::wcsph_substep(float dt, uint32_t& held) {
     if (!whole) {
         *h_consts = consts(dt);  // (the last launch that read them was waited for)
         SLF_TRY(enqueue_sort(a, sp, stream, SubstepBegin{d_status, d_consts, h_consts}));
+        SLF_TRY(join_bodies());
         PairLists fl = fluid_lists(), wl = wall_lists();
         timed("density", bytes_per_particle::density_wcsph,
               [&] { density_pass(p, a, fl, wl, rho[nid].p); });
         timed("wcsph_force_advance", bytes_per_particle::wcsph_force,
               [&] { force_pass(p, fl, wl, a, b, nid); });
     }
-    if (!whole) post_status();
+    if (!whole) post_status(d_spoiled);
     // what the bodies' points take is queued behind the status: it runs while the host reads that
     const int32_t felt = mover_felt(dt, p, a, nid);
     SLF_TRY(await_status());
