@@ -1007,11 +1007,9 @@ __global__ void __launch_bounds__(kGroupBlock, kGroupBlocks)
 #define SLF_LIST_UNROLL 4
 #endif
 constexpr int kListUnroll = SLF_LIST_UNROLL;
+constexpr int kViscousBlock = 128;
 // resident blocks per SM the list-walking kernels are compiled for (caps their registers); the
 // solver check runs best at four blocks (64 registers; 76 uncapped, three blocks)
-#ifndef SLF_PAIR_MIN_BLOCKS
-#define SLF_PAIR_MIN_BLOCKS 1
-#endif
 #ifndef SLF_RATE_MIN_BLOCKS
 #define SLF_RATE_MIN_BLOCKS 4
 #endif
@@ -1783,13 +1781,16 @@ __device__ __forceinline__ void viscous_particle(const Params& p, const StepCons
 }
 
 // viscous (step.rs:229-251) + gravity, velocity update (dfsph.rs:90-99); writes a new buffer
-// because neighbours read the old velocities.
-__global__ void __launch_bounds__(kBlock, SLF_PAIR_MIN_BLOCKS) k_viscous(Params p, const StepConsts* __restrict__ sc, PairLists fl,
+// because neighbours read the old velocities.  A row a thread in small blocks: some rows (walls,
+// approaching pairs) take much longer than others, and a short block makes room as soon as its own
+// are done.  Against the resident grid of 256-thread blocks, us: 57.6 -> 51.0 at 250k, 90.3 -> 83.1 at
+// 500k, 152 -> 150 at 1M (64 threads: the same; the push, whose rows are alike, 70 -> 73).
+__global__ void __launch_bounds__(kViscousBlock) k_viscous(Params p, const StepConsts* __restrict__ sc, PairLists fl,
                                                     PairLists wl, const float4* __restrict__ pos,
                                                     const float4* __restrict__ vel, const float* __restrict__ rho,
                                                     const float4* __restrict__ walls, float4* __restrict__ vel_out) {
-    for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < p.n; row += gridDim.x * blockDim.x)
-        viscous_particle(p, sc, fl, wl, fl.particle(row), row, pos, vel, rho, walls, vel_out);
+    const uint32_t row = blockIdx.x * uint32_t(kViscousBlock) + threadIdx.x;
+    if (row < p.n) viscous_particle(p, sc, fl, wl, fl.particle(row), row, pos, vel, rho, walls, vel_out);
 }
 
 __global__ void k_advance(Params p, const StepConsts* __restrict__ sc, const float4* __restrict__ pos_in,
@@ -2134,22 +2135,22 @@ static inline uint32_t blocks_for(uint32_t n) {
     return (n + kBlock - 1) / kBlock;
 }
 
-// The list passes' grids (the solves' check and push, the density pass, the viscosity): with
+// The list passes' grids (the solves' check and push, the density pass, the WCSPH force): with
 // SLF_SOLVER_RESIDENT, no more blocks than the SMs hold at once (each block then strides over
 // rows), so no launch ends on a partial wave and the check's residual sums fewer block partials.
 #ifndef SLF_SOLVER_RESIDENT
 #define SLF_SOLVER_RESIDENT 1
 #endif
-// resident blocks of k_rate<0>, k_rate<1>, k_push, k_density<0>, k_density<1>, k_viscous, k_wcsph_force on the
+// resident blocks of k_rate<0>, k_rate<1>, k_push, k_density<0>, k_density<1>, k_wcsph_force on the
 // device (prepare_solver_grids; 0: not known yet, the grid then covers every row)
-static std::atomic<uint32_t> g_resident[7] = {0, 0, 0, 0, 0, 0, 0};
+static std::atomic<uint32_t> g_resident[6] = {0, 0, 0, 0, 0, 0};
 
 // blocks of the density pass up to which it runs wide: two a SM
 static std::atomic<uint32_t> g_wide_blocks{0};
 
 void prepare_solver_grids() {
     if (!SLF_SOLVER_RESIDENT || g_resident[2].load()) return;
-    int dev = 0, sms = 0, per[7] = {0, 0, 0, 0, 0, 0, 0};
+    int dev = 0, sms = 0, per[6] = {0, 0, 0, 0, 0, 0};
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return;
@@ -2158,10 +2159,9 @@ void prepare_solver_grids() {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[2], k_push, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[3], k_density<0, true, false>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[4], k_density<1, false, false>, kBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[5], k_viscous, kBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[6], k_wcsph_force<true>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[5], k_wcsph_force<true>, kBlock, 0);
     g_wide_blocks.store(2u * uint32_t(std::max(sms, 0)));
-    for (int k = 0; k < 7; ++k) g_resident[k].store(uint32_t(std::max(per[k], 0) * std::max(sms, 0)));
+    for (int k = 0; k < 6; ++k) g_resident[k].store(uint32_t(std::max(per[k], 0) * std::max(sms, 0)));
 }
 
 static uint32_t solver_blocks(uint32_t n, int kernel) {
@@ -2317,7 +2317,7 @@ void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& 
                                                                          walls, pos_out, vel_out, st, vel_pre, M);
         }))
         return;
-    const uint32_t nb = solver_blocks(p.n, 6);
+    const uint32_t nb = solver_blocks(p.n, 5);
     if (T.regions || M.count || slope)
         k_wcsph_force<true><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, press, scaled, walls, pos_out, vel_out,
                                                   st, vel_pre, T, slope, M);
@@ -2431,7 +2431,10 @@ void launch_warm_kappa(const Params& p, const StepConsts* sc, float share, float
 
 void launch_viscous(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl, const float4* pos,
                     const float4* vel, const float* rho, const float4* walls, float4* vel_out, cudaStream_t s) {
-    if (p.n) k_viscous<<<solver_blocks(p.n, 5), kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, walls, vel_out);
+    if (!p.n) return;
+    note_launch();
+    k_viscous<<<(p.n + kViscousBlock - 1) / kViscousBlock, kViscousBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, walls,
+                                                                                  vel_out);
 }
 
 void launch_advance(const Params& p, const StepConsts* sc, const float4* pos_in, float4* pos_out, float4* vel,
