@@ -649,11 +649,13 @@ int32_t World::write_state(const float* p, const float* v, uint64_t k) {
     SLF_CUDA(cudaMemcpyAsync(stage.p, p, k * 12, cudaMemcpyHostToDevice, stream));
     SLF_CUDA(cudaMemcpyAsync(stage.p + 3 * k, v, k * 12, cudaMemcpyHostToDevice, stream));
     Params pr = params();
-    if (rel()) launch_to_relative(pr, uint32_t(k), stage.p, nullptr, pos[t].p, cell[t].p, stream, bad);
-    else launch_unpack3(uint32_t(k), stage.p, pos[t].p, stream, bad);
-    launch_unpack3(uint32_t(k), stage.p + 3 * k, vel[t].p, stream, bad);
-    if (rel()) launch_state_stats_rel(pr, cell[t].p, vel[t].p, d_status, stream);
-    else launch_state_stats(pr, pos[t].p, vel[t].p, d_status, stream);
+    if (rel()) {
+        launch_to_relative(pr, uint32_t(k), stage.p, nullptr, pos[t].p, cell[t].p, stream, bad);
+        launch_unpack3(uint32_t(k), stage.p + 3 * k, vel[t].p, stream, bad);
+        launch_state_stats_rel(pr, cell[t].p, vel[t].p, d_status, stream);
+    } else {
+        launch_unpack_state(pr, stage.p, pos[t].p, vel[t].p, d_status, stream);
+    }
     SLF_TRY(read_status());
     lists_valid = false;
     if (h_status->nonfinite) {
@@ -668,9 +670,12 @@ int32_t World::write_state(const float* p, const float* v, uint64_t k) {
 int32_t World::read_state(float* p, float* v, uint64_t k) {
     if (!k) return SLF_OK;
     SLF_TRY(stage.ensure(6 * k, 0, stream));
-    if (rel()) launch_from_relative(params(), uint32_t(k), pos[cpos].p, cell[cpos].p, stage.p, stream);
-    else launch_pack3(uint32_t(k), pos[cpos].p, stage.p, stream);
-    launch_pack3(uint32_t(k), vel[cpos].p, stage.p + 3 * k, stream);
+    if (rel()) {
+        launch_from_relative(params(), uint32_t(k), pos[cpos].p, cell[cpos].p, stage.p, stream);
+        launch_pack3(uint32_t(k), vel[cpos].p, stage.p + 3 * k, stream);
+    } else {
+        launch_pack_state(uint32_t(k), pos[cpos].p, vel[cpos].p, stage.p, stream);
+    }
     SLF_CUDA(cudaMemcpyAsync(p, stage.p, k * 12, cudaMemcpyDeviceToHost, stream));
     SLF_CUDA(cudaMemcpyAsync(v, stage.p + 3 * k, k * 12, cudaMemcpyDeviceToHost, stream));
     return sync();
