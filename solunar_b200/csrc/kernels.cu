@@ -2306,12 +2306,14 @@ void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float
     if (!p.n) return;
     const PairRecords rec{reinterpret_cast<float*>(pos), reinterpret_cast<float*>(vel)};
     const DensityIn in{{fg, wg}, {pos, walls}, {fl, wl}};
-    if (T.regions == 0 && slope == nullptr && with_lanes(group_lanes(p.n, p.radius / p.spacing), [&](auto lanes) {
+    // (terrain, whose sites every lane would take alike, and a DFSPH row's body points keep a thread a row)
+    const bool shared = T.regions == 0 && slope == nullptr && (p.solver == 0 || M.count == 0);
+    if (shared && with_lanes(group_lanes(p.n, p.radius / p.spacing), [&](auto lanes) {
             constexpr int L = decltype(lanes)::value;
             const uint32_t nb = group_blocks(p.n, L);
             auto launch = [&](auto flight) {
                 constexpr int F = decltype(flight)::value;
-                if (p.solver != 0)  // DFSPH takes no bodies
+                if (p.solver != 0)
                     k_density_group<1, false, L, F><<<nb, kGroupBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, M,
                                                                                scratch, rec);
                 else if (M.count)
@@ -2336,9 +2338,13 @@ void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float
     const uint32_t nb = solver_blocks(p.n, p.solver == 0 ? 3 : 4);
     auto launch = [&](auto wide) {
         constexpr bool W = decltype(wide)::value;
-        if (p.solver != 0)  // DFSPH takes neither terrain nor bodies
+        // (no DFSPH step takes terrain, but the densities of a DFSPH world on terrain have its ground)
+        const bool extra = T.regions || M.count || slope;
+        if (p.solver != 0 && extra)
+            k_density<1, true, W><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch, rec);
+        else if (p.solver != 0)
             k_density<1, false, W><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch, rec);
-        else if (T.regions || M.count || slope)
+        else if (extra)
             k_density<0, true, W><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch, rec);
         else
             k_density<0, false, W><<<nb, kBlock, 0, s>>>(p, in, rho, press, scaled, alpha, st, T, slope, M, scratch, rec);
