@@ -40,6 +40,9 @@ struct Params {
     float inv_rest_sq;     // 1 / rest_density^2
     float settles;         // |gravity| spacing: the speed under which water settles on a body (couple.rs:390)
     float slope_scale;     // scale * -20 (mod.rs:154)
+    float divided_above;   // pressures above this are divided: 0 (the quotient of a zero is known, and its division
+                           // would take the slow path), -1 where the divisor may underflow and 0 / 0 is NaN
+    float parted;          // viscosity(dt) x -0, the damping of a pair that parts: zero, or NaN of an infinite viscosity
     float one;             // 1, where the compiler cannot see it (sum2)
     uint32_t odd_radius;   // the radius is outside the range whose divisions take the reciprocal (div_radius2)
 };
@@ -50,6 +53,7 @@ struct StepConsts {
     float viscosity;       // viscosity(dt) (step.rs:254-259)
     float wall_viscosity;  // min(c r, 0.25 r^2 / dt) (step.rs:282-283)
     float dt_sq;           // dt * dt (dfsph.rs:246)
+    float divided_above;   // as Params', of what is divided by dt_sq
     float mover_damping;   // min(1 c r, 0.25 r r / dt), the body points' damping (step.rs:163-164)
 };
 

@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(kBlock, WIDE ? 2 : 4)
             float ratio = fminf(density / p.rest, 1.1f);
             float pressure = fmaxf(p.stiffness * (pow7(ratio) - 1.0f), 0.0f);
             press[i] = pressure;
-            const float over = pressure > 0.0f ? pressure / (density * density) : 0.0f;
+            const float over = pressure > p.divided_above ? pressure / (density * density) : 0.0f;
             scaled[i] = over;
             rec.pos_w[4 * size_t(i) + 3] = over;
         } else {
@@ -978,7 +978,7 @@ __global__ void __launch_bounds__(kGroupBlock, kGroupBlocks)
                 float ratio = fminf(density / p.rest, 1.1f);
                 float pressure = fmaxf(p.stiffness * (pow7(ratio) - 1.0f), 0.0f);
                 press[i] = pressure;
-                const float over = pressure > 0.0f ? pressure / (density * density) : 0.0f;
+                const float over = pressure > p.divided_above ? pressure / (density * density) : 0.0f;
                 scaled[i] = over;
                 rec.pos_w[4 * size_t(i) + 3] = over;
             } else {
@@ -1297,7 +1297,7 @@ __global__ void __launch_bounds__(kFeltBlock) k_mover_felt(const __grid_constant
         a = pos[i];
         v = vel[i];
         density = rho[i];
-        mirrored = scaled[i] + (press[i] > 0.0f ? press[i] / p.rest_sq : 0.0f);
+        mirrored = scaled[i] + (press[i] > p.divided_above ? press[i] / p.rest_sq : 0.0f);
     }
     // f(k, j, point, gradient * mass, damp) for the particle's k-th pair above the settling speed
     auto pairs = [&](auto&& f) {
@@ -1383,7 +1383,7 @@ __global__ void k_cells_wet(GridDev g, int3 lo, int3 hi, uint32_t* wet) {
 
 // k_wcsph_force by L lanes a row.
 template <bool BODIES, int L>
-__global__ void __launch_bounds__(kGroupBlock)
+__global__ void __launch_bounds__(kGroupBlock, BODIES ? 9 : kGroupBlocks)
     k_wcsph_force_group(Params p, const StepConsts* __restrict__ sc, PairLists fl, PairLists wl,
                         const float4* __restrict__ pos, const float4* __restrict__ vel, const float* __restrict__ rho,
                         const float* __restrict__ press, const float* __restrict__ scaled,
@@ -1445,14 +1445,14 @@ __global__ void __launch_bounds__(kGroupBlock)
                 float squared = dot3(rx, ry, rz, rx, ry, rz);
                 float gx = rx * g, gy = ry * g, gz = rz * g;
                 float toward = dot3(v.x - w[u].x, v.y - w[u].y, v.z - w[u].z, rx, ry, rz);
-                float damp = 0.0f;  // a pair that parts is not damped: no division of a zero
+                float damp = p.parted;  // a pair that parts: no division of a zero
                 if (toward < 0.0f) damp = -visc * toward / (squared + p.soften) * 2.0f / (density + w[u].w);
                 float s = p.mass * (own + q[u].w + damp);
                 const bool pair = squared > 0.0f;
                 t[u][0] = pair ? gx * s : 0.0f, t[u][1] = pair ? gy * s : 0.0f, t[u][2] = pair ? gz * s : 0.0f;
             }
         });
-        const float mirrored = own + (press[i] > 0.0f ? press[i] / p.rest_sq : 0.0f);
+        const float mirrored = own + (press[i] > p.divided_above ? press[i] / p.rest_sq : 0.0f);
         // the walls' pressure, then wall_viscous's two walks (its normal, then its damping)
         const uint32_t walled = walk(wl, std::true_type{}, push, [&](const uint2(&en)[2], float(&t)[2][3]) {
 #pragma unroll
@@ -1575,14 +1575,14 @@ __global__ void __launch_bounds__(kBlock, 3) k_wcsph_force(Params p, const StepC
             // neighbour's p / rho^2 and w.w its density (the density pass put them there)
             float gx = rx * g, gy = ry * g, gz = rz * g;
             float toward = dot3(v.x - w.x, v.y - w.y, v.z - w.z, rx, ry, rz);
-            float damp = 0.0f;  // a pair that parts is not damped: no division of a zero
+            float damp = p.parted;  // a pair that parts: no division of a zero
             if (toward < 0.0f) damp = -visc * toward / (squared + p.soften) * 2.0f / (density + w.w);
             float s = p.mass * (own + q.w + damp);
             px = px - gx * s;
             py = py - gy * s;
             pz = pz - gz * s;
         });
-        float mirrored = own + (press[i] > 0.0f ? press[i] / p.rest_sq : 0.0f);
+        float mirrored = own + (press[i] > p.divided_above ? press[i] / p.rest_sq : 0.0f);
         each_listed(wl, row, walls, [&](uint32_t, float g, float4 q) {
             float rx = a.x - q.x, ry = a.y - q.y, rz = a.z - q.z;
             float s = p.mass * mirrored;
@@ -1661,7 +1661,7 @@ __device__ __forceinline__ void rate_particle(const Params& p, const StepConsts*
     if (WHICH == 1) {
         float over = fmaxf(rho[i] + dt * rate - p.rest, 0.0f);
         // (a quotient of zero is zero, and its division would take the slow path)
-        target = over > 0.0f ? over / sc->dt_sq : 0.0f;
+        target = over > sc->divided_above ? over / sc->dt_sq : 0.0f;
         error = over > 0.0f ? over / p.rest : 0.0f;
     } else {
         float r = fl.count[row] + wl.count[row] < 20u ? 0.0f : fmaxf(rate, 0.0f);

@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kBlock, 4)
             float r2 = ratio * ratio, r4 = r2 * r2;
             float pressure = fmaxf(p.stiffness * (ratio * r2 * r4 - 1.0f), 0.0f);
             press[i] = pressure;
-            const float over = pressure > 0.0f ? pressure / (density * density) : 0.0f;
+            const float over = pressure > p.divided_above ? pressure / (density * density) : 0.0f;
             scaled[i] = over;
             rec.pos_w[4 * size_t(i) + 3] = over;
         } else {
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kBlock) k_wcsph_force_fast(Params p, const Ste
             float toward = fmaf(v.x - w.x, r.x, fmaf(v.y - w.y, r.y, (v.z - w.z) * r.z));
             // the neighbour's density and p / rho^2 ride in the spare lanes (PairRecords); a pair that
             // parts is not damped, and divides no zero (the division's slow path)
-            float damp = 0.0f;
+            float damp = p.parted;
             if (toward < 0.0f) damp = visc2 * toward / ((squared + p.soften) * (density + w.w));
             float s = g * p.mass * (own + q.w + damp);
             px = fmaf(-r.x, s, px);
@@ -604,7 +604,7 @@ __device__ __forceinline__ void rate_particle_fast(const Params& p, const StepCo
     float target, error;
     if (WHICH == 1) {
         float over = fmaxf(fmaf(dt, rate, rho[i]) - p.rest, 0.0f);
-        target = over > 0.0f ? over / sc->dt_sq : 0.0f;  // (no division of a zero: its slow path)
+        target = over > sc->divided_above ? over / sc->dt_sq : 0.0f;  // (no division of a zero: its slow path)
         error = over * p.inv_rest;
     } else {
         float r = fl.count[row] + wl.count[row] < 20u ? 0.0f : fmaxf(rate, 0.0f);

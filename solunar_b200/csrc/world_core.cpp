@@ -222,6 +222,8 @@ Params World::params() const {
     p.inv_rest = 1.0f / s.rest_density;
     p.inv_rest_sq = 1.0f / (s.rest_density * s.rest_density);
     p.slope_scale = scale * -20.0f;
+    // (a particle's own share keeps its density within a factor of support^3 of the rest density)
+    p.divided_above = p.rest_sq > 1e-20f ? 0.0f : -1.0f;
     p.one = 1.0f;
     p.odd_radius = radius >= 1.220703125e-4f && radius <= 1024.0f ? 0u : 1u;
     p.settles = std::sqrt(s.gravity[0] * s.gravity[0] + s.gravity[1] * s.gravity[1] + s.gravity[2] * s.gravity[2]) *
@@ -236,6 +238,7 @@ StepConsts World::consts(float dt) const {
     float stable = radius * radius / dt;
     c.wall_viscosity = rmin(1.0f * s.sound_speed * radius, 0.25f * stable);
     c.dt_sq = dt * dt;
+    c.divided_above = c.dt_sq > 0.0f ? 0.0f : -1.0f;
     c.mover_damping = rmin(1.0f * s.sound_speed * radius, 0.25f * radius * radius / dt);
     return c;
 }

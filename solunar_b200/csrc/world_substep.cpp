@@ -5,6 +5,7 @@ namespace slf {
 
 int32_t World::wcsph_substep(float dt, uint32_t& held) {
     Params p = params();
+    p.parted = -consts(dt).viscosity * 0.0f;
     int a = (cpos + 1) % 3, b = (cpos + 2) % 3;
     int nid = 1 - cid;
     bool whole = whole_substeps();
