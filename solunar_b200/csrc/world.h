@@ -403,8 +403,9 @@ struct World {
     // The coupled bodies' own stream: what their points take of a substep (k_mover_felt, k_mover_fold)
     // and where the next substep carries them (k_mover_carry) run beside the next substep's sort, which
     // leaves most of the SMs idle.  fork_bodies starts behind all queued on the world's stream,
-    // joined_bodies marks its end, and the world's stream waits for that before the next pass that meets
-    // the points and before anything outside the substeps (22 substeps of 75k particles around a box 3.87
+    // mark_bodies marks its end, and the world's stream waits for that (join_bodies) before the next pass
+    // that meets the points, before an attempt is made again, and before anything outside the substeps,
+    // however they end (22 substeps of 75k particles around a box 3.87
     // -> 3.50 ms, of 9k 2.09 -> 1.88).  A profiled world keeps one stream.
     cudaStream_t mstream = nullptr;
     cudaEvent_t mfork = nullptr, mdone = nullptr;
@@ -565,6 +566,7 @@ struct World {
 
     ~World() {
         if (stream) {
+            join_bodies();  // the buffers go behind the bodies' stream too
             for (auto* b : {&pos[0], &pos[1], &pos[2], &vel[0], &vel[1], &vel[2]}) b->release(stream);
             for (auto* b : {&ids[0], &ids[1], &lin, &cslot, &members, &count, &tiles, &keep, &dwstart, &dwnear, &fcnt, &wcnt, &dscratch,
                             &worder, &etaken, &etiles})

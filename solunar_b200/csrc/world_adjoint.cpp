@@ -589,6 +589,11 @@ int32_t World::step_untaped(float dt, slf_report* out) {
             uint32_t substeps = uint32_t(rmin(wanted, cap));
             r.capped = wanted > cap;
             float small = dt / float(substeps);
+            // a step that fails in mid-substep leaves nothing running on the bodies' stream either
+            struct Joined {
+                World& w;
+                ~Joined() { w.join_bodies(); }
+            } joined{*this};
             for (uint32_t i = 0; i < substeps; ++i) {
                 uint32_t held = 0;
                 SLF_TRY(tape_substep(small));

@@ -534,7 +534,6 @@ int32_t World::step_with_bodies(float dt, const slf_body_pose* poses, uint64_t n
         SLF_CUDA(cudaMemsetAsync(dimpulse.p, 0, 2 * coupled.size() * sizeof(float4), stream));
     }
     int32_t st = step(dt, out);
-    SLF_TRY(join_bodies());  // (a step that failed in mid-substep)
     if (st == SLF_OK && !coupled.empty()) {  // the damping the bodies took, as the substeps folded it
         std::vector<float4> imp(2 * coupled.size());
         SLF_CUDA(cudaMemcpyAsync(imp.data(), dimpulse.p, imp.size() * sizeof(float4), cudaMemcpyDeviceToHost, stream));

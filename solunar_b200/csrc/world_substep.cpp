@@ -25,10 +25,15 @@ int32_t World::wcsph_substep(float dt, uint32_t& held) {
     if (!whole) post_status(d_spoiled);
     // what the bodies' points take is queued behind the status: it runs while the host reads that
     const int32_t felt = mover_felt(dt, p, a, nid);
-    SLF_TRY(await_status());
-    SLF_TRY(lists_fit());
-    SLF_TRY(check_state());
-    SLF_TRY(felt);
+    int32_t st = await_status();
+    if (st == SLF_OK) st = lists_fit();
+    if (st == SLF_OK) st = check_state();
+    if (st == SLF_OK) st = felt;
+    if (st != SLF_OK) {
+        // the bodies' stream may still read this attempt's slots, which the next attempt's sort writes
+        SLF_TRY(join_bodies());
+        return st;
+    }
     held = h_status->held;
     cpos = b;
     cid = nid;
