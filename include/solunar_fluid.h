@@ -350,7 +350,7 @@ int32_t slf_step_backward(slf_world* world, const float* dpositions, const float
 /* No counterpart in the reference: the cell sort of slf_update_neighbors for callers that
  * cannot allocate device memory (an engine that hands out all GPU memory from its own pool, a
  * plugin that only receives buffers from its host).  It allocates nothing: its scratch is one
- * fixed array in device memory, about 5.3 MB, that every GPU which loads this library holds
+ * fixed array in device memory, about 6.3 MB, that every GPU which loads this library holds
  * until the process exits.
  *
  * positions: n packed xyz float triples and ids: n ids, both in device memory; radius: the
@@ -367,7 +367,10 @@ int32_t slf_step_backward(slf_world* world, const float* dpositions, const float
  * The first call on a device looks up the scratch array's address there, so make that first
  * call before any stream capture.  All calls share the one array and it keeps the last call's
  * contents (the call clears what must start at zero); calls whose work overlaps on the GPU
- * race on it. */
+ * race on it.
+ * The sort is one launch whose blocks wait for one another, on as many SMs as the device or the
+ * stream's share of it holds blocks on (any number; each call tries what fits).  A wait that runs
+ * out fails the call with SLF_ERR_TIMEOUT.  After any failure order may be partly written. */
 int32_t slf_sort_by_cell_noalloc(const float* positions, const uint32_t* ids, uint64_t n, float radius,
                                  uint32_t* order, void* stream);
 
@@ -421,6 +424,10 @@ int32_t slf_debug_skip_job(slf_world* world, int64_t job);
  * multiple of 8, at least 8), so that the next substep's lists outgrow it and the substep is run
  * again with room for its longest list, from the committed state.  Invalidates the lists. */
 int32_t slf_debug_list_room(slf_world* world, uint32_t room);
+
+/* slf_sort_by_cell_noalloc as where at most `blocks` (0: no limit) of its blocks run at once. */
+int32_t slf_debug_sort_by_cell_noalloc(const float* positions, const uint32_t* ids, uint64_t n, float radius,
+                                       uint32_t* order, void* stream, uint32_t blocks);
 
 #ifdef __cplusplus
 }

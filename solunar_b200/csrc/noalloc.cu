@@ -13,7 +13,6 @@
 // the array and it keeps what the last call left in it; the kernels clear what must start at
 // zero.  Two calls whose work overlaps on the GPU (different streams, or different host threads)
 // race on it.
-#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstdint>
@@ -25,20 +24,21 @@
 #include "../../include/solunar_fluid.h"
 #include "fluid_device.cuh"
 #include "launch.h"
+#include "noalloc_grid.h"
 
 namespace slf {
 
 constexpr uint32_t kNoAllocMaxParticles = 1u << 18;  // 262,144 particles
 constexpr uint32_t kNoAllocMaxCells = 1u << 20;      // 1,048,576 cells in the bounding box
 constexpr uint32_t kNoAllocHeader = 64;               // error flag, arrivals (u32 words)
-constexpr uint32_t kNoAllocBlocks = 256;  // most blocks of the sort's grid
 
 // word offsets inside the scratch array
 constexpr size_t kOffBounds = kNoAllocHeader;                  // each block's box (6 words)
 constexpr size_t kOffSums = kOffBounds + 6 * kNoAllocBlocks;   // each block's share of the counts
 constexpr size_t kOffMembers = kOffSums + kNoAllocBlocks;
-constexpr size_t kOffCount = kOffMembers + kNoAllocMaxParticles;
-constexpr size_t kNoAllocWords = kOffCount + kNoAllocMaxCells + 1;  // about 5.3 MB
+constexpr size_t kOffSlots = kOffMembers + kNoAllocMaxParticles;  // where registers do not hold them
+constexpr size_t kOffCount = kOffSlots + kNoAllocMaxParticles;
+constexpr size_t kNoAllocWords = kOffCount + kNoAllocMaxCells + 1;  // about 6.3 MB
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocWords];
 
@@ -72,37 +72,48 @@ __device__ __forceinline__ bool na_meet(uint32_t* hdr, uint32_t round) {
     return met;
 }
 
-constexpr int kNoAllocThreads = 512;
-constexpr int kNoAllocItems = 4;  // particles a thread keeps in registers from pass to pass
+// A particle on its way through the passes.
+struct NaItem {
+    int3 cell;
+    uint32_t id, lin, slot, first;
+};
 
 // The whole sort in one launch: the box of the cells, a count a cell, their scan, ids by cell, ranks.
 // The grid meets between the passes, each pass touches only the box's cells, and a thread's particles
-// (their cells, slots and ids) stay in its registers.  As eight launches over a table of every cell the
+// (their cells, slots and ids) stay in its registers, or, where so few blocks run at once that they do
+// not fit there (HELD false), are read again in each pass.  As eight launches over a table of every cell the
 // scratch holds, before: 95 -> 60 us a call at 201,544 particles (the call ends with a host wait).
+template <bool HELD>
 __global__ void __launch_bounds__(kNoAllocThreads) k_na_sort(const float* __restrict__ pos,
                                                              const uint32_t* __restrict__ ids, uint32_t n, float radius,
                                                              uint32_t* scratch, uint32_t* __restrict__ order) {
     uint32_t* const hdr = scratch;
     uint32_t* const count = scratch + kOffCount;
     uint32_t* const members = scratch + kOffMembers;
+    uint32_t* const slots = scratch + kOffSlots;
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, width = gridDim.x * kNoAllocThreads;
     __shared__ int part[6][kNoAllocThreads / 32];
     __shared__ uint32_t sums[kNoAllocThreads / 32];
-    int3 cell[kNoAllocItems];
-    uint32_t id[kNoAllocItems], lin[kNoAllocItems], slot[kNoAllocItems];
+    NaItem held[HELD ? kNoAllocItems : 1];
+    // f(item, index) for each of the thread's particles
+    auto each = [&](auto&& f) {
+        const uint32_t i0 = blockIdx.x * kNoAllocThreads + t;
+        if constexpr (HELD) {
+#pragma unroll
+            for (uint32_t k = 0; k < kNoAllocItems; ++k)
+                if (i0 + k * width < n) f(held[k], i0 + k * width);
+        } else {
+            for (uint32_t i = i0; i < n; i += width) f(held[0], i);
+        }
+    };
     // (a thread without a particle takes part with an empty box)
     int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
-#pragma unroll
-    for (int k = 0; k < kNoAllocItems; ++k) {
-        const uint32_t i = blockIdx.x * kNoAllocThreads + t + k * width;
-        cell[k] = make_int3(0, 0, 0);
-        id[k] = lin[k] = slot[k] = 0u;
-        if (i >= n) continue;
-        cell[k] = na_cell(pos, i, radius);
-        id[k] = ids[i];
-        lo[0] = min(lo[0], cell[k].x), lo[1] = min(lo[1], cell[k].y), lo[2] = min(lo[2], cell[k].z);
-        hi[0] = max(hi[0], cell[k].x), hi[1] = max(hi[1], cell[k].y), hi[2] = max(hi[2], cell[k].z);
-    }
+    each([&](NaItem& q, uint32_t i) {
+        q.cell = na_cell(pos, i, radius);
+        q.id = ids[i];
+        lo[0] = min(lo[0], q.cell.x), lo[1] = min(lo[1], q.cell.y), lo[2] = min(lo[2], q.cell.z);
+        hi[0] = max(hi[0], q.cell.x), hi[1] = max(hi[1], q.cell.y), hi[2] = max(hi[2], q.cell.z);
+    });
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
@@ -139,21 +150,24 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_na_sort(const float* __rest
     const uint32_t volume = uint32_t(sx * sy * sz);
     for (uint32_t c = blockIdx.x * kNoAllocThreads + t; c < volume; c += width) count[c] = 0u;
     if (!na_meet(hdr, 2)) return;
-#pragma unroll
-    for (int k = 0; k < kNoAllocItems; ++k) {
-        if (blockIdx.x * kNoAllocThreads + t + k * width >= n) continue;
-        // offsets in 64 bits (a cell minus the box's low corner can pass the i32 range), and every
-        // particle checked against the box before it touches the count table: a cell outside it
-        // (another call's work on the scratch) fails the call instead of writing outside the array
-        const long long x = (long long)cell[k].x - box[0], y = (long long)cell[k].y - box[1],
-                        z = (long long)cell[k].z - box[2];
-        lin[k] = uint32_t((x * sy + y) * sz + z);
+    // the particle's cell in the table: offsets in 64 bits (a cell minus the box's low corner can pass the
+    // i32 range), and every particle checked against the box before it touches the count table: a cell
+    // outside it (another call's work on the scratch) fails the call instead of writing outside the array
+    auto place = [&](NaItem& q, uint32_t i) {
+        if (!HELD) q.cell = na_cell(pos, i, radius);
+        const long long x = (long long)q.cell.x - box[0], y = (long long)q.cell.y - box[1],
+                        z = (long long)q.cell.z - box[2];
+        q.lin = uint32_t((x * sy + y) * sz + z);
         if (x < 0 || x >= sx || y < 0 || y >= sy || z < 0 || z >= sz) {
             atomicMax(&hdr[kHdrError], uint32_t(kErrorBox));
-            lin[k] = 0u;
+            q.lin = 0u;
         }
-        slot[k] = atomicAdd(&count[lin[k]], 1u);
-    }
+    };
+    each([&](NaItem& q, uint32_t i) {
+        place(q, i);
+        q.slot = atomicAdd(&count[q.lin], 1u);
+        if (!HELD) slots[i] = q.slot;
+    });
     if (!na_meet(hdr, 3)) return;
     // exclusive scan: a run of cells a block, a run of those a thread (whole warps read side by side)
     const uint32_t per = ((volume + gridDim.x - 1) / gridDim.x + 31u) & ~31u;
@@ -194,31 +208,33 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_na_sort(const float* __rest
     }
     if (blockIdx.x == 0 && t == 0) count[volume] = n;
     if (!na_meet(hdr, 5)) return;
-    uint32_t first[kNoAllocItems];
-#pragma unroll
-    for (int k = 0; k < kNoAllocItems; ++k) {
-        first[k] = 0u;
-        if (blockIdx.x * kNoAllocThreads + t + k * width >= n) continue;
-        first[k] = __ldcg(&count[lin[k]]);
-        if (first[k] < n && slot[k] < n - first[k]) members[first[k] + slot[k]] = id[k];
-    }
+    auto settle = [&](NaItem& q, uint32_t i) {
+        if (!HELD) {
+            place(q, i);
+            q.id = ids[i];
+            q.slot = slots[i];  // (this thread wrote it)
+        }
+        q.first = __ldcg(&count[q.lin]);
+    };
+    each([&](NaItem& q, uint32_t i) {
+        settle(q, i);
+        if (q.first < n && q.slot < n - q.first) members[q.first + q.slot] = q.id;
+    });
     if (!na_meet(hdr, 6)) return;
     // order[cell start + rank of the id in its cell] = i: the (cell, id) order of mod.rs:541-550.
     // A cell of k particles costs k comparisons a particle (k^2 for the cell).  Equal ids (a world's
     // ids are distinct; a caller's arrays need not be) are ranked by the slot each took in its cell,
     // so order is always a permutation, with repeated ids in no particular order among themselves.
-#pragma unroll
-    for (int k = 0; k < kNoAllocItems; ++k) {
-        const uint32_t i = blockIdx.x * kNoAllocThreads + t + k * width;
-        if (i >= n) continue;
-        const uint32_t e = min(__ldcg(&count[lin[k] + 1]), n), own = first[k] + slot[k];
+    each([&](NaItem& q, uint32_t i) {
+        if (!HELD) settle(q, i);
+        const uint32_t e = min(__ldcg(&count[q.lin + 1]), n), own = q.first + q.slot;
         uint32_t rank = 0;
-        for (uint32_t q = first[k]; q < e; ++q) {
-            const uint32_t m = __ldcg(&members[q]);
-            rank += (m < id[k] || (m == id[k] && q < own)) ? 1u : 0u;
+        for (uint32_t k = q.first; k < e; ++k) {
+            const uint32_t m = __ldcg(&members[k]);
+            rank += (m < q.id || (m == q.id && k < own)) ? 1u : 0u;
         }
-        if (first[k] < n && rank < n - first[k]) order[first[k] + rank] = i;
-    }
+        if (q.first < n && rank < n - q.first) order[q.first + rank] = i;
+    });
 }
 
 namespace {
@@ -251,13 +267,9 @@ int32_t scratch_on_current_device(uint32_t** out) {
     return SLF_OK;
 }
 
-}  // namespace
-
-}  // namespace slf
-
-extern "C" int32_t slf_sort_by_cell_noalloc(const float* positions, const uint32_t* ids, uint64_t n, float radius,
-                                            uint32_t* order, void* stream) {
-    using namespace slf;
+// The sort on a grid of at most `room` blocks (0: a block a SM).
+int32_t sort_noalloc(const float* positions, const uint32_t* ids, uint64_t n, float radius, uint32_t* order,
+                     cudaStream_t s, uint32_t room) {
     if (n == 0) return SLF_OK;
     if (!positions || !ids || !order) return na_fail(SLF_ERR_INVALID_ARGUMENT, "null device pointer");
     if (!(radius > 0.0f) || !std::isfinite(radius)) return na_fail(SLF_ERR_INVALID_ARGUMENT, "radius must be positive");
@@ -265,22 +277,27 @@ extern "C" int32_t slf_sort_by_cell_noalloc(const float* positions, const uint32
     uint32_t* scratch = nullptr;
     int32_t st = scratch_on_current_device(&scratch);
     if (st != SLF_OK) return st;
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
     uint32_t m = uint32_t(n);
-    // a block a SM at most, and no more than there are particles for: they all run at once
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "cudaDeviceGetAttribute", e);
-    uint32_t blocks = std::min<uint32_t>(uint32_t(sms), kNoAllocBlocks);
-    if (uint64_t(blocks) * kNoAllocThreads * kNoAllocItems < kNoAllocMaxParticles)
-        return na_fail(SLF_ERR_CUDA, "the device has too few SMs for the cell sort");
-    blocks = std::min(blocks, (m + 255u) / 256u);
-    blocks = std::max(blocks, (m + kNoAllocThreads * kNoAllocItems - 1u) / (kNoAllocThreads * kNoAllocItems));
+    const uint32_t all = uint32_t(sms > 0 ? sms : 1);
+    room = room && room < all ? room : all;
     e = cudaMemsetAsync(scratch, 0, 2 * 4, s);
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "clearing the header", e);
     void* args[] = {&positions, &ids, &m, &radius, &scratch, &order};
-    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_na_sort), dim3(blocks), dim3(kNoAllocThreads), args, 0, s);
+    for (;; room /= 2) {
+        // (a share of the SMs, of a stream or a process, holds fewer blocks than the device: half as many
+        // are tried until they run at once, as one always does)
+        const NoAllocGrid grid = noalloc_grid(m, room);
+        const void* kernel = grid.held ? reinterpret_cast<const void*>(k_na_sort<true>)
+                                       : reinterpret_cast<const void*>(k_na_sort<false>);
+        e = cudaLaunchCooperativeKernel(kernel, dim3(grid.blocks), dim3(kNoAllocThreads), args, 0, s);
+        if (e != cudaErrorCooperativeLaunchTooLarge || grid.blocks == 1) break;
+        cudaGetLastError();
+        room = grid.blocks;
+    }
     note_launch();
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "launching the cell sort", e);
     e = cudaMemcpyAsync(&h_noalloc_error, scratch + kHdrError, 4, cudaMemcpyDeviceToHost, s);
@@ -289,4 +306,18 @@ extern "C" int32_t slf_sort_by_cell_noalloc(const float* positions, const uint32
     if (h_noalloc_error == kErrorWait) return na_fail(SLF_ERR_TIMEOUT, "the cell sort's blocks did not meet");
     if (h_noalloc_error) return na_fail(SLF_ERR_OUT_OF_RANGE, "particles spread over more cells than the scratch holds");
     return SLF_OK;
+}
+
+}  // namespace
+
+}  // namespace slf
+
+extern "C" int32_t slf_sort_by_cell_noalloc(const float* positions, const uint32_t* ids, uint64_t n, float radius,
+                                            uint32_t* order, void* stream) {
+    return slf::sort_noalloc(positions, ids, n, radius, order, static_cast<cudaStream_t>(stream), 0);
+}
+
+extern "C" int32_t slf_debug_sort_by_cell_noalloc(const float* positions, const uint32_t* ids, uint64_t n, float radius,
+                                                  uint32_t* order, void* stream, uint32_t blocks) {
+    return slf::sort_noalloc(positions, ids, n, radius, order, static_cast<cudaStream_t>(stream), blocks);
 }

@@ -92,6 +92,7 @@ def load_library():
         "slf_profile_reset": [vp],
         "slf_kernel_launches": [u64p],
         "slf_sort_by_cell_noalloc": [vp, vp, ctypes.c_uint64, ctypes.c_float, vp, vp],
+        "slf_debug_sort_by_cell_noalloc": [vp, vp, ctypes.c_uint64, ctypes.c_float, vp, vp, ctypes.c_uint32],
         "slf_tape_begin": [vp, ctypes.c_uint32],
         "slf_tape_end": [vp],
         "slf_step_backward": [vp, fp, fp, ctypes.c_uint64, fp, fp, ctypes.POINTER(CParamGrads)],
