@@ -367,7 +367,7 @@ int32_t slf_step_backward(slf_world* world, const float* dpositions, const float
  * The first call on a device looks up the scratch array's address there, so make that first
  * call before any stream capture.  All calls share the one array and it keeps the last call's
  * contents (the call clears what must start at zero); calls whose work overlaps on the GPU
- * race on it.
+ * race on it: their orders are wrong or they fail, but no access leaves the arrays.
  * The sort is one launch whose blocks wait for one another, on as many SMs as the device or the
  * stream's share of it holds blocks on (any number; each call tries what fits).  A wait that runs
  * out fails the call with SLF_ERR_TIMEOUT.  After any failure order may be partly written. */

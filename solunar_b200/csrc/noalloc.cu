@@ -12,7 +12,9 @@
 // kNoAllocMaxCells cells; larger calls are refused with SLF_ERR_OUT_OF_RANGE.  All calls share
 // the array and it keeps what the last call left in it; the kernels clear what must start at
 // zero.  Two calls whose work overlaps on the GPU (different streams, or different host threads)
-// race on it.
+// race on its tables: their orders are wrong, but each has a header of its own (kNoAllocHeaders
+// calls in turn), so neither waits for the other's blocks, and no access leaves the array.
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdint>
@@ -30,11 +32,12 @@ namespace slf {
 
 constexpr uint32_t kNoAllocMaxParticles = 1u << 18;  // 262,144 particles
 constexpr uint32_t kNoAllocMaxCells = 1u << 20;      // 1,048,576 cells in the bounding box
-constexpr uint32_t kNoAllocHeader = 64;               // error flag, arrivals (u32 words)
+constexpr uint32_t kNoAllocHeaders = 32;             // headers, taken in turn by the calls
+constexpr uint32_t kNoAllocHeader = 2;               // error flag, arrivals (u32 words)
 
 // word offsets inside the scratch array
-constexpr size_t kOffBounds = kNoAllocHeader;                  // each block's box (6 words)
-constexpr size_t kOffSums = kOffBounds + 6 * kNoAllocBlocks;   // each block's share of the counts
+constexpr size_t kOffBounds = size_t(kNoAllocHeaders) * kNoAllocHeader;  // each block's box (6 words)
+constexpr size_t kOffSums = kOffBounds + 6 * kNoAllocBlocks;             // each block's share of the counts
 constexpr size_t kOffMembers = kOffSums + kNoAllocBlocks;
 constexpr size_t kOffSlots = kOffMembers + kNoAllocMaxParticles;  // where registers do not hold them
 constexpr size_t kOffCount = kOffSlots + kNoAllocMaxParticles;
@@ -53,7 +56,8 @@ __device__ __forceinline__ int3 na_cell(const float* pos, uint32_t i, float radi
 }
 
 // All blocks of the grid (a cooperative launch: they are on the GPU together) meet; `round` counts the
-// meetings.  A wait that runs out of patience reports itself and lets every block leave.
+// meetings.  A wait ends where a block has left with an error, and one that runs out of patience
+// reports itself and lets every block leave.
 __device__ __forceinline__ bool na_meet(uint32_t* hdr, uint32_t round) {
     __shared__ bool met;
     __syncthreads();
@@ -61,10 +65,13 @@ __device__ __forceinline__ bool na_meet(uint32_t* hdr, uint32_t round) {
         __threadfence();
         atomicAdd(&hdr[kHdrArrived], 1u);
         const uint32_t all = round * gridDim.x;
-        bool there = false;
-        for (uint32_t spin = 0; spin < (1u << 22) && !there; ++spin)
-            there = *reinterpret_cast<volatile uint32_t*>(&hdr[kHdrArrived]) >= all;
-        if (!there) atomicMax(&hdr[kHdrError], uint32_t(kErrorWait));
+        const volatile uint32_t* const seen = hdr;
+        bool there = false, left = false;
+        for (uint32_t spin = 0; spin < (1u << 22) && !there && !left; ++spin) {
+            there = seen[kHdrArrived] >= all;
+            if ((spin & 63u) == 63u) left = seen[kHdrError] != 0u;
+        }
+        if (!there && !left) atomicMax(&hdr[kHdrError], uint32_t(kErrorWait));
         __threadfence();
         met = there;
     }
@@ -86,8 +93,8 @@ struct NaItem {
 template <bool HELD>
 __global__ void __launch_bounds__(kNoAllocThreads) k_na_sort(const float* __restrict__ pos,
                                                              const uint32_t* __restrict__ ids, uint32_t n, float radius,
-                                                             uint32_t* scratch, uint32_t* __restrict__ order) {
-    uint32_t* const hdr = scratch;
+                                                             uint32_t* scratch, uint32_t* hdr,
+                                                             uint32_t* __restrict__ order) {
     uint32_t* const count = scratch + kOffCount;
     uint32_t* const members = scratch + kOffMembers;
     uint32_t* const slots = scratch + kOffSlots;
@@ -144,7 +151,7 @@ __global__ void __launch_bounds__(kNoAllocThreads) k_na_sort(const float* __rest
     // each side is at most 2^32 cells: bounding them first keeps the products inside 64 bits
     const long long cap = (long long)kNoAllocMaxCells;
     if (sx <= 0 || sy <= 0 || sz <= 0 || sx > cap || sy > cap || sz > cap || sx * sy > cap || sx * sy * sz > cap) {
-        if (blockIdx.x == 0 && t == 0) atomicMax(&hdr[kHdrError], uint32_t(kErrorBox));
+        if (t == 0) atomicMax(&hdr[kHdrError], uint32_t(kErrorBox));
         return;  // every block alike
     }
     const uint32_t volume = uint32_t(sx * sy * sz);
@@ -242,6 +249,7 @@ namespace {
 std::mutex g_noalloc_mutex;
 uint32_t* g_noalloc_ptr[256] = {};  // device address of the scratch array, per device ordinal
 thread_local uint32_t h_noalloc_error;
+std::atomic<uint32_t> g_noalloc_turn{0};
 
 int32_t na_fail(int32_t code, const char* what, cudaError_t e = cudaSuccess) {
     std::string msg = what;
@@ -284,9 +292,10 @@ int32_t sort_noalloc(const float* positions, const uint32_t* ids, uint64_t n, fl
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "cudaDeviceGetAttribute", e);
     const uint32_t all = uint32_t(sms > 0 ? sms : 1);
     room = room && room < all ? room : all;
-    e = cudaMemsetAsync(scratch, 0, 2 * 4, s);
+    uint32_t* hdr = scratch + (g_noalloc_turn.fetch_add(1, std::memory_order_relaxed) % kNoAllocHeaders) * kNoAllocHeader;
+    e = cudaMemsetAsync(hdr, 0, kNoAllocHeader * 4, s);
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "clearing the header", e);
-    void* args[] = {&positions, &ids, &m, &radius, &scratch, &order};
+    void* args[] = {&positions, &ids, &m, &radius, &scratch, &hdr, &order};
     for (;; room /= 2) {
         // (a share of the SMs, of a stream or a process, holds fewer blocks than the device: half as many
         // are tried until they run at once, as one always does)
@@ -300,7 +309,7 @@ int32_t sort_noalloc(const float* positions, const uint32_t* ids, uint64_t n, fl
     }
     note_launch();
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "launching the cell sort", e);
-    e = cudaMemcpyAsync(&h_noalloc_error, scratch + kHdrError, 4, cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(&h_noalloc_error, hdr + kHdrError, 4, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return na_fail(SLF_ERR_CUDA, "finishing the cell sort", e);
     if (h_noalloc_error == kErrorWait) return na_fail(SLF_ERR_TIMEOUT, "the cell sort's blocks did not meet");

@@ -1,10 +1,13 @@
 """The cell sort without allocation where few of its blocks run at once (the threads then stride over the
-particles instead of holding them).
+particles instead of holding them), and from two host threads, whose calls may overlap on the GPU.
 """
 import ctypes
+import threading
 
 import numpy as np
 import pytest
+
+from solunar_b200.abi import PhysicsError
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +40,33 @@ def test_any_number_of_blocks_sorts(gpu_lib, n, blocks):
     assert status == 0
     assert np.array_equal(order.cpu().numpy(), expected(pos, ids))
 
+
+def test_overlapping_calls_end_and_the_next_one_sorts(gpu_lib):
+    import torch
+
+    # the same box in both threads: what one call reads of the other's tables stays plausible, the
+    # orders may be wrong, and neither call may wait for the other's blocks
+    n = 20001
+    pos, ids = arrays(n, 5)
+    d_pos, d_ids = torch.from_numpy(pos).cuda(), torch.from_numpy(ids).cuda()
+    orders = [torch.full((n,), -1, dtype=torch.int32, device="cuda") for _ in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    failures = []
+
+    def call(k, times):
+        for _ in range(times):
+            try:
+                gpu_lib.sort_by_cell_noalloc(d_pos.data_ptr(), d_ids.data_ptr(), n, RADIUS, orders[k].data_ptr(),
+                                             streams[k].cuda_stream)
+            except PhysicsError as e:
+                failures.append(e.kind)
+
+    threads = [threading.Thread(target=call, args=(k, 50)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert "Timeout" not in failures and "Cuda" not in failures
+    call(0, 1)
+    assert np.array_equal(orders[0].cpu().numpy(), expected(pos, ids))
