@@ -397,7 +397,7 @@ struct World {
     Status* d_status = nullptr;
     Status* h_status = nullptr;     // pinned
     uint32_t* h_posted = nullptr;   // pinned: nonzero once the status asked for is in h_status
-    bool polls = true;              // waits for it by polling (unless the device is set to block)
+    bool polls = true;              // waits for it by polling (polls_under)
     uint32_t* d_spoiled = nullptr;  // nonzero: the last substep will run again, or fails
 
     // The coupled bodies' own stream: what their points take of a substep (k_mover_felt, k_mover_fold)

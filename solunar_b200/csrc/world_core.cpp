@@ -2,6 +2,7 @@
 #include <atomic>
 #include <chrono>
 
+#include "status_wait.h"
 #include "world.h"
 
 namespace slf {
@@ -57,7 +58,7 @@ int32_t World::init(const slf_settings& settings) {
     SLF_CUDA(cudaMalloc(&d_spoiled, sizeof(uint32_t)));
     unsigned int flags = 0;
     SLF_CUDA(cudaGetDeviceFlags(&flags));
-    polls = (flags & cudaDeviceScheduleMask) != cudaDeviceScheduleBlockingSync;
+    polls = polls_under(flags);
     SLF_CUDA(cudaMallocHost(&h_consts, sizeof(StepConsts)));
     SLF_CUDA(cudaMemsetAsync(d_status, 0, sizeof(Status), stream));
     build_ground_sites();
