@@ -188,26 +188,33 @@ __global__ void k_scatter_members(uint32_t n, const uint32_t* __restrict__ lin, 
 // before its own in the quad, and the cells before it in its column.  A dozen loads from the table's
 // cache lines in k_rank_reorder (17 -> 21 us at 1M) in place of a count, a scan and a fill of the
 // keys (six nodes, 30 us at 1M and 26 at 75k).
-__device__ __forceinline__ uint32_t walk_row(const uint32_t* __restrict__ start, int3 span, uint32_t lin) {
+// Bricks begin at the box's own corner, not at the padding's: a cell further out, they split the pairs and
+// quads that water against a container fills (us with the bricks on the padding and on the corner: EXACT
+// density 435 -> 415 at 1M and 247 -> 231 at 500k, check 69 -> 67 at 500k; FAST push of 8,000 particles at
+// support 4 63.9 -> 61.8).
+__device__ __forceinline__ uint32_t walk_row(const uint32_t* __restrict__ start, int3 span, int pad, uint32_t lin) {
     const uint32_t sy = uint32_t(span.y), sz = uint32_t(span.z);
-    const uint32_t z = lin % sz, y = lin / sz % sy, x = lin / sz / sy;
-    const uint32_t x0 = x & ~1u, y0 = y & ~1u, z0 = z & ~3u, z1 = min(z0 + 4u, sz);
-    uint32_t row = __ldg(&start[x0 * sy * sz]);
+    const int z = int(lin % sz), y = int(lin / sz % sy), x = int(lin / sz / sy);
+    // bricks begin at the first cell that may hold points: 1 in a padded table (the first brick, of the
+    // padding alone, begins before the table)
+    const int x0 = ((x + pad) & ~1) - pad, y0 = ((y + pad) & ~1) - pad, z0 = ((z + 3 * pad) & ~3) - 3 * pad;
+    const uint32_t za = uint32_t(max(z0, 0)), zb = uint32_t(min(z0 + 4, span.z));
+    uint32_t row = __ldg(&start[uint32_t(max(x0, 0)) * sy * sz]);
 #pragma unroll
-    for (uint32_t dx = 0; dx < 2; ++dx) {
-        if (x0 + dx >= uint32_t(span.x)) continue;
-        const uint32_t slab = (x0 + dx) * sy * sz;
-        row += __ldg(&start[slab + y0 * sz]) - __ldg(&start[slab]);
+    for (int dx = 0; dx < 2; ++dx) {
+        if (uint32_t(x0 + dx) >= uint32_t(span.x)) continue;
+        const uint32_t slab = uint32_t(x0 + dx) * sy * sz;
+        row += __ldg(&start[slab + uint32_t(max(y0, 0)) * sz]) - __ldg(&start[slab]);
 #pragma unroll
-        for (uint32_t dy = 0; dy < 2; ++dy) {
-            if (y0 + dy >= sy) continue;
-            const uint32_t column = slab + (y0 + dy) * sz;
+        for (int dy = 0; dy < 2; ++dy) {
+            if (uint32_t(y0 + dy) >= sy) continue;
+            const uint32_t column = slab + uint32_t(y0 + dy) * sz;
             // columns before the cell's own in the quad count whole quads up to this one
-            const uint32_t upto = 2u * dx + dy < (x & 1u) * 2u + (y & 1u) ? z1 : z0;
+            const uint32_t upto = 2 * dx + dy < 2 * (x - x0) + (y - y0) ? zb : za;
             row += __ldg(&start[column + upto]) - __ldg(&start[column]);
         }
     }
-    return row + __ldg(&start[lin]) - __ldg(&start[lin - z + z0]);
+    return row + __ldg(&start[lin]) - __ldg(&start[lin - uint32_t(z) + za]);
 }
 
 // Final place = cell start + number of the cell's ids below this one's: the (cell, id) order
@@ -221,7 +228,7 @@ __global__ void k_rank_reorder(uint32_t n, const uint32_t* __restrict__ lin, con
                                float4* __restrict__ vel_out, float* __restrict__ rho_out,
                                int4* __restrict__ cells_out, const float2* __restrict__ warm_in,
                                float2* __restrict__ warm_out, uint32_t skip_begin, uint32_t skip_end, Status* st,
-                               uint32_t* __restrict__ dest, int3 span, uint32_t* __restrict__ order) {
+                               uint32_t* __restrict__ dest, int3 span, int pad, uint32_t* __restrict__ order) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     // a job left undone (the fault injection of the dispatcher tests) places nothing; the count
     // of placed particles tells the host whether every particle was placed
@@ -235,7 +242,7 @@ __global__ void k_rank_reorder(uint32_t n, const uint32_t* __restrict__ lin, con
     uint32_t rank = 0;
     for (uint32_t k = b; k < e; ++k) rank += members[k] < id ? 1u : 0u;
     uint32_t f = b + rank;
-    if (order) order[walk_row(start, span, l) + rank] = f;  // every row, a skipped job's too
+    if (order) order[walk_row(start, span, pad, l) + rank] = f;  // every row, a skipped job's too
     if (!work) return;
     if (dest) dest[i] = f;  // where each particle went, for the adjoint's way back
     ids_out[f] = id;
@@ -2285,12 +2292,12 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
                          const uint32_t* ids_in, const float4* pos_in, const float4* vel_in, const float* rho_in,
                          const int4* cells_in, uint32_t* ids_out, float4* pos_out, float4* vel_out, float* rho_out,
                          int4* cells_out, const float2* warm_in, float2* warm_out, uint32_t skip_begin,
-                         uint32_t skip_end, Status* st, uint32_t* dest, int3 span, uint32_t* order, cudaStream_t s) {
+                         uint32_t skip_end, Status* st, uint32_t* dest, int3 span, int pad, uint32_t* order, cudaStream_t s) {
     if (n)
         k_rank_reorder<<<blocks_for(n), kBlock, 0, s>>>(n, lin, start, members, ids_in, pos_in, vel_in, rho_in,
                                                         cells_in, ids_out, pos_out, vel_out, rho_out, cells_out,
                                                         warm_in, warm_out,
-                                                        skip_begin, skip_end, st, dest, span, order);
+                                                        skip_begin, skip_end, st, dest, span, pad, order);
 }
 
 // blocks of a pass that gives each row `lanes` lanes

@@ -904,6 +904,7 @@ struct World {
     struct SortPlan {
         int3 lo{}, span{};
         uint32_t volume = 0;
+        int pad = 0;           // empty cells around the box on every side
         bool ordered = false;  // the lists get a walk order (else they keep the particle order)
         uint32_t job_lo = 0, job_hi = 0;
     };

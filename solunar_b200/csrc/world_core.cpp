@@ -502,7 +502,8 @@ int32_t World::plan_sort(SortPlan& sp, bool stable) {
             }
     }
     // an empty cell around the box, where the table still fits: every particle's 27 cells then lie
-    // inside it, and the density scan needs no bounds checks (cell order does not depend on the box)
+    // inside it, and the density scan needs no bounds checks (cell order does not depend on the box,
+    // and the walk order's bricks begin inside the padding)
     {
         int64_t pl[3], ph[3];
         bool inside = true;
@@ -511,11 +512,11 @@ int32_t World::plan_sort(SortPlan& sp, bool stable) {
             ph[a] = hi[a] + 1;
             inside = inside && pl[a] >= INT32_MIN && ph[a] <= INT32_MAX;
         }
-        if (inside && fits(volume_of(pl, ph)))
-            for (int a = 0; a < 3; ++a) {
-                lo[a] = pl[a];
-                hi[a] = ph[a];
-            }
+        sp.pad = inside && fits(volume_of(pl, ph)) ? 1 : 0;
+        for (int a = 0; a < 3; ++a) {
+            lo[a] -= sp.pad;
+            hi[a] += sp.pad;
+        }
     }
     __int128 vol = volume_of(lo, hi);
     if (!fits(vol))
@@ -565,7 +566,7 @@ int32_t World::enqueue_sort(int to, const SortPlan& sp, cudaStream_t on, Substep
     timed("hash_reorder", bytes_per_particle::reorder, [&] {
         launch_rank_reorder(uint32_t(n), lin.p, count.p, members.p, ids[cid].p, pos[cpos].p, vel[cpos].p,
                             rho[cid].p, cells_of(cpos), ids[1 - cid].p, pos[to].p, vel[to].p, rho[1 - cid].p,
-                            cells_of(to), warm_in(), warm_out(), sp.job_lo, sp.job_hi, d_status, sort_dest, sp.span,
+                            cells_of(to), warm_in(), warm_out(), sp.job_lo, sp.job_hi, d_status, sort_dest, sp.span, sp.pad,
                             sp.ordered ? worder.p : nullptr, on);
     });
     return SLF_OK;
