@@ -191,7 +191,8 @@ __global__ void k_scatter_members(uint32_t n, const uint32_t* __restrict__ lin, 
 // Bricks begin at the box's own corner, not at the padding's: a cell further out, they split the pairs and
 // quads that water against a container fills (us with the bricks on the padding and on the corner: EXACT
 // density 435 -> 415 at 1M and 247 -> 231 at 500k, check 69 -> 67 at 500k; FAST push of 8,000 particles at
-// support 4 63.9 -> 61.8).
+// support 4 63.9 -> 61.8).  Over 36 shapes of 8k to 600k particles the passes take 0.6 % less in sum, single
+// shapes up to 4 % more or 7 % less.
 __device__ __forceinline__ uint32_t walk_row(const uint32_t* __restrict__ start, int3 span, int pad, uint32_t lin) {
     const uint32_t sy = uint32_t(span.y), sz = uint32_t(span.z);
     const int z = int(lin % sz), y = int(lin / sz % sy), x = int(lin / sz / sy);
@@ -1025,16 +1026,16 @@ __global__ void __launch_bounds__(kGroupBlock, kGroupBlocks)
 #endif
 constexpr int kListUnroll = SLF_LIST_UNROLL;
 constexpr int kViscousBlock = 128;
-// resident blocks per SM the list-walking kernels are compiled for (caps their registers); the
-// solver check runs best at four blocks (64 registers; 76 uncapped, three blocks)
-#ifndef SLF_RATE_MIN_BLOCKS
-#define SLF_RATE_MIN_BLOCKS 4
-#endif
-// the push at five blocks a SM (48 registers; 56 uncapped at four blocks: 72.2 -> 70.5 us at 1M;
-// six blocks spill)
-#ifndef SLF_PUSH_MIN_BLOCKS
-#define SLF_PUSH_MIN_BLOCKS 5
-#endif
+// Resident blocks a SM that the solver's check and push are compiled for (caps their registers: check 64
+// and 79, push 48 and 60).  Where the grid fills no more than three blocks a SM the registers are worth
+// more than the warps, which there are none of: kFewBlocks, without spills and with more gathers in
+// flight.  us, check and push, at the blocks for large grids / for few (and before the check lost its
+// other walk, when it took 76 registers to gather ahead):
+//     6,000 of support 4    58.6, 47.0 / 52.5, 45.0 (50.5, 45.4)     4,000  51.7, 39.3 / 44.7, 38.0 (46.5, 41.4)
+//     15,000 of support 3   35.1, 25.9 / 30.9, 25.1 (33.4, 27.1)    60,000 45.7, 37.1 / 43.3, 35.6 (45.5, 35.4)
+//     100,000 of support 2  22.9, 16.3 / 22.9, 14.9 (23.2, 16.9)    150,000 27.0, 18.9 / 31.2, 18.9
+// and the push of 500k, 729k and 360k of support 3 41.3, 54.6, 90.2 / 43.5, 58.2, 101.
+constexpr int kRateBlocks = 4, kPushBlocks = 5, kFewBlocks = 3;
 
 template <class F>
 __device__ __forceinline__ void each_listed(const PairLists& l, uint32_t i, const float4* __restrict__ pts, F&& f) {
@@ -1693,8 +1694,8 @@ __device__ __forceinline__ void rate_particle(const Params& p, const StepConsts*
 
 // One check of the solve, a particle a thread, and the average error of the particles under
 // load (dfsph.rs:263-268) in a last-block finish.
-template <int WHICH>
-__global__ void __launch_bounds__(kBlock, SLF_RATE_MIN_BLOCKS) k_rate(Params p, const StepConsts* __restrict__ sc, PairLists fl,
+template <int WHICH, int BLOCKS>
+__global__ void __launch_bounds__(kBlock, BLOCKS) k_rate(Params p, const StepConsts* __restrict__ sc, PairLists fl,
                                                  PairLists wl, const float4* __restrict__ pos,
                                                  const float4* __restrict__ vel, const float* __restrict__ rho,
                                                  const float* __restrict__ alpha, float* __restrict__ kappa_w,
@@ -1754,7 +1755,8 @@ __device__ __forceinline__ void push_particle(const Params& p, const StepConsts*
     if (applied) applied[2 * (size_t)i] += own * dt;
 }
 
-__global__ void __launch_bounds__(kBlock, SLF_PUSH_MIN_BLOCKS) k_push(Params p, const StepConsts* __restrict__ sc, PairLists fl,
+template <int BLOCKS>
+__global__ void __launch_bounds__(kBlock, BLOCKS) k_push(Params p, const StepConsts* __restrict__ sc, PairLists fl,
                                                  PairLists wl, const float4* __restrict__ pos,
                                                  float4* __restrict__ vel, Status* st,
                                                  float* __restrict__ applied, unsigned long long loop) {
@@ -2197,12 +2199,14 @@ static inline uint32_t blocks_for(uint32_t n) {
 #ifndef SLF_SOLVER_RESIDENT
 #define SLF_SOLVER_RESIDENT 1
 #endif
-// resident blocks of k_rate<0>, k_rate<1>, k_push, k_density<0>, k_density<1>, k_wcsph_force on the
+// resident blocks of k_rate<0>, k_rate<1> and k_push (as large grids run them), k_density<0>, k_density<1>, k_wcsph_force on the
 // device (prepare_solver_grids; 0: not known yet, the grid then covers every row)
 static std::atomic<uint32_t> g_resident[6] = {0, 0, 0, 0, 0, 0};
 
 // blocks of the density pass up to which it runs wide: two a SM
 static std::atomic<uint32_t> g_wide_blocks{0};
+// blocks of the check and the push up to which no SM holds more than kFewBlocks
+static std::atomic<uint32_t> g_few_blocks{0};
 
 void prepare_solver_grids() {
     if (!SLF_SOLVER_RESIDENT || g_resident[2].load()) return;
@@ -2210,13 +2214,14 @@ void prepare_solver_grids() {
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0], k_rate<0>, kBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1], k_rate<1>, kBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[2], k_push, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0], k_rate<0, kRateBlocks>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1], k_rate<1, kRateBlocks>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[2], k_push<kPushBlocks>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[3], k_density<0, true, false>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[4], k_density<1, false, false>, kBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[5], k_wcsph_force<true>, kBlock, 0);
     g_wide_blocks.store(2u * uint32_t(std::max(sms, 0)));
+    g_few_blocks.store(uint32_t(kFewBlocks * std::max(sms, 0)));
     for (int k = 0; k < 6; ++k) g_resident[k].store(uint32_t(std::max(per[k], 0) * std::max(sms, 0)));
 }
 
@@ -2468,17 +2473,24 @@ void launch_rate(int which, const Params& p, const StepConsts* sc, const PairLis
     uint32_t nb = solver_blocks(p.n, which == 0 ? 0 : 1);
     DD* part = static_cast<DD*>(partials);
     uint32_t* loaded = reinterpret_cast<uint32_t*>(part + (p.n + kBlock - 1) / kBlock);
-    if (which == 0)
-        k_rate<0><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, alpha, reinterpret_cast<float*>(pos), part,
-                                        loaded, st, rec, loop);
-    else
-        k_rate<1><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, rho, alpha, reinterpret_cast<float*>(pos), part,
-                                        loaded, st, rec, loop);
+    auto launch = [&](auto w, auto few) {
+        k_rate<decltype(w)::value, decltype(few)::value><<<nb, kBlock, 0, s>>>(
+            p, sc, fl, wl, pos, vel, rho, alpha, reinterpret_cast<float*>(pos), part, loaded, st, rec, loop);
+    };
+    auto sized = [&](auto w) {
+        if (nb <= g_few_blocks.load()) launch(w, std::integral_constant<int, kFewBlocks>{});
+        else launch(w, std::integral_constant<int, kRateBlocks>{});
+    };
+    if (which == 0) sized(std::integral_constant<int, 0>{});
+    else sized(std::integral_constant<int, 1>{});
 }
 
 void launch_push(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl, const float4* pos,
                  float4* vel, Status* st, float* applied, cudaStream_t s, unsigned long long loop) {
-    if (p.n) k_push<<<solver_blocks(p.n, 2), kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, st, applied, loop);
+    if (!p.n) return;
+    const uint32_t nb = solver_blocks(p.n, 2);
+    if (nb <= g_few_blocks.load()) k_push<kFewBlocks><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, st, applied, loop);
+    else k_push<kPushBlocks><<<nb, kBlock, 0, s>>>(p, sc, fl, wl, pos, vel, st, applied, loop);
 }
 
 // Warm start of a solve: the stiffness that applies `share` of the impulse S the particle's last
