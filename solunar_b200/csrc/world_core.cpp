@@ -610,6 +610,7 @@ int32_t World::compute_densities() {
     Params p = params();
     for (;;) {
         SLF_TRY(reset_status());
+        stats_fresh = false;  // (the status loses the state's box and speed; nothing here folds them again)
         density_pass(p, cpos, fluid_lists(), wall_lists(), rho[cid].p);
         SLF_TRY(read_status());
         int32_t st = lists_fit();
