@@ -432,12 +432,19 @@ __device__ __forceinline__ float ground_near(const TerrainDev& T, float px, floa
 // to hide behind.  74k particles: 57 -> 48 us, at support 4 378 -> 302; 111k, three blocks a SM,
 // stay.
 
-// a / radius, rounded as the IEEE division rounds it, without one: with y = RN(1 / r),
-// q = RN(a y), the remainder a - q r is exact in one fma and RN(q + remainder y) is RN(a / r)
-// (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990).  Three
-// operations against the division's ten or so.  The remainder must not underflow: the settings'
-// radius is checked on the host (odd_radius) and numerators under 2^-100 divide.  LOW: whether
-// the numerator may be so small (a distance is 0 or at least 2^-75).
+// a / radius, rounded as the IEEE division rounds it, without one: y = RN(1 / r), q = RN(a y), and
+// RN(q + (a - q r) y) in two fmas, after Markstein ("Computation of elementary functions on the IBM RISC
+// System/6000", 1990).  Three operations against the division's ten or so.  His theorem wants q within an
+// ulp of a / r, and with significands a, r in [1, 2) this q may miss by (a + 1) / 2 ulps where a < r.  So:
+//   - within an ulp the remainder is exact, and the sum errs by |remainder| |y - 1 / r|, near a midpoint
+//     r 2^-50 at most (in units where ulp(q) = 2^-24), while a quotient is 2^-48 / r or more from it.
+//   - further off the remainder may round, by 2^-47, and the sum errs by 2.8 2^-48 at most; but a / r is
+//     (2 - a) 2^-25 or more short of the midpoint an ulp and a half from q.  With a = 2 - k 2^-23 that is
+//     k 2^-48, enough from k = 3 on; k = 1 has no r above it, and k = 2 only r = 2 - 2^-23, where it is
+//     3 2^-48 against an error of 2.5 2^-48.
+// (test_radius_division.py goes through all a for some hundred radii.)  The remainder must not underflow:
+// the settings' radius is checked on the host (odd_radius) and numerators under 2^-100 divide.  LOW:
+// whether the numerator may be so small (a distance is 0 or at least 2^-75).
 template <bool LOW>
 __device__ __forceinline__ f32x2 div_radius2(const Params& p, f32x2 a) {
     const f32x2 y = splat2(p.inv_radius);
