@@ -1,6 +1,8 @@
 // kernels.cu -- the fluid substep on the device.
 //
-// One thread per particle throughout.  Particles live in SoA float4 arrays (x, y, z, unused)
+// One thread per particle, or, in small scenes' density and WCSPH force passes, several lanes of a warp.
+// Particles live in SoA float4 arrays (x, y, z and what a pass leaves for the gathers of the next: p / rho^2
+// or the stiffness beside a position, the density beside a velocity, PairRecords),
 // sorted by (cell, id) like the reference's arrays (src/fluid/mod.rs:540-566); every pass reads
 // neighbours through the cell tables in the reference's list order, so each particle's sums are
 // the reference's sequential sums, bit for bit.  Grid-wide reductions (bounding box, fastest
@@ -104,8 +106,8 @@ __global__ void __launch_bounds__(32) k_post_status(const Status* st, Status* ou
 // ---- spatial hash: counting sort by dense cell index, then id within each cell ------------
 
 // cells (cell-relative positions) non-null: the cell is stored, not computed
-// begin (a substep recorded as a graph): the status starts afresh, and the substep's constants come
-// from the host's copy, which it writes before each launch of the graph
+// begin (a substep recorded as a graph, or a WCSPH substep launch by launch): the status starts afresh,
+// and the substep's constants come from the host's copy, which it writes before each launch
 __global__ void k_count_cells(Params p, const float4* __restrict__ pos, const int4* __restrict__ cells, int3 low,
                               int3 span, uint32_t* count, uint32_t* lin, uint32_t* slot, SubstepBegin begin) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -558,7 +560,6 @@ __device__ __forceinline__ void pair_terms(const Params& p, const PairLists& l, 
 // ---- densities (mod.rs:621-675) and the substep's neighbour lists, with WCSPH pressure
 // (step.rs:147-172) or the DFSPH factors (dfsph.rs:108-163) --------------------------------
 
-// four blocks a SM (64 registers), as the pass compiled before it strode over rows
 // What the pass lists: the fluid (0), then the walls (1).
 struct DensityIn {
     GridDev grid[2];
@@ -566,7 +567,7 @@ struct DensityIn {
     PairLists list[2];
 };
 
-// EXTRA: terrain regions or coupled bodies add their terms
+// EXTRA: terrain regions or coupled bodies add their terms.  WIDE: two blocks a SM, else four (64 registers).
 template <int SOLVER, bool EXTRA, bool WIDE>
 __global__ void __launch_bounds__(kBlock, WIDE ? 2 : 4)
     k_density(const __grid_constant__ Params p, const __grid_constant__ DensityIn in, float* __restrict__ rho,

@@ -14,8 +14,8 @@ namespace slf {
 void launch_state_stats(const Params& p, const float4* pos, const float4* vel, Status* st, cudaStream_t s);
 void launch_max_compression(const Params& p, const float* rho, Status* st, cudaStream_t s);
 
-// What the first kernel of a recorded substep sets (status null: nothing): the status afresh, and the
-// constants from the host's pinned copy.
+// What the first kernel of a substep sets, recorded as a graph or (WCSPH) launch by launch (status null:
+// nothing): the status afresh, and the constants from the host's pinned copy.
 struct SubstepBegin {
     Status* status;
     StepConsts* consts;
@@ -175,11 +175,11 @@ void launch_set_consts(const StepConsts& c, StepConsts* out, cudaStream_t s);
 
 // xyz triples <-> float4
 void launch_pack3(uint32_t n, const float4* in, float* out, cudaStream_t s);
-// bad (optional): incremented for each triple with a non finite component
 // a whole state, n position triples and then n velocity triples, in (with its box, speed and non finite
 // components in the status) and out
 void launch_unpack_state(const Params& p, const float* in, float4* pos, float4* vel, Status* st, cudaStream_t s);
 void launch_pack_state(uint32_t n, const float4* pos, const float4* vel, float* out, cudaStream_t s);
+// bad (optional): incremented for each triple with a non finite component
 void launch_unpack3(uint32_t n, const float* in, float4* out, cudaStream_t s, uint32_t* bad = nullptr);
 
 // FAST arithmetic variants (kernels_fast.cu): same lists, order and sums, fused rounding; the

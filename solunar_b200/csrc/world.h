@@ -708,9 +708,8 @@ struct World {
                       cudaStream_t on = nullptr);
 
     const uint32_t* walk_order() const { return worder_valid ? worder.p : nullptr; }
-    // EXACT DFSPH keeps each pair's gradient for the solver check (16 bytes a slot, fluid and
-    // walls): the check then gathers a neighbour's velocity only, not its position too
-    // EXACT DFSPH keeps each pair's gradient for the solver check, and the walls' for the push
+    // EXACT DFSPH keeps each pair's gradient (16 bytes a slot, fluid and walls): the check then gathers
+    // a neighbour's velocity only, not its position too, and the push gathers nothing of the walls
     bool keeps_gradients() const { return !fast() && s.solver == SLF_SOLVER_DFSPH; }
     PairLists fluid_lists() const {
         return PairLists{list_cap, fent.p, fcnt.p, walk_order(), keeps_gradients() ? fgv.p : nullptr};

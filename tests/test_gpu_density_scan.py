@@ -1,8 +1,8 @@
 """The EXACT density pass where its scan and its packed pair arithmetic can go wrong, bit for bit
 against the restatement: cells of any number of points (remainders of the groups of four), particles
 beside, beyond and far from a free-standing wall, lists that outgrow their room, and radii on both
-sides of the range whose divisions take the reciprocal.  33,000 particles: the pass a thread a
-particle runs (smaller scenes take a warp a particle).
+sides of the range whose divisions take the reciprocal.  33,000 particles: a thread a row at supports
+under 3 (smaller scenes, and larger ones at more support, give a row several lanes).
 """
 import numpy as np
 import pytest
