@@ -58,6 +58,16 @@ __device__ __forceinline__ uint32_t listed_count(const PairLists& l, uint32_t i)
 // hardware flushes such inputs, and 1/0 would turn the pair's zero terms into NaN)
 __device__ __forceinline__ float inv_length(float d2) { return d2 >= 1.17549435e-38f ? rsqrtf(d2) : 0.0f; }
 
+// |r| and 1/|r| of d2 = r.r, each with a Newton step that leaves it within about half an ulp, as the root
+// and the division would; false where inv_length is 0
+__device__ __forceinline__ bool lengths(float d2, float& d, float& inv) {
+    inv = inv_length(d2);
+    d = d2 * inv;
+    d = fmaf(0.5f * inv, fmaf(-d, d, d2), d);
+    inv = fmaf(inv, fmaf(-d, inv, 1.0f), inv);
+    return inv != 0.0f;
+}
+
 // gradient factor g(d) = slope(d) / d = grad_scale (1 - d/r)^3 and its derivative in d
 __device__ __forceinline__ void grad_factor(const Params& p, float d, float& g, float& gp) {
     float om = 1.0f - d * p.inv_radius;
@@ -764,10 +774,10 @@ __global__ void __launch_bounds__(kBlock) k_adj_density_group(Params p, PairList
     const float rbi = rb[i];
     float3 xbar = make_float3(0, 0, 0);
     auto pair = [&](float3 r, float share) {
-        const float d2 = dotf(r, r), inv = inv_length(d2);
-        if (inv == 0.0f) return;
+        float d, inv;
+        if (!lengths(dotf(r, r), d, inv)) return;
         float g, gp;
-        grad_factor(p, d2 * inv, g, gp);
+        grad_factor(p, d, g, gp);
         xbar = xbar + r * (g * p.mass * share);
     };
     const uint32_t nf = valid ? listed_count(fl, row) : 0u;
@@ -820,10 +830,10 @@ __global__ void __launch_bounds__(kBlock) k_adj_density(Params p, PairLists fl, 
                   },
                   [&](uint32_t, float4 q, uint32_t e) {
                       float3 r = pair_off(p, form, xi, q, e);
-                      float d2 = dotf(r, r), inv = inv_length(d2);
-                      if (inv == 0.0f) return;
+                      float d, inv;
+                      if (!lengths(dotf(r, r), d, inv)) return;
                       float g, gp;
-                      grad_factor(p, d2 * inv, g, gp);
+                      grad_factor(p, d, g, gp);
                       xbar = xbar + r * (g * p.mass * (rbi + q.w));
                   });
     uint32_t nw = listed_count(wl, row);
@@ -1138,20 +1148,20 @@ __global__ void __launch_bounds__(kBlock) k_adj_alpha_prep(Params p, PairLists f
     float3 G = make_float3(0, 0, 0);
     walk4<float4>(fl, form, row, [&](uint32_t j) { return __ldg(&pos[j]); }, [&](uint32_t, float4 q, uint32_t e) {
         float3 r = pair_off(p, form, xi, q, e);
-        float d2 = dotf(r, r), inv = inv_length(d2);
-        if (inv == 0.0f) return;
+        float d, inv;
+        if (!lengths(dotf(r, r), d, inv)) return;
         float g, gp;
-        grad_factor(p, d2 * inv, g, gp);
+        grad_factor(p, d, g, gp);
         G = G + r * (g * p.mass);
     });
     uint32_t nw = listed_count(wl, row);
     for (uint32_t k = 0; k < nw; ++k) {
         uint32_t e = listed_raw(wl, form, row, k), j = entry_index(e, form);
         float3 r = pair_off(p, form, xi, __ldg(&walls[j]), e);
-        float d2 = dotf(r, r), inv = inv_length(d2);
-        if (inv == 0.0f) continue;
+        float d, inv;
+        if (!lengths(dotf(r, r), d, inv)) continue;
         float g, gp;
-        grad_factor(p, d2 * inv, g, gp);
+        grad_factor(p, d, g, gp);
         G = G + r * (g * p.mass);
     }
     float a = alpha[i];
@@ -1160,7 +1170,9 @@ __global__ void __launch_bounds__(kBlock) k_adj_alpha_prep(Params p, PairLists f
 
 // Then both passes over the pairs that are left, in one walk: the factors' share, through grad W and
 // its transpose, and the densities' (k_adj_density's).  Two walks of the lists measured 68 us more at
-// 512k particles.
+// 512k particles.  Lengths straight from the reciprocal root save 10 us of the two kernels' 158 at 500k,
+// but the DFSPH position gradients were then up to 1.4 % further from 64 bits (lengths: 0.4 %, the sums'
+// order).
 __global__ void __launch_bounds__(kBlock, 4) k_adj_alpha_density(Params p, PairLists fl, PairLists wl, int form,
                                                               const float4* __restrict__ pos,
                                                               const float4* __restrict__ walls,
@@ -1183,10 +1195,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_alpha_density(Params p, PairL
                },
                [&](uint32_t, const Two& q, uint32_t e) {
                    float3 r = pair_off(p, form, xi, q.a, e);
-                   float d2 = dotf(r, r), inv = inv_length(d2);
-                   if (inv == 0.0f) return;
+                   float d, inv;
+                   if (!lengths(dotf(r, r), d, inv)) return;
                    float g, gp;
-                   grad_factor(p, d2 * inv, g, gp);
+                   grad_factor(p, d, g, gp);
                    float3 gw = r * (g * m);
                    float4 oj = q.b;
                    float3 c = (Gi + gw) * (2.0f * m * tbi) - (f3(oj) - gw) * (2.0f * m * oj.w);
@@ -1196,10 +1208,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_adj_alpha_density(Params p, PairL
     for (uint32_t k = 0; k < nw; ++k) {
         uint32_t e = listed_raw(wl, form, row, k), j = entry_index(e, form);
         float3 r = pair_off(p, form, xi, __ldg(&walls[j]), e);
-        float d2 = dotf(r, r), inv = inv_length(d2);
-        if (inv == 0.0f) continue;
+        float d, inv;
+        if (!lengths(dotf(r, r), d, inv)) continue;
         float g, gp;
-        grad_factor(p, d2 * inv, g, gp);
+        grad_factor(p, d, g, gp);
         float3 c = Gi * (2.0f * m * tbi);
         xacc = xacc + c * g + r * (dotf(c, r) * gp * inv + g * m * rbi);
     }
