@@ -2320,12 +2320,12 @@ static uint32_t group_blocks(uint32_t n, int lanes) {
     return (n + rows - 1) / rows;
 }
 
-size_t density_scratch_words(uint32_t n, uint32_t cap, float support) {
+size_t density_scratch_words(uint32_t n, uint32_t cap, float support, bool dfsph) {
     // one list room a thread of the density pass's grid
     const uint32_t nb = (n + kBlock - 1) / kBlock, r0 = g_resident[3].load(), r1 = g_resident[4].load();
     const uint32_t resident = r0 && r1 ? std::max(r0, r1) : nb;
     // (with lanes to share, a list room a row of the grid, whose last tile may be part empty)
-    const size_t group = group_lanes(n, support) ? size_t(n + kGroupBlock) : 0;
+    const size_t group = group_lanes(n, support, dfsph) ? size_t(n + kGroupBlock) : 0;
     return std::max(size_t(std::min(resident, nb)) * kBlock, group) * cap;
 }
 
@@ -2338,7 +2338,7 @@ void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float
     const DensityIn in{{fg, wg}, {pos, walls}, {fl, wl}};
     // (terrain, whose sites every lane would take alike, and a DFSPH row's body points keep a thread a row)
     const bool shared = T.regions == 0 && slope == nullptr && (p.solver == 0 || M.count == 0);
-    if (shared && with_lanes(group_lanes(p.n, p.radius / p.spacing), [&](auto lanes) {
+    if (shared && with_lanes(group_lanes(p.n, p.radius / p.spacing, p.solver != 0), [&](auto lanes) {
             constexpr int L = decltype(lanes)::value;
             const uint32_t nb = group_blocks(p.n, L);
             auto launch = [&](auto flight) {
@@ -2389,7 +2389,7 @@ void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& 
                         float4* vel_pre, const TerrainDev& T, const float4* slope, cudaStream_t s,
                         const MoverDev& M) {
     if (!p.n) return;
-    if (T.regions == 0 && slope == nullptr && with_lanes(group_lanes(p.n, p.radius / p.spacing), [&](auto lanes) {
+    if (T.regions == 0 && slope == nullptr && with_lanes(group_lanes(p.n, p.radius / p.spacing, false), [&](auto lanes) {
             constexpr int L = decltype(lanes)::value;
             const uint32_t nb = group_blocks(p.n, L);
             if (M.count)

@@ -58,12 +58,22 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
 //        46656              75   88   97    -    -                  388  333  304  347    -
 //        74088              77  109    -    -    -                  469  431  436    -    -
 //       110592              96  149    -    -    -                  617  604  630    -    -
-// (a warp a row with shuffled sums, before: 8,000 particles at support 4 83 + 66.)
-inline int group_lanes(uint32_t n, float support) {
+// (a warp a row with shuffled sums, before: 8,000 particles at support 4 83 + 66.)  DFSPH's density has five
+// ordered sums a row where WCSPH's has one, and no force pass to share the gain, so its lines lie nearer:
+//            n   support 2: thread  L=4  L=8 L=16 L=32     support 4: thread  L=4  L=8 L=16 L=32
+//         1000              41   31   24   16   15                  188  133   66   43   28
+//         5832              43   33   25   18   23                  206  145   78   57   58
+//        17576              43   36   32   33   45                  218  172  108  118  134
+//        27000              44   41   49   45   62                  237  185  168  170  201
+//        32000              46   49   52   52   72                    -    -    -    -    -
+//        46656              49   64   70   69   99                  288  305  249  263  331
+//        74088               -    -    -    -    -                  330  370  361  415  518
+// (at support 3, thread / L=8: 46,656 145 / 142, 74,088 168 / 207).
+inline int group_lanes(uint32_t n, float support, bool dfsph) {
     if (n <= 2048u) return 32;
     if (n <= 8192u) return support >= 3.0f && n <= 4096u ? 32 : 16;
-    if (support >= 3.0f) return n <= 57344u ? 8 : n <= 114688u ? 4 : 0;
-    return n <= 20480u ? 8 : n <= 32768u ? 4 : 0;
+    if (support >= 3.0f) return n <= 57344u ? 8 : n <= 114688u && !dfsph ? 4 : 0;
+    return n <= 20480u ? 8 : n <= (dfsph ? 28672u : 32768u) ? 4 : 0;
 }
 
 // Lanes a row of the WCSPH adjoint (k_adj_force_group, k_adj_density_group) in scenes without terrain
@@ -89,7 +99,7 @@ void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float
                     Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M,
                     uint32_t* scratch, float4* vel);
 // words of launch_density's scratch for n particles and lists of cap slots
-size_t density_scratch_words(uint32_t n, uint32_t cap, float support);
+size_t density_scratch_words(uint32_t n, uint32_t cap, float support, bool dfsph);
 // vel_pre (optional): the velocity before the wall clamp, its w lane the bits of the components
 // the clamp zeroed (1 x, 2 y, 4 z), for the adjoint
 void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,

@@ -354,7 +354,10 @@ int32_t World::ensure_work_buffers() {
     SLF_TRY(cslot.ensure(n, 0, stream));
     SLF_TRY(members.ensure(n, 0, stream));
     SLF_TRY(partials.ensure(rate_partial_bytes(uint32_t(n)), 0, stream));
-    if (!fast()) SLF_TRY(dscratch.ensure(density_scratch_words(uint32_t(n), list_cap, radius / s.spacing), 0, stream));
+    if (!fast()) {
+        const bool dfsph = s.solver == SLF_SOLVER_DFSPH;
+        SLF_TRY(dscratch.ensure(density_scratch_words(uint32_t(n), list_cap, radius / s.spacing, dfsph), 0, stream));
+    }
     return SLF_OK;
 }
 
@@ -535,7 +538,8 @@ int32_t World::plan_sort(SortPlan& sp, bool stable) {
     SLF_TRY(tiles.ensure(scan_tiles(sp.volume) + 1, 0, stream));
     // the walk order of this sort's lists (none where every pass over the lists gives a row
     // several lanes)
-    bool shared_rows = !fast() && s.solver == SLF_SOLVER_WCSPH && group_lanes(uint32_t(n), radius / s.spacing) && terrains.empty();
+    bool shared_rows = !fast() && s.solver == SLF_SOLVER_WCSPH && terrains.empty() &&
+                       group_lanes(uint32_t(n), radius / s.spacing, false);
     sp.ordered = !shared_rows;
     if (sp.ordered) SLF_TRY(worder.ensure(n, 0, stream));
     worder_valid = sp.ordered;

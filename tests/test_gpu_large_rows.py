@@ -42,6 +42,17 @@ def test_dfsph_rows_at_the_edge_of_few_blocks(gpu_lib, oracle_lib, n):
     assert_same(g, o)
 
 
+# where the DFSPH density pass stops giving a row several lanes
+@pytest.mark.parametrize("n,support", [(28672, 2.0), (28673, 2.0), (57344, 3.0), (57345, 3.0)])
+def test_dfsph_rows_at_the_edge_of_several_lanes(gpu_lib, oracle_lib, n, support):
+    settings = FluidSettings(solver=FluidSolver.DFSPH, spacing=SPACING, support=support)
+    g, o = gpu_lib.FluidWorld(settings), oracle_lib.OracleWorld(settings, residual_sum=1)
+    fill((g, o), n)
+    a, b = g.step(3e-4), o.step(3e-4)
+    assert (a.substeps, a.iterations, a.held_back) == (b.substeps, b.iterations, b.held_back)
+    assert_same(g, o)
+
+
 # 296 and 444 blocks of 256 rows: up to two a SM the density pass runs wide, past three the WCSPH force
 # strides over its rows
 @pytest.mark.parametrize("n", [296 * 256, 296 * 256 + 1, 120_001])
