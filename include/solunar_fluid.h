@@ -425,6 +425,10 @@ int32_t slf_debug_skip_job(slf_world* world, int64_t job);
  * again with room for its longest list, from the committed state.  Invalidates the lists. */
 int32_t slf_debug_list_room(slf_world* world, uint32_t room);
 
+/* Test hook: the EXACT density pass has room for the unfinished lists of at most `rows` rows at once
+ * (rounded up to 256; 0: no limit), as where the device's memory is short. */
+int32_t slf_debug_density_rows(slf_world* world, uint64_t rows);
+
 /* slf_sort_by_cell_noalloc as where at most `blocks` (0: no limit) of its blocks run at once. */
 int32_t slf_debug_sort_by_cell_noalloc(const float* positions, const uint32_t* ids, uint64_t n, float radius,
                                        uint32_t* order, void* stream, uint32_t blocks);

@@ -499,6 +499,15 @@ int32_t slf_debug_list_room(slf_world* world, uint32_t room) {
     return w.n ? w.ensure_work_buffers() : SLF_OK;
 }
 
+int32_t slf_debug_density_rows(slf_world* world, uint64_t rows) {
+    SLF_WORLD(world);
+    World& w = world->w;
+    SLF_TRY(w.flush());
+    w.density_rows_most = rows;
+    w.dscratch.release(w.stream);
+    return w.n ? w.ensure_work_buffers() : SLF_OK;
+}
+
 int32_t slf_last_iterations(const slf_world* world, uint32_t* divergence, uint32_t* density) {
     SLF_WORLD(world);
     if (divergence) *divergence = world->w.last_iterations[0];

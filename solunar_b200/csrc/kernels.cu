@@ -2320,24 +2320,26 @@ static uint32_t group_blocks(uint32_t n, int lanes) {
     return (n + rows - 1) / rows;
 }
 
-size_t density_scratch_words(uint32_t n, uint32_t cap, float support, bool dfsph) {
-    // one list room a thread of the density pass's grid
+size_t density_scratch_rows(uint32_t n, float support, bool dfsph) {
+    static_assert(kDensityRowsMin == kBlock, "a block's rows");
+    // one a thread of the density pass's grid
     const uint32_t nb = (n + kBlock - 1) / kBlock, r0 = g_resident[3].load(), r1 = g_resident[4].load();
     const uint32_t resident = r0 && r1 ? std::max(r0, r1) : nb;
-    // (with lanes to share, a list room a row of the grid, whose last tile may be part empty)
+    // (with lanes to share, one a row of the grid, whose last tile may be part empty)
     const size_t group = group_lanes(n, support, dfsph) ? size_t(n + kGroupBlock) : 0;
-    return std::max(size_t(std::min(resident, nb)) * kBlock, group) * cap;
+    return std::max(size_t(std::min(resident, nb)) * kBlock, group);
 }
 
 void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float4* pos, const float4* walls,
                     const PairLists& fl, const PairLists& wl, float* rho, float* press, float* scaled, float* alpha,
                     Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M,
-                    uint32_t* scratch, float4* vel) {
+                    uint32_t* scratch, size_t scratch_rows, float4* vel) {
     if (!p.n) return;
     const PairRecords rec{reinterpret_cast<float*>(pos), reinterpret_cast<float*>(vel)};
     const DensityIn in{{fg, wg}, {pos, walls}, {fl, wl}};
     // (terrain, whose sites every lane would take alike, and a DFSPH row's body points keep a thread a row)
-    const bool shared = T.regions == 0 && slope == nullptr && (p.solver == 0 || M.count == 0);
+    const bool shared = T.regions == 0 && slope == nullptr && (p.solver == 0 || M.count == 0) &&
+                        scratch_rows >= size_t(p.n) + kGroupBlock;
     if (shared && with_lanes(group_lanes(p.n, p.radius / p.spacing, p.solver != 0), [&](auto lanes) {
             constexpr int L = decltype(lanes)::value;
             const uint32_t nb = group_blocks(p.n, L);
@@ -2365,7 +2367,7 @@ void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float
             else launch(std::integral_constant<int, 4>{});
         }))
         return;
-    const uint32_t nb = solver_blocks(p.n, p.solver == 0 ? 3 : 4);
+    const uint32_t nb = uint32_t(std::min<size_t>(solver_blocks(p.n, p.solver == 0 ? 3 : 4), scratch_rows / kBlock));
     auto launch = [&](auto wide) {
         constexpr bool W = decltype(wide)::value;
         // (no DFSPH step takes terrain, but the densities of a DFSPH world on terrain have its ground)

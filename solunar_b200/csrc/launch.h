@@ -97,9 +97,11 @@ inline int adjoint_lanes(uint32_t n, float support) {
 void launch_density(const Params& p, const GridDev& fg, const GridDev& wg, float4* pos, const float4* walls,
                     const PairLists& fl, const PairLists& wl, float* rho, float* press, float* scaled, float* alpha,
                     Status* st, const TerrainDev& T, float4* slope, cudaStream_t s, const MoverDev& M,
-                    uint32_t* scratch, float4* vel);
-// words of launch_density's scratch for n particles and lists of cap slots
-size_t density_scratch_words(uint32_t n, uint32_t cap, float support, bool dfsph);
+                    uint32_t* scratch, size_t scratch_rows, float4* vel);
+// rows whose lists launch_density's scratch holds at once for n particles, a list's room each; a scratch of
+// fewer (kBlock at least) runs fewer blocks, a thread a row
+size_t density_scratch_rows(uint32_t n, float support, bool dfsph);
+constexpr size_t kDensityRowsMin = 256;
 // vel_pre (optional): the velocity before the wall clamp, its w lane the bits of the components
 // the clamp zeroed (1 x, 2 y, 4 z), for the adjoint
 void launch_wcsph_force(const Params& p, const StepConsts* sc, const PairLists& fl, const PairLists& wl,

@@ -346,7 +346,12 @@ struct World {
     // EXACT DFSPH: each pair's kernel gradient at the same slots (PairLists::gv), for the check
     DevBuf<float4> fgv, wgv;
     DevBuf<uint32_t> fcnt, wcnt;
-    DevBuf<uint32_t> dscratch;  // the EXACT density pass's unfinished lists (density_scratch_words)
+    // the EXACT density pass's unfinished lists, of density_rows rows at once: those of its grid, or, where
+    // the device has no room for them (crowds, whose lists run to megabytes a row), half as many and so on
+    DevBuf<uint32_t> dscratch;
+    size_t density_rows = 0;
+    size_t density_rows_most = 0;  // testing: no more than this (0: no limit)
+    int32_t ensure_density_scratch();
     uint32_t list_cap = 0;
     DevBuf<uint8_t> partials;
     bool stats_fresh = false;  // status holds bbox and speed of the committed state

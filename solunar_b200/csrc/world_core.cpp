@@ -354,10 +354,21 @@ int32_t World::ensure_work_buffers() {
     SLF_TRY(cslot.ensure(n, 0, stream));
     SLF_TRY(members.ensure(n, 0, stream));
     SLF_TRY(partials.ensure(rate_partial_bytes(uint32_t(n)), 0, stream));
-    if (!fast()) {
-        const bool dfsph = s.solver == SLF_SOLVER_DFSPH;
-        SLF_TRY(dscratch.ensure(density_scratch_words(uint32_t(n), list_cap, radius / s.spacing, dfsph), 0, stream));
+    if (!fast()) SLF_TRY(ensure_density_scratch());
+    return SLF_OK;
+}
+
+int32_t World::ensure_density_scratch() {
+    size_t rows = density_scratch_rows(uint32_t(n), radius / s.spacing, s.solver == SLF_SOLVER_DFSPH);
+    if (density_rows_most) rows = std::min(rows, std::max(density_rows_most, kDensityRowsMin));
+    for (;;) {
+        const int32_t st = dscratch.ensure(rows * list_cap, 0, stream);
+        if (st == SLF_OK) break;
+        cudaGetLastError();
+        if (rows <= kDensityRowsMin) return st;
+        rows = (rows / 2 + kDensityRowsMin - 1) / kDensityRowsMin * kDensityRowsMin;
     }
+    density_rows = rows;
     return SLF_OK;
 }
 
@@ -368,7 +379,7 @@ void World::density_pass(const Params& p, int a, const PairLists& fl, const Pair
                             alpha.p, d_status, on, vel[a].p);
     else
         launch_density(p, fgrid, wgrid, pos[a].p, dwalls.p, fl, wl, rh, press.p, scaled.p, alpha.p, d_status,
-                       tdev, ground_slopes(), on, mover_dev(), dscratch.p, vel[a].p);
+                       tdev, ground_slopes(), on, mover_dev(), dscratch.p, density_rows, vel[a].p);
 }
 
 void World::force_pass(const Params& p, const PairLists& fl, const PairLists& wl, int a, int b, int nid, cudaStream_t on) {

@@ -251,6 +251,7 @@ std::vector<uint8_t> World::substep_key(const Params& p, int a, int b, int nid, 
     key_add(k, sp.span);
     key_add(k, sp.volume);
     key_add(k, sp.pad);
+    key_add(k, density_rows);
     key_add(k, int32_t(sp.ordered));
     key_add(k, sp.job_lo);
     key_add(k, sp.job_hi);

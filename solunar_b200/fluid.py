@@ -83,6 +83,7 @@ def load_library():
         "slf_last_iterations": [vp, u32p, u32p],
         "slf_debug_skip_job": [vp, ctypes.c_int64],
         "slf_debug_list_room": [vp, ctypes.c_uint32],
+        "slf_debug_density_rows": [vp, ctypes.c_uint64],
         "slf_write_state": [vp, fp, fp, ctypes.c_uint64],
         "slf_get_stream": [vp, ctypes.POINTER(vp)],
         "slf_profile_enable": [vp, ctypes.c_int32],
@@ -328,6 +329,10 @@ class FluidWorld:
     def debug_list_room(self, room: int):
         """Test hook: shrinks the neighbour lists' room so the next substep outgrows it and runs again."""
         _check(_lib.slf_debug_list_room(self._h, room))
+
+    def debug_density_rows(self, rows: int):
+        """Test hook: limits the rows whose unfinished lists the EXACT density pass has room for."""
+        _check(_lib.slf_debug_density_rows(self._h, rows))
 
     # ---- read-outs (mod.rs:393-408, 612, 678) ----
     def ids(self) -> np.ndarray:
