@@ -2207,8 +2207,8 @@ static inline uint32_t blocks_for(uint32_t n) {
 #ifndef SLF_SOLVER_RESIDENT
 #define SLF_SOLVER_RESIDENT 1
 #endif
-// resident blocks of k_rate<0>, k_rate<1> and k_push (as large grids run them), k_density<0>, k_density<1>, k_wcsph_force on the
-// device (prepare_solver_grids; 0: not known yet, the grid then covers every row)
+// resident blocks of k_rate<0>, k_rate<1> and k_push (as large grids run them), k_density<0>,
+// k_density<1> and k_wcsph_force on the device (prepare_solver_grids; 0: not known yet, the grid then covers every row)
 static std::atomic<uint32_t> g_resident[6] = {0, 0, 0, 0, 0, 0};
 
 // blocks of the density pass up to which it runs wide: two a SM
@@ -2305,7 +2305,8 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
                          const uint32_t* ids_in, const float4* pos_in, const float4* vel_in, const float* rho_in,
                          const int4* cells_in, uint32_t* ids_out, float4* pos_out, float4* vel_out, float* rho_out,
                          int4* cells_out, const float2* warm_in, float2* warm_out, uint32_t skip_begin,
-                         uint32_t skip_end, Status* st, uint32_t* dest, int3 span, int pad, uint32_t* order, cudaStream_t s) {
+                         uint32_t skip_end, Status* st, uint32_t* dest, int3 span, int pad, uint32_t* order,
+                         cudaStream_t s) {
     if (n)
         k_rank_reorder<<<blocks_for(n), kBlock, 0, s>>>(n, lin, start, members, ids_in, pos_in, vel_in, rho_in,
                                                         cells_in, ids_out, pos_out, vel_out, rho_out, cells_out,

@@ -42,7 +42,8 @@ void launch_rank_reorder(uint32_t n, const uint32_t* lin, const uint32_t* start,
                          const uint32_t* ids_in, const float4* pos_in, const float4* vel_in, const float* rho_in,
                          const int4* cells_in, uint32_t* ids_out, float4* pos_out, float4* vel_out, float* rho_out,
                          int4* cells_out, const float2* warm_in, float2* warm_out, uint32_t skip_begin,
-                         uint32_t skip_end, Status* st, uint32_t* dest, int3 span, int pad, uint32_t* order, cudaStream_t s);
+                         uint32_t skip_end, Status* st, uint32_t* dest, int3 span, int pad, uint32_t* order,
+                         cudaStream_t s);
 
 // Lanes a row of the EXACT density pass and the WCSPH force pass (k_density_group,
 // k_wcsph_force_group) in scenes without terrain; 0: a thread a row.  A row's lanes keep the SMs

@@ -581,8 +581,8 @@ int32_t World::enqueue_sort(int to, const SortPlan& sp, cudaStream_t on, Substep
     timed("hash_reorder", bytes_per_particle::reorder, [&] {
         launch_rank_reorder(uint32_t(n), lin.p, count.p, members.p, ids[cid].p, pos[cpos].p, vel[cpos].p,
                             rho[cid].p, cells_of(cpos), ids[1 - cid].p, pos[to].p, vel[to].p, rho[1 - cid].p,
-                            cells_of(to), warm_in(), warm_out(), sp.job_lo, sp.job_hi, d_status, sort_dest, sp.span, sp.pad,
-                            sp.ordered ? worder.p : nullptr, on);
+                            cells_of(to), warm_in(), warm_out(), sp.job_lo, sp.job_hi, d_status, sort_dest, sp.span,
+                            sp.pad, sp.ordered ? worder.p : nullptr, on);
     });
     return SLF_OK;
 }
